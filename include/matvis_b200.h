@@ -130,10 +130,10 @@ int mvb_beam_interp(const void *grids, int grid_kind, int nbeam, int nax, int nf
                     const double *params, const double *crd, int64_t ld, const int32_t *n_dev, int64_t nsrc,
                     void *out, int out_c128, int64_t nout, int32_t *status, void *ws, size_t ws_bytes,
                     void *stream);
-/* Workspace of mvb_beam_interp (2 nbeam nout doubles).  With it (ws != NULL)
- * each source's az/za and grid coordinates are computed once for all planes
- * (a first kernel), with the same FP64 expressions; with ws = NULL every
- * plane's threads recompute them. */
+/* Workspace of mvb_beam_interp (2 nbeam nout doubles).  With it (ws != NULL) a
+ * call with many sources first lays the four planes of complex 2 x 2 grids side
+ * by side there (a first kernel), so that one gather serves them; with ws = NULL
+ * the planes are gathered one by one.  Same FP64 expressions, same results. */
 size_t mvb_beam_interp_ws_bytes(int nbeam, int64_t nout);
 /* Same interpolation at given (azimuth, zenith angle) rows azza (SoA, leading
  * dim ld): the reference's gpu_beam_interpolation(beam, daz, dza, azmin, az, za)

@@ -193,7 +193,7 @@ class B200BeamInterpolator(BeamInterpolator):
         nout = out.shape[-1]
         sh = stream_handle(stream)
         if self.use_interp:
-            # per-source grid coordinates, computed once for all the planes
+            # room for the grids laid out value by value (large calls)
             if self._coord_ws is None or self._coord_ws.numel() < 2 * self.nbeam * nout:
                 self._coord_ws = torch.empty(2 * self.nbeam * nout, dtype=torch.float64, device=self.device)
             ws = self._coord_ws

@@ -11,20 +11,26 @@
 // weight 0).
 //
 // Layout: grids (nbeam, nax, nfeed, nza, naz), complex64 or float32 power;
-// output (nbeam, nfeed, nax, nout) complex.  One CTA stages ONE real plane
-// (a component of one (beam, ax, feed) grid, <= 200 KB) in shared memory and
-// interpolates it for a slice of the sources.  With a workspace, a first kernel
-// computes each source's FP64 (az, za) and its grid coordinates for every beam
-// once; without one, every plane's CTA recomputes them.  Planes larger than the
-// shared memory budget are read through L2 instead.
+// output (nbeam, nfeed, nax, nout) complex.  One thread per source: the FP64
+// (az, za) and each beam's grid coordinates are computed once and serve all its
+// planes, whose 2 x 2 neighbours are gathered through L1 / L2 (a beam's grids are
+// about 1 MB: they stay in L2).  What bounds it is the gathers' sectors: four
+// planes of a complex beam stored apart take 2.6 sectors per (plane, source) for
+// scattered sources; with the four values of a grid point side by side
+// (beam_pack_kernel, into the caller's workspace) one neighbour is one 32-byte
+// sector for all of them.  Measured, 91 x 361 grids: 98,304 map sources x 4
+// polarised beams 16.5 us, 500,000 scattered sources x 4 70 us, 2,500 sources x 1
+// 6.2 us.  The form this replaces staged one real 131 KB plane per CTA in shared
+// memory (one CTA of 8 warps per SM, each plane reading the coordinates that a pass
+// before it had written): 95, 521 and 16.5 us.
 #include <math_constants.h>
 
 #include "common.cuh"
 
 namespace mvb {
 
-constexpr int kBeamThreads = 256;
-constexpr size_t kBeamSmemMax = 200 * 1024;
+constexpr int kBeamThreads = 128;
+constexpr int64_t kBeamPackMin = 300000;  // (source slots - 2 grid points) x beams from which packing pays
 
 struct BeamParams {
   double daz, dza, azmin;
@@ -46,103 +52,145 @@ __device__ __forceinline__ void az_za_uvbeam(double e, double n, double &az, dou
   az = py_mod(0.5 * CUDART_PI - a, 2.0 * CUDART_PI);
 }
 
-// Bilinear (order-1, mode='constant') sample of a real plane `p` (nza x naz,
-// row-major, element stride `es` floats).
-template <typename Load>
-__device__ __forceinline__ double bilinear(Load p, int nza, int naz, double row, double col) {
-  if (!(row >= 0.0 && row <= (double)(nza - 1) && col >= 0.0 && col <= (double)(naz - 1))) return 0.0;
+// Order-1 neighbours of one grid position: offsets (in grid points) and weights;
+// in = false outside [0, n - 1] on either axis (the sample is then 0).
+struct Cell {
+  int64_t o00, o01, o10, o11;
+  double fr, fc;
+  bool in;
+};
+
+__device__ __forceinline__ Cell grid_cell(int nza, int naz, double row, double col) {
+  Cell c{0, 0, 0, 0, 0.0, 0.0, false};
+  if (!(row >= 0.0 && row <= (double)(nza - 1) && col >= 0.0 && col <= (double)(naz - 1))) return c;
   const int r0 = min((int)floor(row), nza - 1);
   const int c0 = min((int)floor(col), naz - 1);
-  const double fr = row - r0, fc = col - c0;
+  c.fr = row - r0;
+  c.fc = col - c0;
   const int r1 = min(r0 + 1, nza - 1), c1 = min(c0 + 1, naz - 1);
-  const double v00 = p(r0, c0), v01 = p(r0, c1), v10 = p(r1, c0), v11 = p(r1, c1);
-  return (1.0 - fr) * ((1.0 - fc) * v00 + fc * v01) + fr * ((1.0 - fc) * v10 + fc * v11);
+  c.o00 = (int64_t)r0 * naz + c0;
+  c.o01 = (int64_t)r0 * naz + c1;
+  c.o10 = (int64_t)r1 * naz + c0;
+  c.o11 = (int64_t)r1 * naz + c1;
+  c.in = true;
+  return c;
 }
 
-// Grid coordinates of every source for every beam, once per call:
-// rc[(2 b) nout + i] = za / dza_b, rc[(2 b + 1) nout + i] = (az - azmin_b) / daz_b
-// (the plane kernel's own FP64 expressions), and row -1 (outside every grid:
-// a zero) for the slots i >= n.  One thread per source.
-__global__ void beam_rowcol_kernel(const BeamParams *__restrict__ params, int nbeam, const double *__restrict__ crd,
-                                   int64_t ld, const int32_t *__restrict__ n_dev, int64_t nsrc, int64_t nout,
-                                   double *__restrict__ rc) {
-  const int64_t n = n_dev ? min((int64_t)*n_dev, nsrc) : nsrc;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nout; i += (int64_t)gridDim.x * blockDim.x) {
-    double az = 0.0, za = 0.0;
-    if (i < n) az_za_uvbeam(crd[i], crd[ld + i], az, za);
-    for (int b = 0; b < nbeam; ++b) {
-      const BeamParams bp = params[b];
-      rc[(2 * b) * nout + i] = i < n ? za / bp.dza : -1.0;
-      rc[(2 * b + 1) * nout + i] = i < n ? (az - bp.azmin) / bp.daz : -1.0;
-    }
+__device__ __forceinline__ double blend(const Cell &c, double v00, double v01, double v10, double v11) {
+  return (1.0 - c.fr) * ((1.0 - c.fc) * v00 + c.fc * v01) + c.fr * ((1.0 - c.fc) * v10 + c.fc * v11);
+}
+
+// kind 0: complex64, 1: complex128 (one store); 2, 3: the same for an output that is
+// not aligned to its complex elements (a C caller's), one store per component.
+__device__ __forceinline__ void store_beam(void *out, int kind, int64_t idx, double re, double im) {
+  if (kind == 0) {
+    static_cast<float2 *>(out)[idx] = make_float2((float)re, (float)im);
+  } else if (kind == 1) {
+    static_cast<double2 *>(out)[idx] = make_double2(re, im);
+  } else if (kind == 2) {
+    static_cast<float *>(out)[2 * idx] = (float)re;
+    static_cast<float *>(out)[2 * idx + 1] = (float)im;
+  } else {
+    static_cast<double *>(out)[2 * idx] = re;
+    static_cast<double *>(out)[2 * idx + 1] = im;
   }
 }
 
-// grid_kind 0: complex64 (ncomp = 2), 1: float32 power (ncomp = 1).
-// plane q = ((b * nax + ax) * nfeed + fd) * ncomp + comp.
-// kCoord 0: crd holds ENU (e, n) rows, az/za computed here per plane;
-// 1: crd holds (az, za) rows; 2: crd holds beam_rowcol_kernel's grid
-// coordinates (leading dimension nout), so no per-plane trigonometry.
-template <bool kStaged, int kCoord = 0>
+// A complex value of a grid; `whole`: the grids are 8-byte aligned.
+__device__ __forceinline__ float2 load_grid(const float *g, int64_t o, bool whole) {
+  return whole ? __ldg(reinterpret_cast<const float2 *>(g) + o) : make_float2(__ldg(g + 2 * o), __ldg(g + 2 * o + 1));
+}
+
+// The four complex planes of every beam, (nbeam, 4, points) -> (nbeam, points, 4).
+__global__ void beam_pack_kernel(const float2 *__restrict__ grids, int64_t points, int nbeam,
+                                 float4 *__restrict__ packed) {
+  const int64_t total = (int64_t)nbeam * points;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = i / points, p = i % points;
+    const float2 *g = grids + 4 * b * points + p;
+    const float2 v0 = g[0], v1 = g[points], v2 = g[2 * points], v3 = g[3 * points];
+    packed[2 * i] = make_float4(v0.x, v0.y, v1.x, v1.y);
+    packed[2 * i + 1] = make_float4(v2.x, v2.y, v3.x, v3.y);
+  }
+}
+
+// One thread per source; blockIdx.y = a slice of `per_y` beams.  KIND 0: complex64
+// planes, 1: float32 power planes, 2: packed complex64 (4 values per grid point,
+// nax = nfeed = 2).  AZZA: crd holds (az, za) rows instead of ENU (e, n).
+template <int KIND, bool AZZA>
 __global__ void __launch_bounds__(kBeamThreads)
-    beam_plane_kernel(const float *__restrict__ grids, int grid_kind, int nbeam, int nax, int nfeed, int nza, int naz,
-                      const BeamParams *__restrict__ params, const double *__restrict__ crd, int64_t ld,
-                      const int32_t *__restrict__ n_dev, int64_t nsrc, void *__restrict__ out, int out_c128,
-                      int64_t nout, int32_t *__restrict__ status) {
-  extern __shared__ float plane_smem[];
-  const int ncomp = grid_kind == 0 ? 2 : 1;
-  const int q = blockIdx.x;
-  const int comp = q % ncomp;
-  const int gidx = q / ncomp;  // (b, ax, fd) flattened
-  const int fd = gidx % nfeed;
-  const int ax = (gidx / nfeed) % nax;
-  const int b = gidx / (nfeed * nax);
-  const int64_t plane_elems = (int64_t)nza * naz;
-  const float *src = grids + (int64_t)gidx * plane_elems * ncomp + comp;
-
-  if (kStaged) {
-    for (int64_t i = threadIdx.x; i < plane_elems; i += kBeamThreads) plane_smem[i] = src[i * ncomp];
-    __syncthreads();
-  }
+    beam_gather_kernel(const float *__restrict__ grids, int nbeam, int per_y, int nax, int nfeed, int nza, int naz,
+                       const BeamParams *__restrict__ params, const double *__restrict__ crd, int64_t ld,
+                       const int32_t *__restrict__ n_dev, int64_t nsrc, void *__restrict__ out, int out_kind,
+                       int64_t nout, int32_t *__restrict__ status) {
   const int64_t n = n_dev ? min((int64_t)*n_dev, nsrc) : nsrc;
-  const BeamParams bp = params[b];
-  const int64_t out_row = (((int64_t)b * nfeed + fd) * nax + ax) * nout;  // (b, fd, ax, :)
-
-  for (int64_t i = blockIdx.y * (int64_t)kBeamThreads + threadIdx.x; i < nout; i += (int64_t)gridDim.y * kBeamThreads) {
-    double v = 0.0;
-    if (i < n) {
-      double row, col;
-      if constexpr (kCoord == 2) {
-        row = crd[(2 * b) * nout + i];
-        col = crd[(2 * b + 1) * nout + i];
-      } else {
-        double az, za;
-        if constexpr (kCoord == 1) {
-          az = crd[i];
-          za = crd[ld + i];
-        } else {
-          az_za_uvbeam(crd[i], crd[ld + i], az, za);
-        }
-        row = za / bp.dza;
-        col = (az - bp.azmin) / bp.daz;
-      }
-      if (kStaged)
-        v = bilinear([&](int r, int c) { return (double)plane_smem[(int64_t)r * naz + c]; }, nza, naz, row, col);
-      else
-        v = bilinear([&](int r, int c) { return (double)__ldg(src + ((int64_t)r * naz + c) * ncomp); }, nza, naz,
-                     row, col);
-      if (grid_kind == 1) v = sqrt(v);
-      if (status && !isfinite(v)) atomicOr(status, MVB_DEV_NONFINITE);
+  const bool whole = reinterpret_cast<uintptr_t>(grids) % 8 == 0;
+  const int b0 = blockIdx.y * per_y, b1 = min(b0 + per_y, nbeam);
+  const int64_t points = (int64_t)nza * naz;
+  const int ngrid = nax * nfeed;
+  for (int64_t i = blockIdx.x * (int64_t)kBeamThreads + threadIdx.x; i < nout; i += (int64_t)gridDim.x * kBeamThreads) {
+    if (i >= n) {  // slots past the count hold zeros
+      for (int64_t q = (int64_t)b0 * ngrid; q < (int64_t)b1 * ngrid; ++q) store_beam(out, out_kind, q * nout + i, 0.0, 0.0);
+      continue;
     }
-    if (out_c128) {
-      double *o = static_cast<double *>(out) + 2 * (out_row + i);
-      o[comp] = v;
-      if (ncomp == 1) o[1] = 0.0;
+    double az, za;
+    if constexpr (AZZA) {
+      az = crd[i];
+      za = crd[ld + i];
     } else {
-      float *o = static_cast<float *>(out) + 2 * (out_row + i);
-      o[comp] = (float)v;
-      if (ncomp == 1) o[1] = 0.0f;
+      az_za_uvbeam(crd[i], crd[ld + i], az, za);
     }
+    bool finite = true;
+    for (int b = b0; b < b1; ++b) {
+      const BeamParams bp = params[b];
+      const Cell c = grid_cell(nza, naz, za / bp.dza, (az - bp.azmin) / bp.daz);
+      const int64_t row0 = (int64_t)b * ngrid * nout + i;  // output (b, feed, axis, i), rows nout apart
+      if constexpr (KIND == 2) {
+        const float4 *g = reinterpret_cast<const float4 *>(grids) + 2 * (int64_t)b * points;
+        // values of a point: (ax 0, feed 0), (ax 0, feed 1), (ax 1, feed 0), (ax 1, feed 1)
+        double v[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 v00 = c.in ? __ldg(g + 2 * c.o00 + h) : z4, v01 = c.in ? __ldg(g + 2 * c.o01 + h) : z4;
+          const float4 v10 = c.in ? __ldg(g + 2 * c.o10 + h) : z4, v11 = c.in ? __ldg(g + 2 * c.o11 + h) : z4;
+          v[4 * h + 0] = blend(c, v00.x, v01.x, v10.x, v11.x);
+          v[4 * h + 1] = blend(c, v00.y, v01.y, v10.y, v11.y);
+          v[4 * h + 2] = blend(c, v00.z, v01.z, v10.z, v11.z);
+          v[4 * h + 3] = blend(c, v00.w, v01.w, v10.w, v11.w);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // q = 2 ax + feed -> output row 2 feed + ax
+          const double re = v[2 * q], im = v[2 * q + 1];
+          finite = finite && isfinite(re) && isfinite(im);
+          store_beam(out, out_kind, row0 + (int64_t)(2 * (q & 1) + (q >> 1)) * nout, re, im);
+        }
+      } else {
+#pragma unroll 2
+        for (int q = 0; q < ngrid; ++q) {
+          const int ax = q / nfeed, fd = q % nfeed;
+          double re = 0.0, im = 0.0;
+          if (KIND == 0) {
+            if (c.in) {
+              const float *g = grids + 2 * ((int64_t)b * ngrid + q) * points;
+              const float2 v00 = load_grid(g, c.o00, whole), v01 = load_grid(g, c.o01, whole),
+                           v10 = load_grid(g, c.o10, whole), v11 = load_grid(g, c.o11, whole);
+              re = blend(c, v00.x, v01.x, v10.x, v11.x);
+              im = blend(c, v00.y, v01.y, v10.y, v11.y);
+            }
+          } else {
+            if (c.in) {
+              const float *g = grids + ((int64_t)b * ngrid + q) * points;
+              re = blend(c, __ldg(g + c.o00), __ldg(g + c.o01), __ldg(g + c.o10), __ldg(g + c.o11));
+            }
+            re = sqrt(re);
+          }
+          finite = finite && isfinite(re) && isfinite(im);
+          store_beam(out, out_kind, row0 + (int64_t)(fd * nax + ax) * nout, re, im);
+        }
+      }
+    }
+    if (status && !finite) atomicOr(status, MVB_DEV_NONFINITE);
   }
 }
 
@@ -188,54 +236,50 @@ static int beam_interp_impl(bool azza, const void *grids, int grid_kind, int nbe
   if (ws && (ws_bytes < (size_t)2 * nbeam * nout * sizeof(double) || reinterpret_cast<uintptr_t>(ws) % 8))
     return fail(MVB_ERR_ARG, "%s: workspace too small", who);
   if (nout == 0) return MVB_OK;
-  const int ncomp = grid_kind == 0 ? 2 : 1;
-  const int nplanes = nbeam * nax * nfeed * ncomp;
-  const size_t plane_bytes = (size_t)nza * naz * sizeof(float);
   const int nsm = num_sms();
-  const int64_t ychunks = std::max<int64_t>(1, std::min<int64_t>(ceil_div(nout, kBeamThreads),
-                                                                  ceil_div((int64_t)nsm * 2, nplanes)));
-  dim3 grid(nplanes, (unsigned)ychunks);
-  cudaStream_t s = as_stream(stream);
+  const int64_t points = (int64_t)nza * naz;
   const BeamParams *bp = reinterpret_cast<const BeamParams *>(params);
   const float *g = static_cast<const float *>(grids);
-  // with a workspace, the grid coordinates of each source are computed once for
-  // all planes (the ENU form only)
-  const bool pre = ws && !azza;
-  const double *coords = crd;
-  if (pre) {
-    const int64_t blocks = std::min<int64_t>(ceil_div(nout, kBeamThreads), (int64_t)nsm * 8);
-    beam_rowcol_kernel<<<(unsigned)blocks, kBeamThreads, 0, s>>>(bp, nbeam, crd, ld, n_dev, nsrc, nout,
-                                                                 static_cast<double *>(ws));
-    int rc = check_launch("beam_rowcol_kernel");
+  cudaStream_t s = as_stream(stream);
+  // Packing costs a launch (about 2 us) and one read and write of the grids, and
+  // saves the gathers sectors: 91 x 361 grids, half of the slots occupied by
+  // scattered sources: 4 beams, 66,000 slots 14.0 us packed, 12.4 not; 120,000 slots
+  // 18.5 both; 196,608 slots 22.7 and 28.7; 1 beam, 500,000 slots 17.7 and 17.6.
+  const bool pack = !azza && ws && grid_kind == 0 && nax == 2 && nfeed == 2 && nbeam * (nout - 2 * points) >= kBeamPackMin &&
+                    ws_bytes >= (size_t)nbeam * points * 32 && reinterpret_cast<uintptr_t>(ws) % 16 == 0 &&
+                    reinterpret_cast<uintptr_t>(grids) % 8 == 0;
+  const int out_kind = (out_c128 ? 1 : 0) + (reinterpret_cast<uintptr_t>(out) % (out_c128 ? 16 : 8) ? 2 : 0);
+  if (pack) {
+    const int64_t blocks = std::min<int64_t>(ceil_div(nbeam * points, 256), (int64_t)nsm * 8);
+    beam_pack_kernel<<<(unsigned)blocks, 256, 0, s>>>(static_cast<const float2 *>(grids), points, nbeam,
+                                                      static_cast<float4 *>(ws));
+    int rc = check_launch("beam_pack_kernel");
     if (rc) return rc;
-    coords = static_cast<const double *>(ws);
+    g = static_cast<const float *>(ws);
   }
-#define MVB_BEAM(ST, CO, SM)                                                                                        \
-  beam_plane_kernel<ST, CO><<<grid, kBeamThreads, SM, s>>>(g, grid_kind, nbeam, nax, nfeed, nza, naz, bp, coords, ld, \
-                                                           n_dev, nsrc, out, out_c128, nout, status)
-  const int co = pre ? 2 : (azza ? 1 : 0);
-  if (plane_bytes <= kBeamSmemMax) {
-    const void *fn = co == 2 ? reinterpret_cast<const void *>(beam_plane_kernel<true, 2>)
-                             : (co == 1 ? reinterpret_cast<const void *>(beam_plane_kernel<true, 1>)
-                                        : reinterpret_cast<const void *>(beam_plane_kernel<true, 0>));
-    int rc = set_smem_once(fn, (int)kBeamSmemMax, 10 + co);
-    if (rc) return rc;
-    if (co == 2)
-      MVB_BEAM(true, 2, plane_bytes);
-    else if (co == 1)
-      MVB_BEAM(true, 1, plane_bytes);
+  // few sources: the beams go to different CTAs (each repeats the source's az/za)
+  const int64_t xblocks = std::min<int64_t>(ceil_div(nout, kBeamThreads), (int64_t)nsm * 64);
+  const int per_y = xblocks >= (int64_t)nsm * 4 ? nbeam : 1;
+  const dim3 grid((unsigned)xblocks, (unsigned)std::min<int64_t>(ceil_div(nbeam, per_y), 65535));
+  const int per = (int)ceil_div(nbeam, grid.y);
+#define MVB_BEAM(KIND, AZZA)                                                                                          \
+  beam_gather_kernel<KIND, AZZA><<<grid, kBeamThreads, 0, s>>>(g, nbeam, per, nax, nfeed, nza, naz, bp, crd, ld, n_dev, \
+                                                               nsrc, out, out_kind, nout, status)
+  if (pack)
+    MVB_BEAM(2, false);
+  else if (grid_kind == 0) {
+    if (azza)
+      MVB_BEAM(0, true);
     else
-      MVB_BEAM(true, 0, plane_bytes);
+      MVB_BEAM(0, false);
   } else {
-    if (co == 2)
-      MVB_BEAM(false, 2, 0);
-    else if (co == 1)
-      MVB_BEAM(false, 1, 0);
+    if (azza)
+      MVB_BEAM(1, true);
     else
-      MVB_BEAM(false, 0, 0);
+      MVB_BEAM(1, false);
   }
 #undef MVB_BEAM
-  return check_launch("beam_plane_kernel");
+  return check_launch("beam_gather_kernel");
 }
 
 extern "C" size_t mvb_beam_interp_ws_bytes(int nbeam, int64_t nout) {

@@ -283,7 +283,7 @@ class VisEngine:
             bf.setup()
             if self.bmfuncs:
                 # the per-frequency interpolators run in turn on one stream: one
-                # output and one coordinate workspace serve them all
+                # output and one workspace serve them all
                 bf.interpolated_beam = self.bmfuncs[0].interpolated_beam
             self.bmfuncs.append(bf)
         if self.bmfuncs[0].use_interp:
@@ -516,7 +516,7 @@ class VisEngine:
         # and its reduction (mvb_herk[_grouped] + reduce, or vecdot_kernel + its slice reduction)
         per_f = 3
         nlaunch = len(self.freqs) if self.fgroup <= 1 else -(-len(self.freqs) // self.fgroup)
-        # a gridded beam is two launches (grid coordinates, then the planes), an analytic one one
+        # a gridded beam is at most two launches (a large call lays the grids out first), an analytic one one
         bl = 1 if all(hasattr(b, "sigma") for b in self.spec.beams) else 2
         # count + scatter + beam (+ frame), per frequency (+ its beam for a beamfits beam)
         per_chunk = 2 + bl * int(not self.chromatic) + (per_f + bl * int(self.chromatic)) * nlaunch + int(self.pol_sky)
