@@ -122,37 +122,36 @@ __device__ __forceinline__ void product_terms(int nprod, int q, uint32_t &pa, ui
 // n_tiles * nsplit work units fill whole waves of nsm SMs as evenly as possible
 // (a candidate replaces the best so far only when 1e-3 more efficient, so ties
 // keep fewer slices; the scan stops at the first candidate of 64 columns).
-// Each lane of a warp evaluates one candidate and the scan runs over the
-// shuffled efficiencies, so every warp reaches the same plan in one candidate's
-// arithmetic; every lane of the warp must call it.  Used identically by the
-// product and its reductions.
+// Each lane of a warp evaluates one candidate, and the scan jumps from one
+// improvement to the next with a ballot, so every warp reaches the same plan in
+// one candidate's arithmetic and a few votes; every lane of the warp must call it.
+// Every count fits 32 bits (check_herk_shape).  Used identically by the product
+// and its reductions.
 __device__ __forceinline__ void plan_splits(int64_t kvalid, int n_tiles, int kmax, int nsm, int &nsplit, int64_t &kc) {
   if (kvalid <= 0) {  // kvalid is uniform over the grid
     nsplit = 0;
     kc = kmax;
     return;
   }
-  const int64_t nmin = (kvalid + kmax - 1) / kmax;
-  const int64_t n = nmin + (threadIdx.x & 31);
-  int64_t c = (kvalid + n - 1) / n;
-  c = ((c + 63) / 64) * 64;
-  const int64_t ne = (kvalid + c - 1) / c;
-  const int64_t units = (int64_t)n_tiles * ne;
-  const int64_t waves = (units + nsm - 1) / nsm;
-  const double eff = (double)units / (double)(waves * nsm);
+  const uint32_t kv = (uint32_t)kvalid, lane = threadIdx.x & 31;
+  const uint32_t n = (kv + (uint32_t)kmax - 1) / (uint32_t)kmax + lane;
+  const uint32_t c = ((kv + n - 1) / n + 63) / 64 * 64;
+  const uint32_t ne = (kv + c - 1) / c;
+  const uint32_t units = (uint32_t)n_tiles * ne;
+  const uint32_t waves = (units + (uint32_t)nsm - 1) / (uint32_t)nsm;
+  const double eff = (double)units / ((double)waves * (double)nsm);
   const unsigned stop = __ballot_sync(0xffffffffu, c <= 64);
-  double best = -1.0;
+  const unsigned allowed = stop ? 0xffffffffu >> (32 - __ffs(stop)) : 0xffffffffu;  // up to the first stop, inclusive
   int win = 0;
-  for (int l = 0; l <= kPlanExtra; ++l) {
-    const double e = __shfl_sync(0xffffffffu, eff, l);
-    if (e > best + 1e-3) {
-      best = e;
-      win = l;
-    }
-    if ((stop >> l) & 1u) break;
+  double best = __shfl_sync(0xffffffffu, eff, 0);
+  while (true) {
+    const unsigned better = __ballot_sync(0xffffffffu, eff > best + 1e-3) & allowed & (0xfffffffeu << win);
+    if (!better) break;
+    win = __ffs(better) - 1;
+    best = __shfl_sync(0xffffffffu, eff, win);
   }
   nsplit = (int)__shfl_sync(0xffffffffu, ne, win);
-  kc = __shfl_sync(0xffffffffu, c, win);
+  kc = (int64_t)__shfl_sync(0xffffffffu, c, win);
 }
 
 // Valid K columns: (source count) x (columns per source), clamped to the panel.
@@ -585,7 +584,8 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
 // FP64 reduction of the partial tiles into the reference output layout
 // out[pair, p, q] = V[ant_i * F + q, ant_j * F + p].
 // ---------------------------------------------------------------------------
-constexpr int kRedGroups = 16;  // 8-column groups per 128-column tile
+constexpr int kRedBlocks = 16;    // 32 x 32 blocks of a 128 x 128 tile, one CTA each
+constexpr int kRedThreads = 256;  // threads over one block: four rows of one column each
 
 __device__ __forceinline__ int tile_index(int I, int J, int T) { return I * T - (I * (I - 1)) / 2 + (J - I); }
 
@@ -617,126 +617,95 @@ struct FF {
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
 
-// Sums of the k-slices' partial values of this thread's four rows r0 .. r0 + 3
-// of column c, real and imaginary halves.
-__device__ __forceinline__ void sum_slices(const float *__restrict__ tile, int nsplit, size_t tstride, int c, int r0,
-                                           FF (&are)[4], FF (&aim)[4]) {
-  const size_t sstride = tstride / 4;  // in float4
-  const float4 *pre = reinterpret_cast<const float4 *>(tile + c * 128 + r0);
-  const float4 *pim = reinterpret_cast<const float4 *>(tile + (128 + c) * 128 + r0);
-  int s = 0;
-  // eight slices per step: 16 independent 16-byte loads in flight, sums in slice order
-  for (; s + 8 <= nsplit; s += 8) {
-    float4 vr[8], vi[8];
+// Adds the slices of NP runs of four rows (a float4 each, sstride float4 apart
+// per slice) to their float-float sums in slice order, U slices' loads in flight
+// at a time.
+template <int NP, int U>
+__device__ __forceinline__ void sum_slices(const float4 *const (&p)[NP], int nsplit, size_t sstride,
+                                           FF (&acc)[NP][4]) {
+  for (int s = 0; s < nsplit; s += U) {
+    float4 v[U][NP];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      vr[u] = __ldg(pre + (s + u) * sstride);
-      vi[u] = __ldg(pim + (s + u) * sstride);
-    }
+    for (int u = 0; u < U; ++u)
+      if (s + u < nsplit) {
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      are[0].add(vr[u].x), are[1].add(vr[u].y), are[2].add(vr[u].z), are[3].add(vr[u].w);
-      aim[0].add(vi[u].x), aim[1].add(vi[u].y), aim[2].add(vi[u].z), aim[3].add(vi[u].w);
-    }
-  }
-  for (; s < nsplit; ++s) {
-    const float4 vr = __ldg(pre + s * sstride), vi = __ldg(pim + s * sstride);
-    are[0].add(vr.x), are[1].add(vr.y), are[2].add(vr.z), are[3].add(vr.w);
-    aim[0].add(vi.x), aim[1].add(vi.y), aim[2].add(vi.z), aim[3].add(vi.w);
-  }
-}
-
-// sum_slices for a diagonal tile, plus the imaginary half's transposed elements
-// (row c, columns r0 .. r0 + 3) for Im V = W - W^T.  The CTA (columns c0 ..
-// c0 + 7, warp w = c - c0) stages them through shared memory two slices at a
-// time (eight held 176 registers a thread and four spilled at the 80 registers
-// that keep three CTAs of the kernel on an SM): thread i loads 16 bytes of column i / 2 (rows c0 + 4 (i % 2) .. + 3, two
-// threads per 32-byte sector) and scatters them so that every thread then
-// reads its four values as one 16-byte word.  Every thread of the CTA must
-// call it: it holds __syncthreads, and nsplit is uniform over the CTA.
-__device__ __forceinline__ void sum_slices_diag(const float *__restrict__ tile, int nsplit, size_t tstride, int c0,
-                                                int w, int lane, FF (&are)[4], FF (&aim)[4], FF (&aimt)[4]) {
-  constexpr int kS = 2;              // slices per step
-  __shared__ float4 tsm[kS][8][32];  // [slice of the step][column warp][lane]: rows 4 lane .. 4 lane + 3
-  const int c = c0 + w, r0 = 4 * lane;
-  const size_t sstride = tstride / 4;  // in float4
-  const float4 *pre = reinterpret_cast<const float4 *>(tile + c * 128 + r0);
-  const float4 *pim = reinterpret_cast<const float4 *>(tile + (128 + c) * 128 + r0);
-  const int rr = threadIdx.x >> 1, hh = threadIdx.x & 1;  // this thread's load: column rr, rows c0 + 4 hh ..
-  const float4 *pt = reinterpret_cast<const float4 *>(tile + (128 + rr) * 128 + c0 + 4 * hh);
-  // element (row c0 + 4 hh + j, column rr) belongs to warp 4 hh + j, lane rr / 4, component rr % 4
-  float *tdst = reinterpret_cast<float *>(&tsm[0][4 * hh][rr >> 2]) + (rr & 3);
-  for (int s = 0; s < nsplit; s += kS) {
-    const int nu = min(kS, nsplit - s);
-    float4 vr[kS], vi[kS], vt[kS];
-#pragma unroll
-    for (int u = 0; u < kS; ++u)
-      if (u < nu) {
-        vr[u] = __ldg(pre + (s + u) * sstride);
-        vi[u] = __ldg(pim + (s + u) * sstride);
-        vt[u] = __ldg(pt + (s + u) * sstride);
+        for (int k = 0; k < NP; ++k) v[u][k] = __ldg(p[k] + (s + u) * sstride);
       }
-    __syncthreads();  // the previous step's reads of tsm are done
 #pragma unroll
-    for (int u = 0; u < kS; ++u)
-      if (u < nu) {
-        float *d = tdst + u * (8 * 32 * 4);
-        d[0 * 32 * 4] = vt[u].x;
-        d[1 * 32 * 4] = vt[u].y;
-        d[2 * 32 * 4] = vt[u].z;
-        d[3 * 32 * 4] = vt[u].w;
-      }
-    __syncthreads();
+    for (int u = 0; u < U; ++u)
+      if (s + u < nsplit) {
 #pragma unroll
-    for (int u = 0; u < kS; ++u)
-      if (u < nu) {
-        const float4 t4 = tsm[u][w][lane];
-        are[0].add(vr[u].x), are[1].add(vr[u].y), are[2].add(vr[u].z), are[3].add(vr[u].w);
-        aim[0].add(vi[u].x), aim[1].add(vi[u].y), aim[2].add(vi[u].z), aim[3].add(vi[u].w);
-        aimt[0].add(t4.x), aimt[1].add(t4.y), aimt[2].add(t4.z), aimt[3].add(t4.w);
+        for (int k = 0; k < NP; ++k) {
+          acc[k][0].add(v[u][k].x);
+          acc[k][1].add(v[u][k].y);
+          acc[k][2].add(v[u][k].z);
+          acc[k][3].add(v[u][k].w);
+        }
       }
   }
 }
 
-// One CTA (8 warps) per 8 columns of an upper tile: warp w sums column c0 + w,
-// lane l rows 4l .. 4l + 3 (a 16-byte load per component per k-slice; a warp
-// reads the column's two contiguous 512-byte runs).  A diagonal tile's
-// imaginary half is W - W^T of its partial sums (the product leaves W there).
+// One CTA per 32 x 32 block of an upper tile; a thread sums four rows of one
+// column.  A diagonal tile's imaginary half is W - W^T of its partial sums (the
+// product leaves W there): its CTA also sums the mirrored block of W and the two
+// are transposed through shared memory once, after the sums.  Blocks of padding
+// rows are not read.
+// What bounds it: the slices' bytes where there are many tiles, the chain of
+// loads of one thread where there are few (the plan then cuts many slices).  Both
+// want loads in flight and no barrier between them: 15 or 16 independent 16-byte
+// loads a thread.  Measured against CTAs of 8 columns x 128 rows, whose diagonal
+// tiles transposed every second slice through shared memory (two barriers each):
+// 8 panels of 700 rows, K = 196,608: 302 -> 251 us (4.2 TB/s of partial tiles); one
+// 43.5 -> 28.0; 8 panels of 90 rows, K = 11,180: 12.2 -> 8.6; one of 122 rows,
+// K = 20,000, slices of 576: 23.2 -> 13.4.  Four groups of threads sharing a block's
+// slices (1,024-thread CTAs) were slower: 10.8 us on the 90 rows, 14.2 on the 122.
 // F is a template parameter (no runtime integer division in the index
 // arithmetic).  blockIdx.y is the panel of a grouped product; its output is
 // out_stride bytes further.
 template <typename OT, int F>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(kRedThreads, 2)
     herk_reduce_all_kernel(const float *__restrict__ part, int ngroup, int T, int n_tiles,
                            const int32_t *__restrict__ n_dev, int64_t n_host, int kmul, int64_t Kcap, int k_chunk,
                            int nsm, int A, void *__restrict__ out_base, int64_t out_stride, double vscale,
                            int accumulate) {
-  const int t = blockIdx.x / kRedGroups, g = blockIdx.x % kRedGroups;
+  __shared__ FF turn_sm[32][33];
+  const int t = blockIdx.x / kRedBlocks, rb = blockIdx.x % 4, cb = blockIdx.x / 4 % 4;
   int I, J;
   decode_tile(t, T, I, J);
+  const int M = A * F;
+  if (I * 128 + rb * 32 >= M || J * 128 + cb * 32 >= M) return;  // padding (uniform over the CTA)
   const int64_t kvalid = valid_k(n_dev, n_host, kmul, Kcap);
   int nsplit;
   int64_t kc;
   plan_splits(kvalid, n_tiles * ngroup, k_chunk, nsm, nsplit, kc);
   void *out = static_cast<uint8_t *>(out_base) + (int64_t)blockIdx.y * out_stride;
   part += (size_t)blockIdx.y * nsplit * n_tiles * (256 * 128);
-  const int M = A * F;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = g * 8 + w;
-  const int n = J * 128 + c;
-  const int r0 = 4 * lane;
-  const bool live = n < M && I * 128 + r0 < M;  // this thread has outputs to write
-  FF are[4], aim[4], aimt[4];
+  const int cc = threadIdx.x >> 3, rr = 4 * (threadIdx.x & 7);  // column and first row within the block
+  const int c = cb * 32 + cc, r0 = rb * 32 + rr;
   const float *tile = part + (size_t)t * (256 * 128);
-  const size_t tstride = (size_t)n_tiles * (256 * 128);
-  if (I == J) {
-    // every thread takes part (the staging synchronises the CTA); its reads stay inside the tile
-    sum_slices_diag(tile, nsplit, tstride, g * 8, w, lane, are, aim, aimt);
-    if (!live) return;
+  const size_t sstride = (size_t)n_tiles * (256 * 128) / 4;  // in float4
+  const bool diag = I == J;
+  const float4 *pre = reinterpret_cast<const float4 *>(tile + c * 128 + r0);
+  const float4 *pim = reinterpret_cast<const float4 *>(tile + (128 + c) * 128 + r0);
+  FF acc[3][4];
+  if (diag && rb != cb) {
+    // the mirrored block: its column rb * 32 + cc, rows cb * 32 + rr ..
+    const float4 *const p[3] = {
+        pre, pim, reinterpret_cast<const float4 *>(tile + (128 + rb * 32 + cc) * 128 + cb * 32 + rr)};
+    sum_slices<3, 5>(p, nsplit, sstride, acc);
   } else {
-    if (!live) return;
-    sum_slices(tile, nsplit, tstride, c, r0, are, aim);
+    const float4 *const p[2] = {pre, pim};
+    FF(&acc2)[2][4] = reinterpret_cast<FF(&)[2][4]>(acc);
+    sum_slices<2, 8>(p, nsplit, sstride, acc2);
   }
+  if (diag) {
+    // element (row r, column c) subtracts W(c, r): column r, row c of the mirrored block
+#pragma unroll
+    for (int j = 0; j < 4; ++j) turn_sm[cc][rr + j] = rb != cb ? acc[2][j] : acc[1][j];
+    __syncthreads();
+  }
+  const int n = J * 128 + c;
+  if (n >= M) return;
   const int64_t AF2 = (int64_t)A * F * F;
   const int jj = n / F, pp = n % F;  // F is 1 or 2: shifts and masks
 #pragma unroll
@@ -744,14 +713,14 @@ __global__ void __launch_bounds__(256, 3)
     const int m = I * 128 + r0 + k;
     if (m >= M) break;
     // an autocorrelation of one feed (m == n) is real, as conj(z) z is in the reference
-    const double wi = I == J ? aim[k].value() - aimt[k].value() : aim[k].value();
-    const double re = are[k].value() * vscale, im = m == n ? 0.0 : wi * vscale;
+    const double wi = diag ? acc[1][k].value() - turn_sm[rr + k][cc].value() : acc[1][k].value();
+    const double re = acc[0][k].value() * vscale, im = m == n ? 0.0 : wi * vscale;
     const int i = m / F, q = m % F;
     // direct: rows m -> (i, q), columns n -> (j, p); out[(i*A + j)*F*F + p*F + q]
     store_out<OT>(out, i * AF2 + (int64_t)jj * F * F + pp * F + q, re, im, accumulate);
     // mirror: V[n, m] = conj(V[m, n]) for the off-diagonal tiles (a diagonal tile
     // holds both triangles and is written directly)
-    if (I != J) store_out<OT>(out, jj * AF2 + (int64_t)i * F * F + q * F + pp, re, -im, accumulate);
+    if (!diag) store_out<OT>(out, jj * AF2 + (int64_t)i * F * F + q * F + pp, re, -im, accumulate);
   }
 }
 
@@ -791,11 +760,26 @@ __global__ void herk_reduce_pairs_kernel(const float *__restrict__ part, int ngr
     const int r = m % 128, c = n % 128;
     const bool diag = m / 128 == n / 128;  // imaginary half W - W^T (see herk_reduce_all_kernel)
     FF re, im, imt;
-    for (int s = 0; s < nsplit; ++s) {
-      const float *p0 = part + ((size_t)s * n_tiles + t) * (256 * 128);
-      re.add(__ldg(p0 + c * 128 + r));
-      im.add(__ldg(p0 + (128 + c) * 128 + r));
-      if (diag) imt.add(__ldg(p0 + (128 + r) * 128 + c));
+    const float *p0 = part + (size_t)t * (256 * 128);
+    const size_t sstride = (size_t)n_tiles * (256 * 128);
+    constexpr int U = 8;  // slices in flight: the chain of scattered loads bounds a thread
+    for (int s = 0; s < nsplit; s += U) {
+      float vr[U], vi[U], vt[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (s + u < nsplit) {
+          const float *ps = p0 + (s + u) * sstride;
+          vr[u] = __ldg(ps + c * 128 + r);
+          vi[u] = __ldg(ps + (128 + c) * 128 + r);
+          if (diag) vt[u] = __ldg(ps + (128 + r) * 128 + c);
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (s + u < nsplit) {
+          re.add(vr[u]);
+          im.add(vi[u]);
+          if (diag) imt.add(vt[u]);
+        }
     }
     const double wi = diag ? im.value() - imt.value() : im.value();
     const double vi = m == n ? 0.0 : (conj ? -wi : wi) * vscale;  // one-feed autos are real
@@ -951,10 +935,10 @@ static int reduce_impl(const char *who, const void *ws, size_t ws_bytes, int ngr
   const float *part = static_cast<const float *>(ws);
   cudaStream_t s = as_stream(stream);
   if (!pairs) {
-    const dim3 grid((unsigned)(n_tiles * kRedGroups), (unsigned)ngroup);
-#define MVB_RED(OT, FF_)                                                                                    \
-  herk_reduce_all_kernel<OT, FF_><<<grid, 256, 0, s>>>(part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap, \
-                                                       k_chunk, nsm, nant, out, out_stride, vscale, accumulate)
+    const dim3 grid((unsigned)(n_tiles * kRedBlocks), (unsigned)ngroup);
+#define MVB_RED(OT, FF_)                                                                                           \
+  herk_reduce_all_kernel<OT, FF_><<<grid, kRedThreads, 0, s>>>(part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap, \
+                                                               k_chunk, nsm, nant, out, out_stride, vscale, accumulate)
     if (out_c128) {
       if (nfeed == 2) MVB_RED(double2, 2); else MVB_RED(double2, 1);
     } else {
