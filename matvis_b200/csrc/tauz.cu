@@ -18,6 +18,9 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
 
 namespace mvb {
@@ -204,111 +207,298 @@ struct PanelWriter {
   }
 };
 
-// CTA = 128 threads over 32 sources x 64 antennas: thread bits 0..2 pick a group
-// of 4 consecutive sources (16-byte stores per plane at X = 2), bits 3..6 one of
-// 16 antenna lanes, each lane taking every 16th antenna of the block.  A CTA
-// thus writes only 4 k-blocks (X = 2) of 128 rows, so the Z lines it has open at
-// any time fit, summed over the resident CTAs, well inside L2 (a wider k-range
-// per CTA left partially written lines to be evicted); a warp's store writes 16
-// whole 32-byte sectors.  The CTA's beam values (nbeam * F * X x 32 sources)
-// are staged once in shared memory for its 16 antenna lanes.
+// ---------------------------------------------------------------------------
+// Fused writer.  CTA = 128 threads over 64 panel columns (32 sources at X = 2, 64
+// at X = 1) x 64 antennas x `per_z` frequencies: thread bits 0..2 pick a group of
+// 8 consecutive columns (16-byte stores per plane at 16 bits), bits 3..6 one of 16
+// antenna lanes, each lane taking every 16th antenna of the block.  A CTA writes 2
+// or 4 k-blocks of 128 rows per frequency, so the Z lines it has open at any time
+// fit, summed over the resident CTAs, well inside L2 (a wider k-range per CTA left
+// partially written lines to be evicted); a warp's store writes 16 whole 32-byte
+// sectors.
+// What bounds it: instructions.  Per (antenna, source, frequency) it needs the
+// phase reduction and sincos, F X complex products and their split and stores; the
+// path difference, the beam values and the offsets depend on (antenna, source)
+// only and stay in registers for the frequencies of the group, and what depends on
+// (source, frequency) only -- the flux, or a polarised sky's Cholesky factor -- is
+// staged once per CTA for its 16 antenna lanes.  fp16x3, 350 polarised antennas x
+// 98,304 sources x 8 frequencies: 1,390 us, 6.3 TB/s written (0.97 of the copy
+// rate), against 1,650 us with a frequency per CTA, which read the beam from shared
+// memory and formed the path difference for each; 512 unpolarised antennas x 30,001
+// sources x 8: 224 against 390 us (4.4 TB/s: instructions); 90 x 11,180 x 8: 23
+// against 32 us; polarised sky, 350 x 24,576 x 4: 194 against 321 us (every antenna
+// lane factored the coherency again).  The results are bit-identical.
+// ---------------------------------------------------------------------------
 constexpr int kTauZThreads = 128;
-constexpr int kTauZSrc = 4;                 // consecutive sources per thread
-constexpr int kTauZGroups = 8;              // source groups per CTA
+constexpr int kTauZCols = 8;                // consecutive columns per thread
+constexpr int kTauZGroups = 8;              // column groups per CTA
 constexpr int kTauZAntLanes = kTauZThreads / kTauZGroups;
 constexpr int kTauZAnts = 64;               // antennas per CTA
-constexpr int kTauZBlockSrc = kTauZGroups * kTauZSrc;
-constexpr int kTauZRow = kTauZBlockSrc + 1;  // staged beam values per q, padded
-constexpr int kTauZMaxBFX = 16;              // beam planes staged in shared memory, else read through L1
+constexpr int kTauZMaxBFX = 16;             // beam planes staged in shared memory, else read through L1
+constexpr int kTauZMaxFreq = 8;             // frequencies per CTA
+constexpr int kTauZCtasPerSm = 8;           // CTAs per SM that a small launch is cut into
+constexpr int kTauZBeamRow = kTauZCols * kTauZGroups;  // staged values of one (beam, feed)
 
-// grid.x: blocks of kTauZBlockSrc sources, grid.y: blocks of kTauZAnts antennas,
-// grid.z: the frequencies of a grouped launch (freqs != nullptr): frequency
-// freqs[z], fluxes sflux + z sflux_ld (coh + z coh_ld), panel z + z zstride bytes.
-// EXT = 0: phase from antpos . crd (fused tau); EXT = 1 / 2: phase factor read
-// from a caller exptau (A, e_ld) in complex64 / complex128, multiplied by sflux.
-// POL (EXT = 0, X = 2): polarised sky.  Instead of sqrt(0.5 I) the source
-// carries its coherency C (coh[sidx[s]] = C00, C11, Re C01, Im C01 at this
-// frequency) and frame rotation R (rot[s] = cos X, sin X); with C' = R^T C R =
-// L L^H (lower-triangular L), Z[a, f, (s, y)] = exptau(a, s) sum_x
-// beam[f, x, s] L[x, y, s], so that Z Z^H gives exptau_j conj(exptau_i)
-// E_j C' E_i^H per source.
-template <int MODE, int X, int EXT = 0, bool STAGED = true, bool POL = false>
-__global__ void __launch_bounds__(kTauZThreads)
-    tau_z_kernel(const double *__restrict__ antpos, int A, double f_over_c, const double *__restrict__ crd, int64_t ld,
-                 const int32_t *__restrict__ n_dev, int64_t nsrc, const float *__restrict__ sflux,
-                 const int32_t *__restrict__ sidx, const float2 *__restrict__ beam, int64_t beam_ld, int nbeam,
-                 const int32_t *__restrict__ beam_idx, int F, float zscale, void *__restrict__ z, int64_t Mpad,
-                 int64_t Kcap, const void *__restrict__ ext = nullptr, int64_t e_ld = 0,
-                 const float4 *__restrict__ coh = nullptr, const double2 *__restrict__ rot = nullptr,
-                 const double *__restrict__ freqs = nullptr, int64_t sflux_ld = 0, int64_t coh_ld = 0,
-                 int64_t zstride = 0) {
-  static_assert(!POL || (X == 2 && EXT == 0), "the polarised sky needs two beam axes and the fused phase");
-  if (freqs) {  // grouped: this block's frequency
-    const int gz = blockIdx.z;
-    f_over_c = freqs[gz] * kInvC;
-    if (sflux) sflux += gz * sflux_ld;
-    if (coh) coh += gz * coh_ld;
-    z = static_cast<uint8_t *>(z) + gz * zstride;
-  }
-  const int64_t n = n_dev ? min((int64_t)*n_dev, nsrc) : nsrc;
-  const int64_t s_end = round_up(n * X, kKAlign) / X;  // zero-fill up to here
-  const int64_t s0 = (int64_t)blockIdx.x * kTauZBlockSrc + (threadIdx.x % kTauZGroups) * kTauZSrc;
-  const int alane = threadIdx.x / kTauZGroups;
-  if ((int64_t)blockIdx.x * kTauZBlockSrc >= s_end) return;  // uniform per CTA
-  const bool write = s0 < s_end;  // s_end is a multiple of kTauZSrc (64 / X)
+// Resident CTAs per SM that the registers are held to (the best of 4, 5, 6, 8 and
+// no bound, by form: the polarised group form keeps 32 beam values a thread).
+constexpr int tau_z_min_blocks(int mode, int X, int F, bool group) {
+  return X * F == 4 ? (!group ? 6 : (mode == MVB_GEMM_TF32_3 ? 5 : 4)) : (X == 1 && F == 2 ? 5 : 6);
+}
 
-  double cx[kTauZSrc], cy[kTauZSrc], cz[kTauZSrc];
-  float sf[kTauZSrc];
-  float l00[POL ? kTauZSrc : 1], l10r[POL ? kTauZSrc : 1], l10i[POL ? kTauZSrc : 1], l11[POL ? kTauZSrc : 1];
+struct TauZArgs {
+  const double *antpos, *crd, *freqs;  // freqs: device array of the group, or null (f_over_c)
+  double f_over_c;
+  int64_t ld, nsrc, beam_ld, sflux_ld, coh_ld, zstride, Mpad, Kcap;
+  const int32_t *n_dev, *sidx, *beam_idx;
+  const float *sflux;
+  const float2 *beam;
+  const float4 *coh;
+  const double2 *rot;
+  void *z;
+  int A, ants, nbeam, nfreq, per_z;  // ants: antennas per CTA
+  float scale_beam, scale_flux;  // their product is the panel's power-of-two scale
+  bool staged;                   // the beam planes fit the shared-memory stage
+};
+
+// Lower-triangular L of C' = R^T C R = L L^H (clamped at the PSD boundary), for
+// the coherency c = (C00, C11, Re C01, Im C01) and R's (cos X, sin X).
+__device__ __forceinline__ float4 coherency_factor(float4 c, double2 r) {
+  const double cr = r.x, sr = r.y;
+  const double a = c.x, d = c.y, br = c.z, bi = c.w;
+  const double c00 = cr * cr * a + sr * sr * d - 2.0 * cr * sr * br;
+  const double c11 = sr * sr * a + cr * cr * d + 2.0 * cr * sr * br;
+  // C'_10 = conj(C'_01), C'_01 = cr sr (a - d) + cr^2 b - sr^2 conj(b)
+  const double c10r = cr * sr * (a - d) + (cr * cr - sr * sr) * br;
+  const double c10i = -(cr * cr + sr * sr) * bi;
+  const double L00 = sqrt(fmax(c00, 0.0));
+  const double L10r = L00 > 0.0 ? c10r / L00 : 0.0, L10i = L00 > 0.0 ? c10i / L00 : 0.0;
+  return make_float4((float)L00, (float)L10r, (float)L10i,
+                     (float)sqrt(fmax(c11 - L10r * L10r - L10i * L10i, 0.0)));
+}
+
+// POL: polarised sky.  Instead of sqrt(0.5 I) the source carries its coherency C
+// (coh[sidx[s]] at this frequency) and frame rotation R (rot[s] = cos X, sin X);
+// with C' = R^T C R = L L^H, Z[a, f, (s, y)] = exptau(a, s) sum_x beam[f, x, s]
+// L[x, y, s], so that Z Z^H gives exptau_j conj(exptau_i) E_j C' E_i^H per source.
+// grid.x: blocks of 64 columns, grid.y: blocks of kTauZAnts antennas, grid.z: per_z
+// frequencies each, frequency g: fluxes sflux + g sflux_ld (coh + g coh_ld), panel
+// z + g zstride bytes.
+template <int MODE, int X, int F, bool POL, bool GROUP>
+__global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GROUP)) tau_z_kernel(const __grid_constant__ TauZArgs p) {
+  static_assert(!POL || (X == 2 && F == 2), "the polarised sky needs two feeds and two beam axes");
+  constexpr int NS = kTauZCols / X;        // sources per thread
+  constexpr int BS = kTauZGroups * NS;     // sources per CTA
+  const int64_t n = p.n_dev ? min((int64_t)*p.n_dev, p.nsrc) : p.nsrc;
+  const int64_t s_end = round_up(n * X, kKAlign) / X;  // zero-fill up to here: a multiple of BS
+  const int64_t sb = (int64_t)blockIdx.x * BS;
+  if (sb >= s_end) return;  // uniform per CTA
+  const int g0 = blockIdx.z * p.per_z, gn = min(p.per_z, p.nfreq - g0);
+
+  __shared__ double crd_sm[3][BS], foc_sm[kTauZMaxFreq];
+  extern __shared__ float4 dyn_sm[];
+  // per (frequency, source): the flux, or the Cholesky factor; then the beam values
+  // [(beam, feed)][column pair][group][2]: a thread's pair of columns is 16 bytes
+  float *flux_sm = reinterpret_cast<float *>(dyn_sm);
+  float4 *fac_sm = dyn_sm;
+  float2 *beam_sm = reinterpret_cast<float2 *>(dyn_sm) + (POL ? 2 : 1) * (p.per_z * BS) / (POL ? 1 : 2);
+  // every load of the prologue is issued before the first value is stored: the
+  // CTA's start is one chain of loads (the flux behind its index), not four
+  constexpr int PER = kTauZThreads / BS;  // (frequencies, coordinates, beam planes) the threads cover at a time
+  const int sl = threadIdx.x % BS, lane0 = threadIdx.x / BS;
+  const int64_t s = sb + sl;
+  const bool live = s < n;
+  const int64_t src = live && p.sidx ? __ldg(p.sidx + s) : s;
+  constexpr int NC = (3 + PER - 1) / PER, NB = kTauZMaxBFX / PER, NG = kTauZMaxFreq / PER;
+  double c_in[NC];
 #pragma unroll
-  for (int j = 0; j < kTauZSrc; ++j) {
-    const int64_t s = s0 + j;
-    const bool live = s < n;
-    cx[j] = cy[j] = cz[j] = 0.0;
-    sf[j] = 0.f;
-    if (live) {
-      if (EXT == 0) {
-        cx[j] = crd[s];
-        cy[j] = crd[ld + s];
-        cz[j] = crd[2 * ld + s];
-      }
-      if constexpr (POL) {
-        // C' = R^T C R, then its Cholesky factor (clamped at the PSD boundary)
-        const float4 c = coh[sidx ? sidx[s] : s];
-        const double2 r = rot[s];
-        const double cr = r.x, sr = r.y;
-        const double a = c.x, d = c.y, br = c.z, bi = c.w;
-        const double c00 = cr * cr * a + sr * sr * d - 2.0 * cr * sr * br;
-        const double c11 = sr * sr * a + cr * cr * d + 2.0 * cr * sr * br;
-        // C'_10 = conj(C'_01), C'_01 = cr sr (a - d) + cr^2 b - sr^2 conj(b)
-        const double c10r = cr * sr * (a - d) + (cr * cr - sr * sr) * br;
-        const double c10i = -(cr * cr + sr * sr) * bi;
-        const double L00 = sqrt(fmax(c00, 0.0));
-        const double L10r = L00 > 0.0 ? c10r / L00 : 0.0, L10i = L00 > 0.0 ? c10i / L00 : 0.0;
-        l00[j] = (float)L00;
-        l10r[j] = (float)L10r;
-        l10i[j] = (float)L10i;
-        l11[j] = (float)sqrt(fmax(c11 - L10r * L10r - L10i * L10i, 0.0));
-        sf[j] = 1.f;
-      } else {
-        sf[j] = sflux[sidx ? sidx[s] : s];
-      }
-    } else if constexpr (POL) {
-      l00[j] = l10r[j] = l10i[j] = l11[j] = 0.f;
+  for (int i = 0; i < NC; ++i) c_in[i] = live && lane0 + i * PER < 3 ? __ldg(p.crd + (lane0 + i * PER) * p.ld + s) : 0.0;
+  const int nq = p.staged ? p.nbeam * F * X : 0;
+  float2 b_in[NB];
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+    b_in[i] = live && lane0 + i * PER < nq ? __ldg(p.beam + (int64_t)(lane0 + i * PER) * p.beam_ld + s)
+                                           : make_float2(0.f, 0.f);
+  if (threadIdx.x < gn) foc_sm[threadIdx.x] = p.freqs ? __ldg(p.freqs + g0 + threadIdx.x) * kInvC : p.f_over_c;
+  if constexpr (POL) {
+    const double2 rot = live ? __ldg(p.rot + s) : make_double2(0.0, 0.0);
+    for (int g = lane0; g < gn; g += PER) {
+      float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (live) l = coherency_factor(__ldg(p.coh + (g0 + g) * p.coh_ld + src), rot);
+      fac_sm[g * BS + sl] =
+          make_float4(l.x * p.scale_flux, l.y * p.scale_flux, l.z * p.scale_flux, l.w * p.scale_flux);
+    }
+  } else {
+    float f_in[NG];
+#pragma unroll
+    for (int i = 0; i < NG; ++i)
+      f_in[i] = live && lane0 + i * PER < gn ? __ldg(p.sflux + (g0 + lane0 + i * PER) * p.sflux_ld + src) : 0.f;
+#pragma unroll
+    for (int i = 0; i < NG; ++i)
+      if (lane0 + i * PER < gn) flux_sm[(lane0 + i * PER) * BS + sl] = f_in[i] * p.scale_flux;
+  }
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+    if (lane0 + i * PER < 3) crd_sm[lane0 + i * PER][sl] = c_in[i];
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    const int q = lane0 + i * PER;
+    if (q < nq) {
+      const int k = (sl % NS) * X + q % X;  // the thread's column
+      beam_sm[(q / X) * kTauZBeamRow + ((k >> 1) * kTauZGroups + sl / NS) * 2 + (k & 1)] =
+          make_float2(b_in[i].x * p.scale_beam, b_in[i].y * p.scale_beam);
     }
   }
-  // STAGED: the CTA's beam values, shared by its 16 antenna lanes, in shared
-  // memory as [q][j][group] with a row of 33 values per q (q = (beam * F + f) *
-  // X + x): the 8 source groups of a warp read 8 consecutive values, and lanes
-  // with different beams land on different banks.  Otherwise (more than 16 beam
-  // planes) the values are read through L1 per antenna.
+  __syncthreads();
+
+  const int sg = threadIdx.x % kTauZGroups, alane = threadIdx.x / kTauZGroups;
+  const int64_t k0 = (sb + sg * NS) * X;
+  const int a0 = blockIdx.y * p.ants, a1 = min(a0 + p.ants, p.A);
+  // one frequency: a thread's four sources' coordinates and fluxes stay in registers instead
+  constexpr bool KEEP = !GROUP && NS <= 4;
+  double cx[KEEP ? NS : 1], cy[KEEP ? NS : 1], cz[KEEP ? NS : 1];
+  float sf1[KEEP ? NS : 1];
+  if constexpr (KEEP) {
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+      cx[j] = crd_sm[0][sg * NS + j];
+      cy[j] = crd_sm[1][sg * NS + j];
+      cz[j] = crd_sm[2][sg * NS + j];
+      sf1[j] = POL ? 1.f : flux_sm[sg * NS + j];
+    }
+  }
+  for (int a = a0 + alane; a < a1; a += kTauZAntLanes) {
+    const int b = p.beam_idx ? __ldg(p.beam_idx + a) : 0;
+    const double dx = __ldg(p.antpos + 3 * a), dy = __ldg(p.antpos + 3 * a + 1), dz = __ldg(p.antpos + 3 * a + 2);
+    double path[NS];
+#pragma unroll
+    for (int j = 0; j < NS; ++j)
+      path[j] = KEEP ? dx * cx[KEEP ? j : 0] + dy * cy[KEEP ? j : 0] + dz * cz[KEEP ? j : 0]
+                     : dx * crd_sm[0][sg * NS + j] + dy * crd_sm[1][sg * NS + j] + dz * crd_sm[2][sg * NS + j];
+    float2 bv[GROUP ? F : 1][kTauZCols];
+    auto load_beam = [&](int f, float2(&v)[kTauZCols]) {
+      if (p.staged) {
+        const float4 *src = reinterpret_cast<const float4 *>(beam_sm + (b * F + f) * kTauZBeamRow) + sg;
+#pragma unroll
+        for (int k = 0; k < kTauZCols; k += 2) {
+          const float4 v2 = src[(k >> 1) * kTauZGroups];
+          v[k] = make_float2(v2.x, v2.y);
+          v[k + 1] = make_float2(v2.z, v2.w);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < kTauZCols; ++k) {
+          const int64_t s = sb + sg * NS + k / X;
+          const float2 v1 = s < n ? __ldg(p.beam + (int64_t)((b * F + f) * X + k % X) * p.beam_ld + s)
+                                  : make_float2(0.f, 0.f);
+          v[k] = make_float2(v1.x * p.scale_beam, v1.y * p.scale_beam);
+        }
+      }
+    };
+    if constexpr (GROUP) {
+#pragma unroll
+      for (int f = 0; f < F; ++f) load_beam(f, bv[f]);
+    }
+#pragma unroll 1
+    for (int g = 0; g < (GROUP ? gn : 1); ++g) {
+      const double foc = foc_sm[g];
+      float er[NS], ei[NS];
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        const double t = path[j] * foc;
+        const double r = t - round_half_even(t);
+        float sn, cs;
+        sincospif(2.f * (float)r, &sn, &cs);
+        if constexpr (POL) {
+          er[j] = cs;
+          ei[j] = sn;
+        } else {
+          const float sf = KEEP ? sf1[KEEP ? j : 0] : flux_sm[g * BS + sg * NS + j];
+          er[j] = cs * sf;
+          ei[j] = sn * sf;
+        }
+      }
+      uint8_t *zg = static_cast<uint8_t *>(p.z) + (g0 + g) * p.zstride;
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        float vr[kTauZCols], vi[kTauZCols];
+        if constexpr (!GROUP) load_beam(f, bv[0]);
+#pragma unroll
+        for (int k = 0; k < kTauZCols; ++k) {
+          const float2 v = bv[GROUP ? f : 0][k];
+          vr[k] = er[k / X] * v.x - ei[k / X] * v.y;
+          vi[k] = er[k / X] * v.y + ei[k / X] * v.x;
+        }
+        if constexpr (POL) {
+          // (g0, g1) = exptau * beam[f, 0:2]  ->  (g0 L00 + g1 L10, g1 L11)
+#pragma unroll
+          for (int j = 0; j < NS; ++j) {
+            const float4 l = fac_sm[g * BS + sg * NS + j];
+            const float g0r = vr[2 * j], g0i = vi[2 * j], g1r = vr[2 * j + 1], g1i = vi[2 * j + 1];
+            vr[2 * j] = fmaf(-g1i, l.z, fmaf(g0r, l.x, g1r * l.y));
+            vi[2 * j] = fmaf(g1i, l.y, fmaf(g1r, l.z, g0i * l.x));
+            vr[2 * j + 1] = g1r * l.w;
+            vi[2 * j + 1] = g1i * l.w;
+          }
+        }
+        const int64_t m = (int64_t)a * F + f;
+        if constexpr (MODE == MVB_Z_C64) {
+          // the row's 8 values start 64-byte aligned (Kcap a multiple of 64): whole
+          // 32-byte sectors, four values each
+          float2 *zp = reinterpret_cast<float2 *>(zg) + m * p.Kcap + k0;
+#pragma unroll
+          for (int i = 0; i < kTauZCols; i += 4) {
+            const uint32_t w[8] = {__float_as_uint(vr[i]),     __float_as_uint(vi[i]),     __float_as_uint(vr[i + 1]),
+                                   __float_as_uint(vi[i + 1]), __float_as_uint(vr[i + 2]), __float_as_uint(vi[i + 2]),
+                                   __float_as_uint(vr[i + 3]), __float_as_uint(vi[i + 3])};
+            store_sector(zp + i, w);
+          }
+        } else {
+          // 8 consecutive k from a multiple of 8: inside one k-block
+          constexpr int KB = kKBlockBytes / (MODE == MVB_GEMM_TF32_3 ? 4 : 2);
+          constexpr int NPL = MODE == MVB_GEMM_BF16_6 ? 6 : 4;
+          const int64_t off = panel_off(m, k0, p.Mpad, KB, NPL);
+          const int64_t off2 = panel_off(m, k0 + kTauZCols / 2, p.Mpad, KB, NPL);
+          put_split<MODE, kTauZCols>(zg, panel_plane_stride(KB), off, off2, 0, vr, 1.f);
+          put_split<MODE, kTauZCols>(zg, panel_plane_stride(KB), off, off2, 1, vi, 1.f);
+        }
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Z from a caller's exptau (A, e_ld), complex64 (EXT = 1) or complex128 (EXT = 2):
+// 32 sources x 64 antennas per CTA, four consecutive sources per thread.  The
+// CTA's beam values are staged in shared memory for its 16 antenna lanes (or read
+// through L1 beyond kTauZMaxBFX planes).
+// ---------------------------------------------------------------------------
+constexpr int kZExtSrc = 4;
+constexpr int kZExtBlockSrc = kTauZGroups * kZExtSrc;
+constexpr int kZExtRow = kZExtBlockSrc + 1;  // staged beam values per q, padded
+
+template <int MODE, int X, int EXT, bool STAGED>
+__global__ void __launch_bounds__(kTauZThreads)
+    z_exptau_kernel(const void *__restrict__ ext, int64_t e_ld, int A, int64_t n, const float *__restrict__ sflux,
+                    const float2 *__restrict__ beam, int64_t beam_ld, int nbeam, const int32_t *__restrict__ beam_idx,
+                    int F, float zscale, void *__restrict__ z, int64_t Mpad, int64_t Kcap) {
+  const int64_t s_end = round_up(n * X, kKAlign) / X;  // zero-fill up to here
+  const int64_t s0 = (int64_t)blockIdx.x * kZExtBlockSrc + (threadIdx.x % kTauZGroups) * kZExtSrc;
+  const int alane = threadIdx.x / kTauZGroups;
+  if ((int64_t)blockIdx.x * kZExtBlockSrc >= s_end) return;  // uniform per CTA
+  const bool write = s0 < s_end;  // s_end is a multiple of kZExtSrc (64 / X)
+  float sf[kZExtSrc];
+#pragma unroll
+  for (int j = 0; j < kZExtSrc; ++j) sf[j] = s0 + j < n ? sflux[s0 + j] : 0.f;
+  // staged as [q][j][group], rows of 33 values (q = (beam * F + f) * X + x): the 8
+  // source groups of a warp read 8 consecutive values, and lanes with different
+  // beams land on different banks
   extern __shared__ float2 bsm[];
   if constexpr (STAGED) {
     const int nq = nbeam * F * X;
-    for (int e = threadIdx.x; e < nq * kTauZBlockSrc; e += kTauZThreads) {
-      const int q = e / kTauZBlockSrc, sl = e % kTauZBlockSrc;  // sl = group * kTauZSrc + j
-      const int64_t ss = (int64_t)blockIdx.x * kTauZBlockSrc + sl;
-      bsm[q * kTauZRow + (sl % kTauZSrc) * kTauZGroups + sl / kTauZSrc] =
+    for (int e = threadIdx.x; e < nq * kZExtBlockSrc; e += kTauZThreads) {
+      const int q = e / kZExtBlockSrc, sl = e % kZExtBlockSrc;  // sl = group * kZExtSrc + j
+      const int64_t ss = (int64_t)blockIdx.x * kZExtBlockSrc + sl;
+      bsm[q * kZExtRow + (sl % kZExtSrc) * kTauZGroups + sl / kZExtSrc] =
           ss < n ? __ldg(beam + (int64_t)q * beam_ld + ss) : make_float2(0.f, 0.f);
     }
     __syncthreads();
@@ -316,87 +506,61 @@ __global__ void __launch_bounds__(kTauZThreads)
   const int sg = threadIdx.x % kTauZGroups;
   const int a0 = blockIdx.y * kTauZAnts;
   const int a1 = min(a0 + kTauZAnts, A);
-  {
-    for (int a = a0 + alane; a < a1; a += kTauZAntLanes) {
-      const int b = beam_idx ? beam_idx[a] : 0;
-      float er[kTauZSrc], ei[kTauZSrc];
-      double dx = 0, dy = 0, dz = 0;
-      if (EXT == 0) {
-        dx = antpos[3 * a];
-        dy = antpos[3 * a + 1];
-        dz = antpos[3 * a + 2];
+  for (int a = a0 + alane; a < a1; a += kTauZAntLanes) {
+    const int b = beam_idx ? beam_idx[a] : 0;
+    float er[kZExtSrc], ei[kZExtSrc];
+#pragma unroll
+    for (int j = 0; j < kZExtSrc; ++j) {
+      er[j] = ei[j] = 0.f;
+      if (s0 + j >= n) continue;
+      if (EXT == 1) {
+        const float2 e = static_cast<const float2 *>(ext)[(int64_t)a * e_ld + s0 + j];
+        er[j] = e.x * sf[j];
+        ei[j] = e.y * sf[j];
+      } else {
+        const double2 e = static_cast<const double2 *>(ext)[(int64_t)a * e_ld + s0 + j];
+        er[j] = (float)(e.x * (double)sf[j]);
+        ei[j] = (float)(e.y * (double)sf[j]);
       }
+    }
 #pragma unroll
-      for (int j = 0; j < kTauZSrc; ++j) {
-        er[j] = ei[j] = 0.f;
-        if (s0 + j >= n) continue;
-        if (EXT == 1) {
-          const float2 e = static_cast<const float2 *>(ext)[(int64_t)a * e_ld + s0 + j];
-          er[j] = e.x * sf[j];
-          ei[j] = e.y * sf[j];
-        } else if (EXT == 2) {
-          const double2 e = static_cast<const double2 *>(ext)[(int64_t)a * e_ld + s0 + j];
-          er[j] = (float)(e.x * (double)sf[j]);
-          ei[j] = (float)(e.y * (double)sf[j]);
-        } else {
-          const double t = (dx * cx[j] + dy * cy[j] + dz * cz[j]) * f_over_c;
-          const double r = t - round_half_even(t);
-          float sn, cs;
-          sincospif((float)(2.0 * r), &sn, &cs);
-          er[j] = cs * sf[j];
-          ei[j] = sn * sf[j];
+    for (int f = 0; f < 2; ++f) {
+      if (f >= F) break;
+      float vr[kZExtSrc * X], vi[kZExtSrc * X];
+#pragma unroll
+      for (int j = 0; j < kZExtSrc; ++j)
+#pragma unroll
+        for (int x = 0; x < X; ++x) {
+          const int q = (b * F + f) * X + x;
+          float2 bv;
+          if constexpr (STAGED)
+            bv = bsm[q * kZExtRow + j * kTauZGroups + sg];
+          else
+            bv = (s0 + j < n) ? __ldg(beam + (int64_t)q * beam_ld + s0 + j) : make_float2(0.f, 0.f);
+          vr[j * X + x] = er[j] * bv.x - ei[j] * bv.y;
+          vi[j * X + x] = er[j] * bv.y + ei[j] * bv.x;
         }
-      }
+      if (!write) continue;
+      const int64_t m = (int64_t)a * F + f;
+      if constexpr (MODE == MVB_Z_C64) {
+        // the row's kZExtSrc * X values start 32-byte aligned (Kcap a multiple
+        // of 64, s0 X of 4): whole 32-byte sectors, four values each
+        float2 *zp = static_cast<float2 *>(z) + m * Kcap + s0 * X;
 #pragma unroll
-      for (int f = 0; f < 2; ++f) {
-        if (f >= F) break;
-        float vr[kTauZSrc * X], vi[kTauZSrc * X];
-#pragma unroll
-        for (int j = 0; j < kTauZSrc; ++j)
-#pragma unroll
-          for (int x = 0; x < X; ++x) {
-            const int q = (b * F + f) * X + x;
-            float2 bv;
-            if constexpr (STAGED)
-              bv = bsm[q * kTauZRow + j * kTauZGroups + sg];
-            else
-              bv = (s0 + j < n) ? __ldg(beam + (int64_t)q * beam_ld + s0 + j) : make_float2(0.f, 0.f);
-            vr[j * X + x] = er[j] * bv.x - ei[j] * bv.y;
-            vi[j * X + x] = er[j] * bv.y + ei[j] * bv.x;
-          }
-        if constexpr (POL) {
-          // (g0, g1) = exptau * beam[f, 0:2]  ->  (g0 L00 + g1 L10, g1 L11)
-#pragma unroll
-          for (int j = 0; j < kTauZSrc; ++j) {
-            const float g0r = vr[2 * j], g0i = vi[2 * j], g1r = vr[2 * j + 1], g1i = vi[2 * j + 1];
-            vr[2 * j] = g0r * l00[j] + g1r * l10r[j] - g1i * l10i[j];
-            vi[2 * j] = g0i * l00[j] + g1r * l10i[j] + g1i * l10r[j];
-            vr[2 * j + 1] = g1r * l11[j];
-            vi[2 * j + 1] = g1i * l11[j];
-          }
+        for (int i = 0; i < kZExtSrc * X; i += 4) {
+          const uint32_t w[8] = {__float_as_uint(vr[i]),     __float_as_uint(vi[i]),     __float_as_uint(vr[i + 1]),
+                                 __float_as_uint(vi[i + 1]), __float_as_uint(vr[i + 2]), __float_as_uint(vi[i + 2]),
+                                 __float_as_uint(vr[i + 3]), __float_as_uint(vi[i + 3])};
+          store_sector(zp + i, w);
         }
-        if (!write) continue;
-        const int64_t m = (int64_t)a * F + f;
-        if constexpr (MODE == MVB_Z_C64) {
-          // the row's kTauZSrc * X values start 32-byte aligned (Kcap a multiple
-          // of 64, s0 X of 4): whole 32-byte sectors, four values each
-          float2 *zp = static_cast<float2 *>(z) + m * Kcap + s0 * X;
-#pragma unroll
-          for (int i = 0; i < kTauZSrc * X; i += 4) {
-            const uint32_t w[8] = {__float_as_uint(vr[i]),     __float_as_uint(vi[i]),     __float_as_uint(vr[i + 1]),
-                                   __float_as_uint(vi[i + 1]), __float_as_uint(vr[i + 2]), __float_as_uint(vi[i + 2]),
-                                   __float_as_uint(vr[i + 3]), __float_as_uint(vi[i + 3])};
-            store_sector(zp + i, w);
-          }
-        } else {
-          // kTauZSrc * X consecutive k from a multiple of kTauZSrc * X: inside one k-block
-          constexpr int KB = kKBlockBytes / (MODE == MVB_GEMM_TF32_3 ? 4 : 2);
-          constexpr int NPL = MODE == MVB_GEMM_BF16_6 ? 6 : 4;
-          const int64_t off = panel_off(m, s0 * X, Mpad, KB, NPL);
-          const int64_t off2 = panel_off(m, s0 * X + kTauZSrc * X / 2, Mpad, KB, NPL);
-          put_split<MODE, kTauZSrc * X>(z, panel_plane_stride(KB), off, off2, 0, vr, zscale);
-          put_split<MODE, kTauZSrc * X>(z, panel_plane_stride(KB), off, off2, 1, vi, zscale);
-        }
+      } else {
+        // kZExtSrc * X consecutive k from a multiple of kZExtSrc * X: inside one k-block
+        constexpr int KB = kKBlockBytes / (MODE == MVB_GEMM_TF32_3 ? 4 : 2);
+        constexpr int NPL = MODE == MVB_GEMM_BF16_6 ? 6 : 4;
+        const int64_t off = panel_off(m, s0 * X, Mpad, KB, NPL);
+        const int64_t off2 = panel_off(m, s0 * X + kZExtSrc * X / 2, Mpad, KB, NPL);
+        put_split<MODE, kZExtSrc * X>(z, panel_plane_stride(KB), off, off2, 0, vr, zscale);
+        put_split<MODE, kZExtSrc * X>(z, panel_plane_stride(KB), off, off2, 1, vi, zscale);
       }
     }
   }
@@ -508,6 +672,99 @@ extern "C" int mvb_exptau(const double *antpos, int A, double freq, const double
   return check_launch("exptau_kernel");
 }
 
+template <int MODE, bool POL, bool GROUP>
+static void launch_tau_z_form(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
+  if constexpr (POL) {
+    tau_z_kernel<MODE, 2, 2, true, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+  } else if (X == 2) {
+    if (F == 2)
+      tau_z_kernel<MODE, 2, 2, false, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+    else
+      tau_z_kernel<MODE, 2, 1, false, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+  } else {
+    if (F == 2)
+      tau_z_kernel<MODE, 1, 2, false, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+    else
+      tau_z_kernel<MODE, 1, 1, false, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+  }
+}
+
+template <int MODE, bool POL>
+static void launch_tau_z_mode(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
+  if (p.per_z > 1)
+    launch_tau_z_form<MODE, POL, true>(p, F, X, grid, smem, s);
+  else
+    launch_tau_z_form<MODE, POL, false>(p, F, X, grid, smem, s);
+}
+
+// The launch of both fused writers (arguments checked by the callers).
+template <bool POL>
+static int launch_tau_z(TauZArgs p, const double *antpos, int A, double freq, const double *freqs_dev, int nfreq,
+                        const double *crd, int64_t ld, const int32_t *n_dev, int64_t nsrc, const int32_t *sidx,
+                        const void *beam, int64_t beam_ld, int nbeam, const int32_t *beam_idx, int F, int X, int mode,
+                        float zscale, void *z, int64_t z_stride, int64_t Mpad, int64_t Kcap, void *stream) {
+  const int64_t cols = round_up(nsrc * X, kKAlign);
+  if (cols == 0) return MVB_OK;
+  p.antpos = antpos;
+  p.crd = crd;
+  p.freqs = freqs_dev;
+  p.f_over_c = freq * kInvC;
+  p.ld = ld;
+  p.nsrc = nsrc;
+  p.beam_ld = beam_ld;
+  p.zstride = z_stride;
+  p.Mpad = Mpad;
+  p.Kcap = Kcap;
+  p.n_dev = n_dev;
+  p.sidx = sidx;
+  p.beam_idx = beam_idx;
+  p.beam = static_cast<const float2 *>(beam);
+  p.z = z;
+  p.A = A;
+  p.nbeam = nbeam;
+  p.nfreq = nfreq;
+  // the fp16 panel's power-of-two scale, half of its exponent on the beam and half
+  // on the flux (exact, and neither leaves the range of FP32)
+  p.scale_beam = p.scale_flux = 1.f;
+  if (mode == MVB_GEMM_F16_3) {
+    int e;
+    const bool pow2 = std::isfinite(zscale) && std::frexp(zscale, &e) == 0.5f;
+    p.scale_beam = !pow2 ? zscale : std::ldexp(1.f, (e - 1) / 2);
+    p.scale_flux = !pow2 ? 1.f : std::ldexp(1.f, (e - 1) - (e - 1) / 2);
+  }
+  const int nq = nbeam * F * X;
+  p.staged = nq <= kTauZMaxBFX;
+  // A CTA's share in units of (16 antennas x one frequency of its columns): all 8
+  // frequencies of 64 antennas in a large launch, less where that leaves fewer than 8
+  // CTAs per SM (about half of a sky's slots are below the horizon), frequencies
+  // before antennas, since they share more.  Measured with 4 / 8 / 12 / 16 CTAs per
+  // SM: 90 unpolarised antennas x 11,180 sources x 8 frequencies 25.8 / 22.7 / 22.6 /
+  // 25.4 us, 37 polarised x 2,501 x 7 7.8 / 8.5 / 9.9 / 9.8, 256 unpolarised x 3,000 x
+  // 8 22.4 / 17.7 / 20.3 / 20.2; larger ones within 1 %.
+  const int64_t xblocks = cols / (kTauZCols * kTauZGroups);
+  const int64_t units = xblocks * ceil_div(A, kTauZAntLanes) * nfreq;
+  const int64_t share = std::max<int64_t>(1, units / ((int64_t)num_sms() * kTauZCtasPerSm));
+  const int64_t parts = ceil_div(nfreq, std::min<int64_t>({share, (int64_t)kTauZMaxFreq, (int64_t)nfreq}));
+  p.per_z = (int)ceil_div(nfreq, parts);
+  const int64_t lanes = std::min<int64_t>(std::max<int64_t>(share / p.per_z, 1), kTauZAnts / kTauZAntLanes);
+  const int64_t ablocks = ceil_div(A, lanes * kTauZAntLanes);
+  p.ants = (int)round_up(ceil_div(A, ablocks), kTauZAntLanes);  // even shares, whole lanes
+  const dim3 grid((unsigned)(cols / (kTauZCols * kTauZGroups)), (unsigned)ceil_div(A, p.ants),
+                  (unsigned)ceil_div(nfreq, p.per_z));
+  const int bs = kTauZCols / X * kTauZGroups;
+  const size_t smem = (size_t)p.per_z * bs * (POL ? sizeof(float4) : sizeof(float)) +
+                      (p.staged ? (size_t)nbeam * F * kTauZBeamRow * sizeof(float2) : 0);
+  cudaStream_t s = as_stream(stream);
+  switch (mode) {
+    case MVB_GEMM_BF16_3: launch_tau_z_mode<MVB_GEMM_BF16_3, POL>(p, F, X, grid, smem, s); break;
+    case MVB_GEMM_BF16_6: launch_tau_z_mode<MVB_GEMM_BF16_6, POL>(p, F, X, grid, smem, s); break;
+    case MVB_GEMM_TF32_3: launch_tau_z_mode<MVB_GEMM_TF32_3, POL>(p, F, X, grid, smem, s); break;
+    case MVB_GEMM_F16_3: launch_tau_z_mode<MVB_GEMM_F16_3, POL>(p, F, X, grid, smem, s); break;
+    default: launch_tau_z_mode<MVB_Z_C64, POL>(p, F, X, grid, smem, s); break;
+  }
+  return check_launch("tau_z_kernel");
+}
+
 // Fused phase + Z writer for nfreq frequencies: freqs_dev == nullptr means one
 // frequency, freq; otherwise freqs_dev[0 .. nfreq) on the device, with the
 // fluxes sflux_ld floats and the panels z_stride bytes apart.
@@ -524,40 +781,11 @@ static int tau_z_impl(const char *who, const double *antpos, int A, double freq,
   if (round_up(nsrc * X, kKAlign) > Kcap) return fail(MVB_ERR_ARG, "%s: Kcap too small for nsrc * nax", who);
   if (nfreq > 1 && (sflux_ld < nsrc || z_stride < (int64_t)mvb_zpanel_bytes(mode, Mpad, Kcap) || z_stride % 16))
     return fail(MVB_ERR_ARG, "%s: flux rows or panels overlap", who);
-  const int64_t s_max = round_up(nsrc * X, kKAlign) / X;
-  if (s_max == 0) return MVB_OK;
-  dim3 grid((unsigned)ceil_div(s_max, kTauZBlockSrc), (unsigned)ceil_div(A, kTauZAnts), (unsigned)nfreq);
-  const bool staged = nbeam * F * X <= kTauZMaxBFX;
-  const size_t smem = staged ? (size_t)nbeam * F * X * kTauZRow * sizeof(float2) : 0;
-  const double foc = freq * kInvC;
-  const float2 *bm = static_cast<const float2 *>(beam);
-  cudaStream_t s = as_stream(stream);
-#define MVB_TAUZ(M, XX)                                                                                       \
-  do {                                                                                                        \
-    if (staged)                                                                                               \
-      tau_z_kernel<M, XX, 0, true, false><<<grid, kTauZThreads, smem, s>>>(                                   \
-          antpos, A, foc, crd, ld, n_dev, nsrc, sflux, sidx, bm, beam_ld, nbeam, beam_idx, F, zscale, z, Mpad, \
-          Kcap, nullptr, 0, nullptr, nullptr, freqs_dev, sflux_ld, 0, z_stride);                              \
-    else                                                                                                      \
-      tau_z_kernel<M, XX, 0, false, false><<<grid, kTauZThreads, 0, s>>>(                                     \
-          antpos, A, foc, crd, ld, n_dev, nsrc, sflux, sidx, bm, beam_ld, nbeam, beam_idx, F, zscale, z, Mpad, \
-          Kcap, nullptr, 0, nullptr, nullptr, freqs_dev, sflux_ld, 0, z_stride);                              \
-  } while (0)
-#define MVB_TAUZ2(M) \
-  if (X == 2)        \
-    MVB_TAUZ(M, 2);  \
-  else               \
-    MVB_TAUZ(M, 1)
-  switch (mode) {
-    case MVB_GEMM_BF16_3: MVB_TAUZ2(MVB_GEMM_BF16_3); break;
-    case MVB_GEMM_BF16_6: MVB_TAUZ2(MVB_GEMM_BF16_6); break;
-    case MVB_GEMM_TF32_3: MVB_TAUZ2(MVB_GEMM_TF32_3); break;
-    case MVB_GEMM_F16_3: MVB_TAUZ2(MVB_GEMM_F16_3); break;
-    default: MVB_TAUZ2(MVB_Z_C64); break;
-  }
-#undef MVB_TAUZ2
-#undef MVB_TAUZ
-  return check_launch("tau_z_kernel");
+  TauZArgs p{};
+  p.sflux = sflux;
+  p.sflux_ld = sflux_ld;
+  return launch_tau_z<false>(p, antpos, A, freq, freqs_dev, nfreq, crd, ld, n_dev, nsrc, sidx, beam, beam_ld, nbeam,
+                             beam_idx, F, X, mode, zscale, z, z_stride, Mpad, Kcap, stream);
 }
 
 extern "C" int mvb_tau_z(const double *antpos, int A, double freq, const double *crd, int64_t ld, const int32_t *n_dev,
@@ -625,36 +853,12 @@ static int tau_z_pol_impl(const char *who, const double *antpos, int A, double f
     return fail(MVB_ERR_ARG, "%s: coh and rot must be 16-byte aligned", who);
   if (nfreq > 1 && (coh_ld < nsrc || z_stride < (int64_t)mvb_zpanel_bytes(mode, Mpad, Kcap) || z_stride % 16))
     return fail(MVB_ERR_ARG, "%s: coherency rows or panels overlap", who);
-  const int64_t s_max = round_up(nsrc * X, kKAlign) / X;
-  if (s_max == 0) return MVB_OK;
-  dim3 grid((unsigned)ceil_div(s_max, kTauZBlockSrc), (unsigned)ceil_div(A, kTauZAnts), (unsigned)nfreq);
-  const bool staged = nbeam * F * X <= kTauZMaxBFX;
-  const size_t smem = staged ? (size_t)nbeam * F * X * kTauZRow * sizeof(float2) : 0;
-  const double foc = freq * kInvC;
-  const float2 *bm = static_cast<const float2 *>(beam);
-  const float4 *c4 = reinterpret_cast<const float4 *>(coh);
-  const double2 *r2 = reinterpret_cast<const double2 *>(rot);
-  cudaStream_t s = as_stream(stream);
-#define MVB_TZP(M)                                                                                                \
-  do {                                                                                                             \
-    if (staged)                                                                                                    \
-      tau_z_kernel<M, 2, 0, true, true><<<grid, kTauZThreads, smem, s>>>(antpos, A, foc, crd, ld, n_dev, nsrc,      \
-          nullptr, sidx, bm, beam_ld, nbeam, beam_idx, F, zscale, z, Mpad, Kcap, nullptr, 0, c4, r2, freqs_dev, 0,  \
-          coh_ld, z_stride);                                                                                       \
-    else                                                                                                           \
-      tau_z_kernel<M, 2, 0, false, true><<<grid, kTauZThreads, 0, s>>>(antpos, A, foc, crd, ld, n_dev, nsrc,        \
-          nullptr, sidx, bm, beam_ld, nbeam, beam_idx, F, zscale, z, Mpad, Kcap, nullptr, 0, c4, r2, freqs_dev, 0,  \
-          coh_ld, z_stride);                                                                                       \
-  } while (0)
-  switch (mode) {
-    case MVB_GEMM_BF16_3: MVB_TZP(MVB_GEMM_BF16_3); break;
-    case MVB_GEMM_BF16_6: MVB_TZP(MVB_GEMM_BF16_6); break;
-    case MVB_GEMM_TF32_3: MVB_TZP(MVB_GEMM_TF32_3); break;
-    case MVB_GEMM_F16_3: MVB_TZP(MVB_GEMM_F16_3); break;
-    default: MVB_TZP(MVB_Z_C64); break;
-  }
-#undef MVB_TZP
-  return check_launch("tau_z_kernel(pol)");
+  TauZArgs p{};
+  p.coh = reinterpret_cast<const float4 *>(coh);
+  p.coh_ld = coh_ld;
+  p.rot = reinterpret_cast<const double2 *>(rot);
+  return launch_tau_z<true>(p, antpos, A, freq, freqs_dev, nfreq, crd, ld, n_dev, nsrc, sidx, beam, beam_ld, nbeam,
+                            beam_idx, F, X, mode, zscale, z, z_stride, Mpad, Kcap, stream);
 }
 
 extern "C" int mvb_tau_z_pol(const double *antpos, int A, double freq, const double *crd, int64_t ld,
@@ -688,19 +892,19 @@ extern "C" int mvb_z_from_exptau(const void *exptau, int e_c128, int64_t e_ld, i
   if (round_up(nsrc * X, kKAlign) > Kcap) return fail(MVB_ERR_ARG, "mvb_z_from_exptau: Kcap too small");
   const int64_t s_max = round_up(nsrc * X, kKAlign) / X;
   if (s_max == 0) return MVB_OK;
-  dim3 grid((unsigned)ceil_div(s_max, kTauZBlockSrc), (unsigned)ceil_div(A, kTauZAnts));
+  dim3 grid((unsigned)ceil_div(s_max, kZExtBlockSrc), (unsigned)ceil_div(A, kTauZAnts));
   const bool staged = nbeam * F * X <= kTauZMaxBFX;
-  const size_t smem = staged ? (size_t)nbeam * F * X * kTauZRow * sizeof(float2) : 0;
+  const size_t smem = staged ? (size_t)nbeam * F * X * kZExtRow * sizeof(float2) : 0;
   const float2 *bm = static_cast<const float2 *>(beam);
   cudaStream_t s = as_stream(stream);
-#define MVB_ZX(M, XX, E)                                                                                      \
-  do {                                                                                                             \
-    if (staged)                                                                                                    \
-      tau_z_kernel<M, XX, E, true, false><<<grid, kTauZThreads, smem, s>>>(nullptr, A, 0.0, nullptr, 0, nullptr,    \
-          nsrc, sflux, nullptr, bm, beam_ld, nbeam, beam_idx, F, zscale, z, Mpad, Kcap, exptau, e_ld);              \
-    else                                                                                                           \
-      tau_z_kernel<M, XX, E, false, false><<<grid, kTauZThreads, 0, s>>>(nullptr, A, 0.0, nullptr, 0, nullptr,      \
-          nsrc, sflux, nullptr, bm, beam_ld, nbeam, beam_idx, F, zscale, z, Mpad, Kcap, exptau, e_ld);              \
+#define MVB_ZX(M, XX, E)                                                                                            \
+  do {                                                                                                              \
+    if (staged)                                                                                                     \
+      z_exptau_kernel<M, XX, E, true><<<grid, kTauZThreads, smem, s>>>(exptau, e_ld, A, nsrc, sflux, bm, beam_ld,    \
+                                                                       nbeam, beam_idx, F, zscale, z, Mpad, Kcap);  \
+    else                                                                                                            \
+      z_exptau_kernel<M, XX, E, false><<<grid, kTauZThreads, 0, s>>>(exptau, e_ld, A, nsrc, sflux, bm, beam_ld,     \
+                                                                     nbeam, beam_idx, F, zscale, z, Mpad, Kcap);    \
   } while (0)
 #define MVB_ZX3(M, E) \
   if (X == 2)         \
@@ -722,7 +926,7 @@ extern "C" int mvb_z_from_exptau(const void *exptau, int e_c128, int64_t e_ld, i
 #undef MVB_ZX2
 #undef MVB_ZX3
 #undef MVB_ZX
-  return check_launch("tau_z_kernel(exptau)");
+  return check_launch("z_exptau_kernel");
 }
 
 // sqrt(0.5 I) per source and frequency (cpu/cpu.py:188), transposed from the
