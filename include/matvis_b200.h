@@ -207,6 +207,13 @@ int mvb_z_pack(const void *zsrc, int z_c128, int64_t M, int64_t K, int64_t ldz, 
 /* max |z| over n complex values (complex64 or complex128) -> *out (device
  * float32, caller-zeroed); used to choose the MVB_GEMM_F16_3 scale. */
 int mvb_absmax(const void *z, int z_c128, int64_t n, float *out, void *stream);
+/* mvb_absmax and mvb_z_pack of a contiguous non-empty z (ldz = K) with the scale
+ * chosen on the device, so that the caller need not wait for the maximum:
+ * scale[0] = max |z|, scale[1] = the power of two s with max |s z| < 2^15 (1 for
+ * a zero or infinite z), which the panel holds z multiplied by.  scale: two
+ * device floats; scale + 1 goes to mvb_herk_reduce_scaled. */
+int mvb_z_pack_scaled(const void *zsrc, int z_c128, int64_t M, int64_t K, int64_t ldz, int mode, float *scale,
+                      void *z, int64_t Mpad, int64_t Kcap, void *stream);
 
 /* ---- A7: Hermitian product on the tensor cores ------------------------------ */
 /* In the entry points below the valid K extent of the panel is
@@ -291,6 +298,12 @@ int mvb_herk_batch(const mvb_herk_group *groups, int ngroups, int mode, int drai
 int mvb_herk_reduce(const void *ws, size_t ws_bytes, int64_t Mpad, int64_t Kcap, const int32_t *n_dev,
                     int64_t n_host, int kmul, int k_chunk, int nant, int nfeed, const int32_t *pairs, int64_t npairs,
                     void *out, int out_c128, double vscale, int accumulate, void *stream);
+/* mvb_herk_reduce with vscale = 1 / s^2 for the panel scale s = *zscale (a device
+ * float, as mvb_z_pack_scaled leaves it). */
+int mvb_herk_reduce_scaled(const void *ws, size_t ws_bytes, int64_t Mpad, int64_t Kcap, const int32_t *n_dev,
+                           int64_t n_host, int kmul, int k_chunk, int nant, int nfeed, const int32_t *pairs,
+                           int64_t npairs, void *out, int out_c128, const float *zscale, int accumulate,
+                           void *stream);
 /* mvb_herk_reduce for the ngroup panels of one mvb_herk_grouped call (same
  * ws, ngroup and shape arguments): panel g's visibilities go to
  * out + g * out_stride bytes. */

@@ -85,6 +85,7 @@ _SIGNATURES = {
          c_int64, _p],
     ),
     "mvb_z_pack": (c_int, [_p, c_int, c_int64, c_int64, c_int64, c_int, c_float, _p, c_int64, c_int64, _p]),
+    "mvb_z_pack_scaled": (c_int, [_p, c_int, c_int64, c_int64, c_int64, c_int, _p, _p, c_int64, c_int64, _p]),
     "mvb_absmax": (c_int, [_p, c_int, c_int64, _p, _p]),
     "mvb_herk_ws_bytes": (c_size_t, [c_int64, c_int64, c_int]),
     "mvb_herk": (c_int, [_p, c_int, c_int64, c_int64, _p, c_int64, c_int, c_int, c_int, _p, c_size_t, _p, _p]),
@@ -92,6 +93,10 @@ _SIGNATURES = {
         c_int,
         [_p, c_size_t, c_int64, c_int64, _p, c_int64, c_int, c_int, c_int, c_int, _p, c_int64, _p, c_int, c_double,
          c_int, _p],
+    ),
+    "mvb_herk_reduce_scaled": (
+        c_int,
+        [_p, c_size_t, c_int64, c_int64, _p, c_int64, c_int, c_int, c_int, c_int, _p, c_int64, _p, c_int, _p, c_int, _p],
     ),
     "mvb_set_wait_limit_ns": (ctypes.c_uint64, [ctypes.c_uint64]),
     "mvb_herk_grouped": (c_int, [_p, c_size_t, c_int, c_int, c_int64, c_int64, _p, c_int64, c_int, c_int, c_int, _p,

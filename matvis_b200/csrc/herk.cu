@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(kRedThreads, 2)
     herk_reduce_all_kernel(const float *__restrict__ part, int ngroup, int T, int n_tiles,
                            const int32_t *__restrict__ n_dev, int64_t n_host, int kmul, int64_t Kcap, int k_chunk,
                            int nsm, int A, void *__restrict__ out_base, int64_t out_stride, double vscale,
-                           int accumulate) {
+                           const float *__restrict__ zscale, int accumulate) {
   __shared__ FF turn_sm[32][33];
   const int t = blockIdx.x / kRedBlocks, rb = blockIdx.x % 4, cb = blockIdx.x / 4 % 4;
   int I, J;
@@ -678,6 +678,7 @@ __global__ void __launch_bounds__(kRedThreads, 2)
   int nsplit;
   int64_t kc;
   plan_splits(kvalid, n_tiles * ngroup, k_chunk, nsm, nsplit, kc);
+  if (zscale) vscale = 1.0 / ((double)*zscale * (double)*zscale);
   void *out = static_cast<uint8_t *>(out_base) + (int64_t)blockIdx.y * out_stride;
   part += (size_t)blockIdx.y * nsplit * n_tiles * (256 * 128);
   const int cc = threadIdx.x >> 3, rr = 4 * (threadIdx.x & 7);  // column and first row within the block
@@ -732,12 +733,13 @@ __global__ void herk_reduce_pairs_kernel(const float *__restrict__ part, int ngr
                                          const int32_t *__restrict__ n_dev, int64_t n_host, int kmul, int64_t Kcap,
                                          int k_chunk, int nsm, int A, int F, const int32_t *__restrict__ pairs,
                                          int64_t npairs, void *__restrict__ out_base, int64_t out_stride,
-                                         double vscale, int accumulate) {
+                                         double vscale, const float *__restrict__ zscale, int accumulate) {
   const int64_t total = npairs * F * F;
   const int64_t kvalid = valid_k(n_dev, n_host, kmul, Kcap);
   int nsplit;
   int64_t kc;
   plan_splits(kvalid, n_tiles * ngroup, k_chunk, nsm, nsplit, kc);
+  if (zscale) vscale = 1.0 / ((double)*zscale * (double)*zscale);
   void *out = static_cast<uint8_t *>(out_base) + (int64_t)blockIdx.y * out_stride;
   part += (size_t)blockIdx.y * nsplit * n_tiles * (256 * 128);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -917,7 +919,7 @@ static int herk_impl(const char *who, const void *z, int64_t zstride, int ngroup
 static int reduce_impl(const char *who, const void *ws, size_t ws_bytes, int ngroup, int64_t Mpad, int64_t Kcap,
                        const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int nant, int nfeed,
                        const int32_t *pairs, int64_t npairs, void *out, int64_t out_stride, int out_c128,
-                       double vscale, int accumulate, void *stream) {
+                       double vscale, const float *zscale, int accumulate, void *stream) {
   // the checks of mvb_herk: the slice plan recomputed here is then the product's
   if (!ws || !out || nant <= 0 || (nfeed != 1 && nfeed != 2) || (int64_t)nant * nfeed > Mpad || (pairs && npairs < 0))
     return fail(MVB_ERR_ARG, "%s: bad arguments", who);
@@ -938,7 +940,8 @@ static int reduce_impl(const char *who, const void *ws, size_t ws_bytes, int ngr
     const dim3 grid((unsigned)(n_tiles * kRedBlocks), (unsigned)ngroup);
 #define MVB_RED(OT, FF_)                                                                                           \
   herk_reduce_all_kernel<OT, FF_><<<grid, kRedThreads, 0, s>>>(part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap, \
-                                                               k_chunk, nsm, nant, out, out_stride, vscale, accumulate)
+                                                               k_chunk, nsm, nant, out, out_stride, vscale, zscale, \
+                                                               accumulate)
     if (out_c128) {
       if (nfeed == 2) MVB_RED(double2, 2); else MVB_RED(double2, 1);
     } else {
@@ -952,11 +955,11 @@ static int reduce_impl(const char *who, const void *ws, size_t ws_bytes, int ngr
     if (out_c128)
       herk_reduce_pairs_kernel<double2><<<grid, 256, 0, s>>>(part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap,
                                                              k_chunk, nsm, nant, nfeed, pairs, npairs, out, out_stride,
-                                                             vscale, accumulate);
+                                                             vscale, zscale, accumulate);
     else
       herk_reduce_pairs_kernel<float2><<<grid, 256, 0, s>>>(part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap,
                                                             k_chunk, nsm, nant, nfeed, pairs, npairs, out, out_stride,
-                                                            vscale, accumulate);
+                                                            vscale, zscale, accumulate);
   }
   return check_launch(who);
 }
@@ -1027,7 +1030,16 @@ extern "C" int mvb_herk_reduce(const void *ws, size_t ws_bytes, int64_t Mpad, in
                                int64_t n_host, int kmul, int k_chunk, int nant, int nfeed, const int32_t *pairs,
                                int64_t npairs, void *out, int out_c128, double vscale, int accumulate, void *stream) {
   return reduce_impl("mvb_herk_reduce", ws, ws_bytes, 1, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, nant, nfeed, pairs,
-                     npairs, out, 0, out_c128, vscale, accumulate, stream);
+                     npairs, out, 0, out_c128, vscale, nullptr, accumulate, stream);
+}
+
+extern "C" int mvb_herk_reduce_scaled(const void *ws, size_t ws_bytes, int64_t Mpad, int64_t Kcap,
+                                      const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int nant, int nfeed,
+                                      const int32_t *pairs, int64_t npairs, void *out, int out_c128,
+                                      const float *zscale, int accumulate, void *stream) {
+  if (!zscale) return fail(MVB_ERR_ARG, "mvb_herk_reduce_scaled: bad arguments");
+  return reduce_impl("mvb_herk_reduce_scaled", ws, ws_bytes, 1, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, nant, nfeed,
+                     pairs, npairs, out, 0, out_c128, 1.0, zscale, accumulate, stream);
 }
 
 extern "C" int mvb_herk_reduce_grouped(const void *ws, size_t ws_bytes, int ngroup, int64_t Mpad, int64_t Kcap,
@@ -1036,7 +1048,7 @@ extern "C" int mvb_herk_reduce_grouped(const void *ws, size_t ws_bytes, int ngro
                                        int out_c128, double vscale, int accumulate, void *stream) {
   if (out_stride > (size_t)INT64_MAX) return fail(MVB_ERR_ARG, "mvb_herk_reduce_grouped: bad arguments");
   return reduce_impl("mvb_herk_reduce_grouped", ws, ws_bytes, ngroup, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, nant,
-                     nfeed, pairs, npairs, out, (int64_t)out_stride, out_c128, vscale, accumulate, stream);
+                     nfeed, pairs, npairs, out, (int64_t)out_stride, out_c128, vscale, nullptr, accumulate, stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -586,64 +586,184 @@ __global__ void exptau_kernel(const double *__restrict__ antpos, int A, double f
   }
 }
 
-// Packs a caller complex matrix (M, K) into a panel; one thread per (m, k-pair).
-template <int MODE, typename CT>
-__global__ void z_pack_kernel(const CT *__restrict__ zs, int64_t M, int64_t K, int64_t ldz, float zscale,
-                              void *__restrict__ z, int64_t Mpad, int64_t Kcap) {
-  const int64_t kend = round_up(K, kKAlign);
-  const int64_t half = kend / 2;
-  const int64_t total = M * half;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = i / half, k = (i % half) * 2;
-    float vr[2], vi[2];
-    for (int x = 0; x < 2; ++x) {
-      if (k + x < K) {
-        const CT v = zs[m * ldz + k + x];
-        vr[x] = (float)v.x;
-        vi[x] = (float)v.y;
-      } else {
-        vr[x] = vi[x] = 0.f;
+// Power-of-two scale s with max |s Z| < 2^15 (the fp16 range) for a panel whose
+// largest |Z| is `m` (with a margin of 2^-10); 1 for an empty or non-finite Z.
+__device__ __forceinline__ float panel_scale(float m) {
+  const double top = (double)m * (1.0 + 1.0 / 1024.0);
+  if (!(top > 0.0) || isinf(top)) return 1.f;
+  const int e = ilogb(16384.0 / top);
+  return ldexpf(1.f, max(min(e, 100), -100));
+}
+
+// C values of a row from column k (zeros past K), whole 16-byte loads when vec.
+template <int C, typename CT>
+__device__ __forceinline__ void load_row(const CT *__restrict__ row, int64_t k, int64_t K, bool vec, float (&vr)[C],
+                                         float (&vi)[C]) {
+  if (vec && k + C <= K) {
+    if constexpr (sizeof(CT) == 8) {
+#pragma unroll
+      for (int i = 0; i < C; i += 2) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(row + k + i));
+        vr[i] = v.x, vi[i] = v.y, vr[i + 1] = v.z, vi[i + 1] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < C; ++i) {
+        const double2 v = __ldg(reinterpret_cast<const double2 *>(row + k + i));
+        vr[i] = (float)v.x, vi[i] = (float)v.y;
       }
     }
-    if constexpr (MODE == MVB_Z_C64) {
-      *reinterpret_cast<float4 *>(static_cast<float2 *>(z) + m * Kcap + k) = make_float4(vr[0], vi[0], vr[1], vi[1]);
-    } else {
-      // (k, k + 1), k even: inside one 16-byte chunk of one k-block row
-      constexpr int KB = kKBlockBytes / (MODE == MVB_GEMM_TF32_3 ? 4 : 2);
-      constexpr int NPL = MODE == MVB_GEMM_BF16_6 ? 6 : 4;
-      const int64_t off = panel_off(m, k, Mpad, KB, NPL);
-      PanelWriter<MODE>::put(z, panel_plane_stride(KB), off, 0, vr, 2, zscale);
-      PanelWriter<MODE>::put(z, panel_plane_stride(KB), off, 1, vi, 2, zscale);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < C; ++i) {
+    vr[i] = vi[i] = 0.f;
+    if (k + i < K) {
+      vr[i] = (float)row[k + i].x;
+      vi[i] = (float)row[k + i].y;
     }
   }
 }
 
+// Packs a caller complex matrix (M, K) into a panel.  CTA = 256 threads: 16 groups
+// of C columns (8 of complex64, 4 of complex128: 64 bytes, beyond which a load
+// instruction touches a line per lane) x 16 row lanes x `lane_rows` rows each, so
+// stores fill 8 or 16 bytes of a plane row.  It is bound by HBM; the row blocks run
+// last to first, so that those a maximum pass has just read come from L2.  With
+// `absmax` the fp16 scale is formed here from that pass's result and written to
+// scale_out.  700 rows x 49,152 columns, complex64 to fp16x3: 83 us (the copy rate),
+// against 125 with two columns a thread (4-byte stores, 64-bit divisions per
+// element); complex128: 118 against 157; to tf32x3: 136 against 197.
+// vec: the source rows allow 16-byte loads; align: the panel's alignment (2: 32
+// bytes, 1: 16, 0: less).
+constexpr int kPackThreads = 256;
+constexpr int kPackGroups = 16;
+
 template <typename CT>
-__global__ void absmax_kernel(const CT *__restrict__ z, int64_t n, float *__restrict__ out) {
-  float m = 0.f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const CT v = z[i];
-    m = fmaxf(m, (float)sqrt((double)v.x * v.x + (double)v.y * v.y));
+constexpr int kPackCols = 64 / (int)sizeof(CT);
+
+template <int MODE, typename CT>
+__global__ void __launch_bounds__(kPackThreads)
+    z_pack_kernel(const CT *__restrict__ zs, int64_t M, int64_t K, int64_t ldz, float zscale,
+                  const float *__restrict__ absmax, float *__restrict__ scale_out, void *__restrict__ z, int64_t Mpad,
+                  int64_t Kcap, int lane_rows, bool vec, int align) {
+  constexpr int C = kPackCols<CT>, LANES = kPackThreads / kPackGroups;
+  if (absmax) {
+    zscale = panel_scale(*absmax);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scale_out = zscale;
   }
+  const int64_t k = ((int64_t)blockIdx.x * kPackGroups + threadIdx.x % kPackGroups) * C;
+  if (k >= round_up(K, kKAlign)) return;
+  const int64_t nrb = ceil_div(M, (int64_t)LANES * lane_rows);
+  for (int64_t rb = blockIdx.y; rb < nrb; rb += gridDim.y) {
+    int64_t m = (nrb - 1 - rb) * LANES * lane_rows + threadIdx.x / kPackGroups;
+#pragma unroll 2
+    for (int i = 0; i < lane_rows; ++i, m += LANES) {
+      if (m >= M) break;
+      float vr[C], vi[C];
+      load_row<C>(zs + m * ldz, k, K, vec, vr, vi);
+      if constexpr (MODE == MVB_Z_C64) {
+        float2 *p = static_cast<float2 *>(z) + m * Kcap + k;
+#pragma unroll
+        for (int j = 0; j < C; j += 4) {
+          const uint32_t w[8] = {__float_as_uint(vr[j]),     __float_as_uint(vi[j]),     __float_as_uint(vr[j + 1]),
+                                 __float_as_uint(vi[j + 1]), __float_as_uint(vr[j + 2]), __float_as_uint(vi[j + 2]),
+                                 __float_as_uint(vr[j + 3]), __float_as_uint(vi[j + 3])};
+          if (align == 2)
+            store_sector(p + j, w);
+          else
+            store_words<8>(p + j, w);
+        }
+      } else {
+        constexpr int KB = kKBlockBytes / (MODE == MVB_GEMM_TF32_3 ? 4 : 2);
+        constexpr int NPL = MODE == MVB_GEMM_BF16_6 ? 6 : 4;
+        const int64_t off = panel_off(m, k, Mpad, KB, NPL);
+        if (align == 2 || (align == 1 && MODE != MVB_GEMM_TF32_3)) {
+          const int64_t off2 = panel_off(m, k + C / 2, Mpad, KB, NPL);
+          put_split<MODE, C>(z, panel_plane_stride(KB), off, off2, 0, vr, zscale);
+          put_split<MODE, C>(z, panel_plane_stride(KB), off, off2, 1, vi, zscale);
+        } else {
+#pragma unroll
+          for (int j = 0; j < C; j += 2) {
+            const int64_t o = panel_off(m, k + j, Mpad, KB, NPL);
+            PanelWriter<MODE>::put(z, panel_plane_stride(KB), o, 0, vr + j, 2, zscale);
+            PanelWriter<MODE>::put(z, panel_plane_stride(KB), o, 1, vi + j, 2, zscale);
+          }
+        }
+      }
+    }
+  }
+}
+
+// Largest |z|: the squares in FP64 (exact for complex64), one square root per
+// thread -- it is monotonic, so the result is that of a root per element, which
+// bounded this pass.  Two elements per load where the source allows (vec), and one
+// atomic per CTA: one per warp, 9,472 on one word, took 8 us whatever the size.
+// 275 MB: 53 us, against 78; 1 M elements: 3.9 against 8.7.
+constexpr int kAbsmaxThreads = 256;
+
+template <typename CT>
+__global__ void __launch_bounds__(kAbsmaxThreads) absmax_kernel(const CT *__restrict__ z, int64_t n, float *__restrict__ out, bool vec) {
+  double m2 = 0.0;
+  auto take = [&](double x, double y) { m2 = fmax(m2, x * x + y * y); };
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  if (sizeof(CT) == 8 && vec) {
+    const float4 *z4 = reinterpret_cast<const float4 *>(z);
+    const int64_t n4 = n / 2;
+    int64_t i = i0;
+    for (; i + 3 * step < n4; i += 4 * step) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = __ldg(z4 + i + u * step);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        take(v[u].x, v[u].y);
+        take(v[u].z, v[u].w);
+      }
+    }
+    for (; i < n4; i += step) {
+      const float4 v = __ldg(z4 + i);
+      take(v.x, v.y);
+      take(v.z, v.w);
+    }
+    if ((n & 1) && i0 == 0) take(z[n - 1].x, z[n - 1].y);
+  } else {
+    for (int64_t i = i0; i < n; i += step) {
+      const CT v = z[i];
+      take(v.x, v.y);
+    }
+  }
+  float m = (float)sqrt(m2);
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  // non-negative floats order like their bit patterns
-  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(out), __float_as_int(m));
+  __shared__ float warp_m[kAbsmaxThreads / 32];
+  if ((threadIdx.x & 31) == 0) warp_m[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kAbsmaxThreads / 32; ++w) m = fmaxf(m, warp_m[w]);
+    // non-negative floats order like their bit patterns
+    atomicMax(reinterpret_cast<int *>(out), __float_as_int(m));
+  }
 }
 
 }  // namespace mvb
 
 using namespace mvb;
 
+static int launch_absmax(const void *z, int z_c128, int64_t n, float *out, cudaStream_t s) {
+  if (n == 0) return MVB_OK;
+  const int threads = kAbsmaxThreads;
+  const int64_t blocks = std::min<int64_t>(ceil_div(n, threads * 4), (int64_t)num_sms() * 8);
+  const bool vec = reinterpret_cast<uintptr_t>(z) % 16 == 0;
+  if (z_c128)
+    absmax_kernel<double2><<<(unsigned)blocks, threads, 0, s>>>(static_cast<const double2 *>(z), n, out, vec);
+  else
+    absmax_kernel<float2><<<(unsigned)blocks, threads, 0, s>>>(static_cast<const float2 *>(z), n, out, vec);
+  return check_launch("absmax_kernel");
+}
+
 extern "C" int mvb_absmax(const void *z, int z_c128, int64_t n, float *out, void *stream) {
   if (!out || n < 0 || (n > 0 && !z)) return fail(MVB_ERR_ARG, "mvb_absmax: bad arguments");
-  if (n == 0) return MVB_OK;
-  const int threads = 256;
-  const int64_t blocks = std::min<int64_t>(ceil_div(n, threads), (int64_t)num_sms() * 8);
-  if (z_c128)
-    absmax_kernel<double2><<<(unsigned)blocks, threads, 0, as_stream(stream)>>>(static_cast<const double2 *>(z), n, out);
-  else
-    absmax_kernel<float2><<<(unsigned)blocks, threads, 0, as_stream(stream)>>>(static_cast<const float2 *>(z), n, out);
-  return check_launch("absmax_kernel");
+  return launch_absmax(z, z_c128, n, out, as_stream(stream));
 }
 
 extern "C" size_t mvb_zpanel_bytes(int mode, int64_t Mpad, int64_t Kcap) {
@@ -806,20 +926,21 @@ extern "C" int mvb_tau_z_grouped(const double *antpos, int A, const double *freq
                     beam, beam_ld, nbeam, beam_idx, F, X, mode, zscale, z, (int64_t)z_stride, Mpad, Kcap, stream);
 }
 
-extern "C" int mvb_z_pack(const void *zsrc, int z_c128, int64_t M, int64_t K, int64_t ldz, int mode, float zscale,
-                          void *z, int64_t Mpad, int64_t Kcap, void *stream) {
-  if (M < 0 || K < 0 || ldz < K || !z || (M * K > 0 && !zsrc)) return fail(MVB_ERR_ARG, "mvb_z_pack: bad arguments");
-  int rc = check_panel(mode, M, Mpad, Kcap, "mvb_z_pack");
-  if (rc) return rc;
-  if (round_up(K, kKAlign) > Kcap) return fail(MVB_ERR_ARG, "mvb_z_pack: Kcap too small");
-  const int64_t total = M * (round_up(K, kKAlign) / 2);
-  if (total == 0) return MVB_OK;
-  const int threads = 256;
-  const int64_t blocks = std::min<int64_t>(ceil_div(total, threads), (int64_t)num_sms() * 16);
-  cudaStream_t s = as_stream(stream);
-#define MVB_PACK(M_, CT)                                                                                             \
-  z_pack_kernel<M_, CT><<<(unsigned)blocks, threads, 0, s>>>(static_cast<const CT *>(zsrc), M, K, ldz, zscale, z, Mpad, \
-                                                             Kcap)
+static int z_pack_impl(const char *who, const void *zsrc, int z_c128, int64_t M, int64_t K, int64_t ldz, int mode,
+                       float zscale, const float *absmax, float *scale_out, void *z, int64_t Mpad, int64_t Kcap,
+                       cudaStream_t s) {
+  const int64_t cols = round_up(K, kKAlign);
+  if (M == 0 || cols == 0) return MVB_OK;
+  const int64_t xblocks = ceil_div(cols, kPackGroups * (z_c128 ? kPackCols<double2> : kPackCols<float2>));
+  // four rows a lane (a 64-row block) where that still leaves eight CTAs per SM
+  constexpr int lanes = kPackThreads / kPackGroups;
+  const int lane_rows = xblocks * ceil_div(M, 4 * lanes) >= (int64_t)num_sms() * 8 ? 4 : 1;
+  const dim3 grid((unsigned)xblocks, (unsigned)std::min<int64_t>(ceil_div(M, (int64_t)lane_rows * lanes), 65535));
+  const bool vec = reinterpret_cast<uintptr_t>(zsrc) % 16 == 0 && (z_c128 || ldz % 2 == 0);
+  const int align = reinterpret_cast<uintptr_t>(z) % 32 == 0 ? 2 : (reinterpret_cast<uintptr_t>(z) % 16 == 0 ? 1 : 0);
+#define MVB_PACK(M_, CT)                                                                                            \
+  z_pack_kernel<M_, CT><<<grid, kPackThreads, 0, s>>>(static_cast<const CT *>(zsrc), M, K, ldz, zscale, absmax,     \
+                                                      scale_out, z, Mpad, Kcap, lane_rows, vec, align)
 #define MVB_PACK2(M_) \
   if (z_c128)         \
     MVB_PACK(M_, double2); \
@@ -835,6 +956,37 @@ extern "C" int mvb_z_pack(const void *zsrc, int z_c128, int64_t M, int64_t K, in
 #undef MVB_PACK2
 #undef MVB_PACK
   return check_launch("z_pack_kernel");
+}
+
+static int check_pack(const char *who, const void *zsrc, int64_t M, int64_t K, int64_t ldz, int mode, const void *z,
+                      int64_t Mpad, int64_t Kcap) {
+  if (M < 0 || K < 0 || ldz < K || !z || (M * K > 0 && !zsrc)) return fail(MVB_ERR_ARG, "%s: bad arguments", who);
+  int rc = check_panel(mode, M, Mpad, Kcap, who);
+  if (rc) return rc;
+  if (round_up(K, kKAlign) > Kcap) return fail(MVB_ERR_ARG, "%s: Kcap too small", who);
+  return MVB_OK;
+}
+
+extern "C" int mvb_z_pack(const void *zsrc, int z_c128, int64_t M, int64_t K, int64_t ldz, int mode, float zscale,
+                          void *z, int64_t Mpad, int64_t Kcap, void *stream) {
+  int rc = check_pack("mvb_z_pack", zsrc, M, K, ldz, mode, z, Mpad, Kcap);
+  if (rc) return rc;
+  return z_pack_impl("mvb_z_pack", zsrc, z_c128, M, K, ldz, mode, zscale, nullptr, nullptr, z, Mpad, Kcap,
+                     as_stream(stream));
+}
+
+extern "C" int mvb_z_pack_scaled(const void *zsrc, int z_c128, int64_t M, int64_t K, int64_t ldz, int mode,
+                                 float *scale, void *z, int64_t Mpad, int64_t Kcap, void *stream) {
+  const char *who = "mvb_z_pack_scaled";
+  int rc = check_pack(who, zsrc, M, K, ldz, mode, z, Mpad, Kcap);
+  if (rc) return rc;
+  if (!scale || ldz != K || M * K == 0) return fail(MVB_ERR_ARG, "%s: bad arguments", who);
+  cudaStream_t s = as_stream(stream);
+  cudaError_t e = cudaMemsetAsync(scale, 0, sizeof(float), s);
+  if (e != cudaSuccess) return fail(MVB_ERR_CUDA, "%s: %s", who, cudaGetErrorString(e));
+  rc = launch_absmax(zsrc, z_c128, M * K, scale, s);
+  if (rc) return rc;
+  return z_pack_impl(who, zsrc, z_c128, M, K, ldz, mode, 1.f, scale, scale + 1, z, Mpad, Kcap, s);
 }
 
 static int tau_z_pol_impl(const char *who, const double *antpos, int A, double freq, const double *freqs_dev,

@@ -41,8 +41,19 @@ class ZPanel:
         self.data = data
         self.n_dev = None
         self.n_host = 0
-        #: power-of-two factor the panel holds Z multiplied by (fp16x3 mode)
         self.scale = 1.0
+
+    @property
+    def scale(self) -> float:
+        """Power-of-two factor the panel holds Z multiplied by (fp16x3 mode); read
+        from the device when it was chosen there."""
+        return self._scale if self.scale_dev is None else float(self.scale_dev[1].item())
+
+    @scale.setter
+    def scale(self, value: float):
+        self._scale = value
+        #: two device floats (max |Z|, scale) when mvb_z_pack_scaled chose the scale
+        self.scale_dev = None
 
     @staticmethod
     def data_shape(mode: int, M: int, Mpad: int, Kcap: int) -> tuple:

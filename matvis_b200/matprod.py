@@ -169,17 +169,15 @@ class MatProd(ABC):
             panel = ZPanel(mode, self.nant, self.nfeed, 1, K, self.device)
             self._packed = {key: panel}
         c128 = 1 if zt.dtype == torch.complex128 else 0
-        scale = 1.0
-        if mode == _lib.GEMM_F16_3:
-            mx = torch.zeros(1, dtype=torch.float32, device=self.device)
-            check(_lib.lib.mvb_absmax(ptr(zt), c128, M * K, ptr(mx), stream_handle()))
-            scale = _lib.f16_scale(float(mx.item()) * (1 + 2**-10))
-        panel.scale = scale
-        check(
-            _lib.lib.mvb_z_pack(
-                ptr(zt), c128, M, K, K, mode, scale, ptr(panel.data), panel.Mpad, panel.Kcap, stream_handle(),
-            )
-        )
+        panel.scale = 1.0
+        if mode == _lib.GEMM_F16_3 and K:
+            # the scale is chosen on the device: no wait for the maximum
+            panel.scale_dev = torch.empty(2, dtype=torch.float32, device=self.device)
+            check(_lib.lib.mvb_z_pack_scaled(ptr(zt), c128, M, K, K, mode, ptr(panel.scale_dev), ptr(panel.data),
+                                             panel.Mpad, panel.Kcap, stream_handle()))
+        else:
+            check(_lib.lib.mvb_z_pack(ptr(zt), c128, M, K, K, mode, 1.0, ptr(panel.data), panel.Mpad, panel.Kcap,
+                                      stream_handle()))
         panel.n_dev = None
         panel.n_host = K
         return panel
@@ -282,11 +280,14 @@ class B200MatMul(MatProd):
             )
         )
         pairs = None if self.all_pairs else self._pairs_dev
+        # a scale chosen on the device stays there
+        reduce, scale = ((_lib.lib.mvb_herk_reduce, 1.0 / panel.scale**2) if panel.scale_dev is None
+                         else (_lib.lib.mvb_herk_reduce_scaled, ptr(panel.scale_dev[1:])))
         check(
-            _lib.lib.mvb_herk_reduce(
+            reduce(
                 ptr(ws), ws.numel(), panel.Mpad, panel.Kcap, ptr(panel.n_dev), panel.n_host, kmul, kc, self.nant,
                 self.nfeed,
-                ptr(pairs), self.npairs, ptr(out), 1 if out.dtype == torch.complex128 else 0, 1.0 / panel.scale**2,
+                ptr(pairs), self.npairs, ptr(out), 1 if out.dtype == torch.complex128 else 0, scale,
                 int(accumulate), sh,
             )
         )
