@@ -58,7 +58,7 @@
 //                   completes in about half the time of the same bytes as tiled
 //                   TMA boxes of 64-byte rows, and the three stages in flight no
 //                   longer leave the MMA waiting;
-//   warp 1        : TMEM owner (512 columns = two k-step blocks); lane 0 issues
+//   warp 1        : TMEM owner (512 columns = two k-step blocks); one lane issues
 //                   the UMMAs and tcgen05.commit's the stage / block barriers;
 //   warps 2..17   : epilogue; warp w drains TMEM lane quadrant (w % 4), column
 //                   quarter (w - 2) / 4 (64 of the 256 columns), 64 FP32
@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
   tc_fence_after();
   const uint32_t tbase = tmem_base_sh;
 
-  uint64_t issued = 0;  // producer: stages issued
+  uint64_t issued = 0;            // producer: stages issued
+  bool lead = warp == 1 && lane == 0;  // the thread that issues the UMMAs
   if (warp == 0 && lane == 0) {
     // ---------------- bulk-copy producer ----------------
     uint32_t st = 0, ph = 0;
@@ -364,8 +365,113 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
         }
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ---------------- UMMA issuer: one fresh TMEM block per KD k-steps ----------------
+  } else if (KD == 2 && warp == 1) {
+    // ---------------- UMMA issuer, KD = 2: one fresh TMEM block per stage ----------------
+    // The warp stays converged and an elected lane issues, so that descriptors and
+    // loop state live in uniform registers; and the barriers of the NEXT block (its
+    // stage filled, its TMEM block drained, at a unit's end the next unit) are waited
+    // on between the last UMMAs of this one.  A single lane that waited between blocks
+    // left the tensor pipe idle for 470 of 1,900 cycles per block: the pipe's queue
+    // holds only the last few UMMAs, and the barrier checks, commits and descriptor
+    // arithmetic took longer than those run.  Tensor pipe busy, 700 rows, fp16x3, by
+    // clock64: 66 % that way, 79 % with both waits before the last k-step, 84-86 %
+    // with the waits apart (tf32x3 66, 83, 89 %).  Under the power cap the clock gives
+    // part of it back: 8 slices of K = 49,152 run at the sustained cuBLAS rate (1.40
+    // PFLOP/s executed), K = 196,608 10.46 -> 9.71 ms, tf32x3 x 3 1.89 -> 1.66 ms; 128
+    // two-feed antennas, K = 30,000 43.1 -> 35.4 us, 90 of one feed x 8 42.6 -> 34.7.
+    // Within a block, products in ascending magnitude across both k-steps -- every
+    // cross term, then the hi x hi products -- so that the block's large partial sum
+    // exists only for its last instructions (the accumulator is truncated toward
+    // zero at each).
+    lead = elect_one();
+    uint32_t st = 0, ph = 0, buf = 0, dph = 0, uk = 0;
+    int nks = 0;
+    bool diag = false, ok = true;
+    auto wait_all = [&](uint64_t *bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, wait_ns)) != 0;
+    };
+    // the next unit's k-step count and tile kind; false when there is none (or a wait ran out)
+    auto next_unit = [&]() {
+      const int us = uk % kUnitRing;
+      if (__any_sync(0xffffffffu, abort_flag)) return false;
+      if (!wait_all(&ufull_bar[us], (uk / kUnitRing) & 1u)) {
+        ok = false;
+        return false;
+      }
+      const int u = __shfl_sync(0xffffffffu, unit_q[us], 0);
+      if (lane == 0) mbar_arrive(&uempty_bar[us]);
+      ++uk;
+      if (u >= n_units) return false;
+      const uint8_t *zpanel;
+      float *partial;
+      int Tu, I, J;
+      int64_t k0, klen;
+      place(u, zpanel, partial, Tu, I, J, k0, klen);
+      nks = __shfl_sync(0xffffffffu, (int)((klen + C::KSTEP - 1) / C::KSTEP), 0);
+      diag = __shfl_sync(0xffffffffu, I == J ? 1 : 0, 0) != 0;
+      return true;
+    };
+    bool have = next_unit();
+    int ks = 0;
+    if (have) ok = wait_all(&dempty_bar[0], 1u) && wait_all(&full_bar[0], 0u);
+    while (have && ok) {
+      tc_fence_after();
+      const int nk = min(2, nks - ks);
+      const uint32_t d = tbase + buf * 256;
+      const uint64_t a0 = umma_desc_sw64(smem_u32(smem) + st * C::STAGE_BYTES);
+      const uint64_t b0 = diag ? a0 : a0 + (C::OPER_BYTES >> 4);
+      const uint32_t id_re = diag ? C::ID128 : C::ID256;
+      const uint32_t st2 = st + 1 == C::STAGES ? 0 : st + 1, ph2 = st2 == 0 ? ph ^ 1u : ph;
+      const uint32_t dph2 = dph ^ (1u << buf);
+#pragma unroll
+      for (int q = 0; q < C::NPROD; ++q) {
+        uint32_t pa, pb;
+        product_terms(C::NPROD, q, pa, pb);
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          // the next block, while the pipe still has the products before the last one
+          // queued; the two waits apart, each covered by the UMMAs around it
+          if (q == C::NPROD - 1 && kk == 0) {
+            ks += 2;
+            if (ks >= nks) {
+              have = next_unit();
+              ks = 0;
+            }
+            if (have) ok = wait_all(&full_bar[st2], ph2);
+          } else if (q == C::NPROD - 1 && have && ok) {
+            ok = wait_all(&dempty_bar[buf ^ 1u], ((dph2 >> (buf ^ 1u)) & 1u) ^ 1u);
+          }
+          if (lead && kk < nk) {
+            const uint64_t a_re = a0 + ((2 * pa * kPlaneBytes + kk * 32) >> 4);
+            const uint64_t a_im = a0 + (((2 * pa + 1) * kPlaneBytes + kk * 32) >> 4);
+            const uint64_t b_re = b0 + ((2 * pb * kPlaneBytes + kk * 32) >> 4);
+            const uint64_t b_im = b0 + (((2 * pb + 1) * kPlaneBytes + kk * 32) >> 4);
+            // the two N = 128 products first: the block's real and imaginary
+            // halves each start from Zi terms, then take the Zr terms
+            const uint32_t acc = (q > 0 || kk > 0) ? 1u : 0u;
+            umma<MODE>(d, a_im, b_im, C::ID128, acc);
+            umma<MODE>(d + 128, a_im, b_re, C::ID128N, acc);
+            umma<MODE>(d, a_re, b_re, id_re, 1u);
+          }
+          __syncwarp();
+        }
+      }
+      if (lead) {
+        tc_commit(&empty_bar[st]);  // the stage is consumed
+        tc_commit(&dfull_bar[buf]);  // the block is complete
+      }
+      __syncwarp();
+      st = st2;
+      ph = ph2;
+      dph = dph2;
+      buf ^= 1u;
+    }
+    if (!ok) {
+      if (lane == 0) flag_timeout();
+      abort_flag = 1;
+    }
+  } else if (KD != 2 && warp == 1 && lane == 0) {
+    // ---------------- UMMA issuer, KD = 1 or 4: one thread, a wait before each block ----------------
     uint32_t st = 0, ph = 0, buf = 0, dph = 0;
     for (uint32_t uk = 0; !abort_flag; ++uk) {
       const int us = uk % kUnitRing;
@@ -385,7 +491,7 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
       const int nks = (int)((klen + C::KSTEP - 1) / C::KSTEP);
       const bool diag = I == J;
       bool ok = true;
-      if constexpr (KD == 2 || KD == 4) {
+      if constexpr (KD == 4) {
         // a TMEM block is KD / 2 whole stages (two k-steps each): products
         // ordered by magnitude across the block's k-steps -- every cross term,
         // then the hi x hi products -- so that the block's large partial sum
@@ -531,13 +637,14 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
         if (!ok) break;
         tc_fence_after();
         const uint32_t taddr = tbase + ((uint32_t)(quad * 32) << 16) + buf * 256 + quarter * 64;
+        constexpr int W = KD == 2 ? 8 : 16;  // columns per load: 16 spill beside the KD = 2 issuer
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t v[16];
-          tmem_ld16(taddr + c * 16, v);
+        for (int c = 0; c < 64 / W; ++c) {
+          uint32_t v[W];
+          tmem_ld<W>(taddr + c * W, v);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[c * 16 + j] += __uint_as_float(v[j]);
+          for (int j = 0; j < W; ++j) acc[c * W + j] += __uint_as_float(v[j]);
         }
         tc_fence_before();
         __syncwarp();
@@ -567,7 +674,7 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
       for (uint64_t i = first; i < issued; ++i)
         mbar_wait(&full_bar[i % C::STAGES], (uint32_t)((i / C::STAGES) & 1), kDrainLimitNs);
     }
-    if (warp == 1 && lane == 0) {
+    if (lead) {
       tc_commit(&drain_bar);
       mbar_wait(&drain_bar, 0, kDrainLimitNs);
     }
