@@ -404,6 +404,57 @@ int mvb_tau_z_pol_grouped(const double *antpos, int A, const double *freqs, int 
                           int mode, float zscale, void *z, size_t z_stride, int64_t Mpad, int64_t Kcap,
                           void *stream);
 
+/* ---- Batched job ------------------------------------------------------------ */
+/* A prepared job: device buffers (but the arrays marked host), sizes and options
+ * of the launch sequence of its ntime x nchunks x nfreq slices. */
+typedef struct {
+  int64_t nsrc, chunk_size, cap; /* sources, sources per chunk, kept-source slots */
+  int ntime, nchunks, nfreq;
+  int nant, nfeed, freq_group;   /* nfeed = beam axes; freq_group: frequencies (panels) per launch */
+  const double *eci, *antpos;    /* (3, nsrc), (nant, 3) */
+  double *bcrs, *topo;           /* bcrs: apparent-place directions, NULL for the LST rotation */
+  const double *rot, *astrom;    /* host: ntime x 9 rotations; ntime x 18 mvb_bcrs parameters */
+  const uint8_t *refresh;        /* host: times that recompute bcrs */
+  double *crd;                   /* (3, cap) */
+  int32_t *kept, *n_above, *status;
+  void *select_ws;
+  size_t select_ws_bytes;
+  const double *sigmas;          /* Gaussian beams, or NULL for grids */
+  const void *const *grids;      /* host: device grids per frequency (one entry unless chromatic) */
+  const double *const *grid_params;
+  int nbeam, grid_kind, nza, naz, chromatic;
+  void *beam;                    /* complex64 (nbeam, nfeed, nfeed, cap) */
+  void *beam_ws;
+  size_t beam_ws_bytes;
+  const int32_t *beam_idx;
+  const float *sflux, *coh;      /* sqrt(0.5 I) rows, or (polarised sky) coherency rows of 4 */
+  int64_t flux_ld;
+  const double *radec, *frame_average; /* polarised sky: (2, nsrc); host ntime x 9 */
+  double *frame_rot;             /* (cap, 2) */
+  const double *freqs, *freqs_dev; /* host, device: nfreq */
+  int mode;                      /* MVB_GEMM_* (Hermitian product) or MVB_Z_C64 (pair sums) */
+  float zscale;
+  void *z;
+  size_t z_stride;
+  int64_t Mpad, Kcap;
+  int k_chunk, drain_ksteps;
+  void *ws;
+  size_t ws_bytes;
+  const int32_t *pairs;          /* NULL: all nant^2 */
+  int64_t npairs;
+  const void *plan;              /* mvb_vecdot_plan bundles: the staged pair sums */
+  int64_t nbundles;
+  void *vis;                     /* frequency f, time t at f vis_f_stride + t vis_t_stride bytes */
+  int64_t vis_f_stride, vis_t_stride;
+  int out_c128;
+} mvb_job;
+/* Enqueues times [t0, t1), chunks [c0, c1) and frequencies [f0, f1) of a job (f0 a
+ * multiple of freq_group): for each time and chunk, if f0 = 0, the rotation (chunk
+ * 0), selection, beam and frame rotation, then the frequency groups' tau/Z, product
+ * and reduction -- the entry points above in the order of the reference's loops
+ * (wrapper.py:180-199, cpu/cpu.py:247-272).  Nothing is kept from the call. */
+int mvb_job_enqueue(const mvb_job *job, int t0, int t1, int c0, int c1, int f0, int f1, void *stream);
+
 /* ---- Redundant-baseline pair selection (host memory, no device work) ------- */
 /* bls: (nant, nant, 2) float64 baselines, bls[i, j] = pos[j, :2] - pos[i, :2].
  * Writes the pairs (i, j), i < j, that get_redundancies (cli.py:273-290) keeps:

@@ -123,6 +123,7 @@ _SIGNATURES = {
         c_int,
         [_p, c_int64, _p, c_int64, c_int, c_int, _p, c_int64, c_int, _p, c_size_t, _p, c_int, c_int, _p],
     ),
+    "mvb_job_enqueue": (c_int, [_p, c_int, c_int, c_int, c_int, c_int, c_int, _p]),
     "mvb_vecdot_plan_bytes": (c_size_t, [c_int64, c_int]),
     "mvb_vecdot_plan": (c_int, [_p, c_int64, c_int, c_int, _p, c_size_t, _p]),
     "mvb_vecdot_stage_columns": (c_int, [c_int, c_int]),
@@ -141,6 +142,27 @@ class HerkGroup(ctypes.Structure):
     _fields_ = [("z", c_void_p), ("z_stride", c_size_t), ("ngroup", c_int), ("Mpad", c_int64), ("Kcap", c_int64),
                 ("n_dev", c_void_p), ("n_host", c_int64), ("kmul", c_int), ("k_chunk", c_int), ("ws", c_void_p),
                 ("ws_bytes", c_size_t), ("status", c_void_p)]
+
+
+class Job(ctypes.Structure):
+    """``mvb_job`` of the C header: the launch sequence of a batched job."""
+
+    _fields_ = (
+        [(n, c_int64) for n in ("nsrc", "chunk_size", "cap")]
+        + [(n, c_int) for n in ("ntime", "nchunks", "nfreq", "nant", "nfeed", "freq_group")]
+        + [(n, c_void_p) for n in ("eci", "antpos", "bcrs", "topo", "rot", "astrom", "refresh", "crd", "kept",
+                                   "n_above", "status", "select_ws")]
+        + [("select_ws_bytes", c_size_t)]
+        + [(n, c_void_p) for n in ("sigmas", "grids", "grid_params")]
+        + [(n, c_int) for n in ("nbeam", "grid_kind", "nza", "naz", "chromatic")]
+        + [("beam", c_void_p), ("beam_ws", c_void_p), ("beam_ws_bytes", c_size_t), ("beam_idx", c_void_p),
+           ("sflux", c_void_p), ("coh", c_void_p), ("flux_ld", c_int64)]
+        + [(n, c_void_p) for n in ("radec", "frame_average", "frame_rot", "freqs", "freqs_dev")]
+        + [("mode", c_int), ("zscale", c_float), ("z", c_void_p), ("z_stride", c_size_t), ("Mpad", c_int64),
+           ("Kcap", c_int64), ("k_chunk", c_int), ("drain_ksteps", c_int), ("ws", c_void_p), ("ws_bytes", c_size_t),
+           ("pairs", c_void_p), ("npairs", c_int64), ("plan", c_void_p), ("nbundles", c_int64), ("vis", c_void_p),
+           ("vis_f_stride", c_int64), ("vis_t_stride", c_int64), ("out_c128", c_int)]
+    )
 
 
 #: panels one mvb_herk_batch launch can hold

@@ -20,6 +20,7 @@ whole job can be captured once as a CUDA graph and replayed.
 
 from __future__ import annotations
 
+import ctypes
 import os
 import queue
 import threading
@@ -375,61 +376,92 @@ class VisEngine:
         return n
 
     # ----------------------------------------------------------------- launch
+    def _launches(self) -> tuple[_lib.Job, list]:
+        """The job's launch sequence for ``mvb_job_enqueue`` and the host arrays it
+        points to (made for one call: buffers and options are read as they are)."""
+        s = self.spec
+        mp, p0, bm = self.matprod, self.panels[0], self.bmfunc
+        herk = self.method == "MatMul"
+        ws = mp.workspace(p0, self.k_chunk, self.fgroup) if herk else mp.workspace(p0)
+        rot = np.ascontiguousarray(self.rot, dtype=np.float64)
+        keep = [rot, ws, self.freqs]
+
+        def at(x):
+            return None if x is None else x.data_ptr()
+
+        def host(x):
+            keep.append(x)
+            return x.ctypes.data
+
+        j = _lib.Job(
+            nsrc=self.nsrc, chunk_size=self.chunk_size, cap=self.cap, ntime=len(self.lsts), nchunks=self.nchunks,
+            nfreq=len(self.freqs), nant=self.nant, nfeed=self.nfeed, freq_group=self.fgroup, eci=at(self.eci),
+            antpos=at(self.antpos), topo=at(self.topo), rot=rot.ctypes.data, crd=at(self.crd), kept=at(self.kept),
+            n_above=at(self.n_above), status=at(self.status), select_ws=at(self.ws_compact),
+            select_ws_bytes=self.ws_compact.numel(), nbeam=bm.nbeam, chromatic=int(self.chromatic),
+            beam=at(bm.interpolated_beam), beam_idx=at(bm.beam_index_dev), freqs=self.freqs.ctypes.data,
+            freqs_dev=at(self.freqs_dev), mode=self.zcalc.mode, zscale=self.zscale, z=at(p0.data),
+            z_stride=p0.nbytes, Mpad=p0.Mpad, Kcap=p0.Kcap, k_chunk=self.k_chunk if herk else mp.k_chunk,
+            ws=at(ws), ws_bytes=ws.numel(), npairs=self.npairs, vis=at(self.vis),
+            vis_f_stride=self.vis.stride(0) * self.vis.element_size(),
+            vis_t_stride=self.vis.stride(1) * self.vis.element_size(),
+            out_c128=1 if self.vis.dtype == torch.complex128 else 0)
+        if self.bcrs_plan is not None:
+            j.bcrs = at(self.bcrs)
+            j.astrom = host(np.ascontiguousarray(np.stack(self.astrom_packed)) if self.astrom_packed
+                            else np.zeros((1, 18)))
+            j.refresh = host(np.asarray(self.bcrs_plan + [False], dtype=np.uint8))
+        if bm.use_interp:
+            j.grid_kind, j.nza, j.naz = bm.grid_kind, bm.nza, bm.naz
+            j.grids = host(np.array([b.grids.data_ptr() for b in self.bmfuncs], dtype=np.uintp))
+            j.grid_params = host(np.array([b.params.data_ptr() for b in self.bmfuncs], dtype=np.uintp))
+            j.beam_ws, j.beam_ws_bytes = at(bm._coord_ws), bm._coord_ws.numel() * 8
+        else:
+            j.sigmas = at(bm.sigmas)
+        if self.pol_sky:
+            j.coh, j.flux_ld, j.radec, j.frame_rot = at(self.coh), self.coh.shape[1], at(self.radec), at(self.rot2)
+            j.frame_average = host(np.ascontiguousarray(np.stack(self.ravg)) if self.ravg else np.zeros((1, 9)))
+        else:
+            j.sflux, j.flux_ld = at(self.sflux), self.sflux.shape[1]
+        if herk:
+            j.drain_ksteps = mp.drain_ksteps
+            j.pairs = None if mp.all_pairs else at(mp._pairs_dev)
+        elif mp.kernel == "staged":
+            j.plan, j.nbundles = at(mp._plan_dev), mp.nbundles
+        else:
+            j.pairs = at(mp._pairs_dev)
+        for p in self.panels:
+            p.n_dev, p.n_host, p.scale = self.n_above, self.cap, self.zscale
+        return j, keep
+
     def enqueue(self, stream=None):
         """Enqueue every kernel of the job on ``stream`` (no host synchronisation)."""
-        for t in range(len(self.lsts)):
-            self.enqueue_time(t, stream)
+        job, _keep = self._launches()
+        _lib.check(_lib.lib.mvb_job_enqueue(ctypes.byref(job), 0, len(self.lsts), 0, self.nchunks, 0, len(self.freqs),
+                                            _lib.stream_handle(stream)))
 
-    def enqueue_time(self, t: int, stream=None, after=None):
+    def enqueue_time(self, t: int, stream=None, after=None, launches=None):
         """Enqueue the kernels of time index t (all chunks and frequencies).
 
         ``after(f0, g)``, if given, is called once the launches that complete
         frequencies f0 .. f0 + g - 1 of this time are enqueued (for a results
-        copy that can start as soon as they have run)."""
-        L = _lib.lib
+        copy that can start as soon as they have run).  ``launches``: the
+        ``_launches()`` of this job, if the caller already has them."""
+        job, _keep = launches or self._launches()
         sh = _lib.stream_handle(stream)
-        chk = _lib.check
-        A = self.nant
-        F, X = self.nfeed, self.nax
-        panel = self.zcalc.z
-        for c in range(self.nchunks):
-            beam = self.chunk_prologue(t, c, stream)
-            last = c == self.nchunks - 1
-            if self.fgroup > 1:
-                for f0 in range(0, len(self.freqs), self.fgroup):
-                    g = self.tau_z_group(t, f0, beam, stream)
-                    self.matprod.enqueue_grouped(self.panels[:g], self.vis[f0:f0 + g, t], accumulate=c > 0,
-                                                 stream=stream, k_chunk=self.k_chunk)
-                    if last and after is not None:
-                        after(f0, g)
-                continue
-            for f in range(len(self.freqs)):
-                if self.chromatic:
-                    self.bmfuncs[f].launch(self.crd, self.cap, self.n_above, self.cap, beam, stream=stream,
-                                           status=self.status)
-                if self.pol_sky:
-                    chk(L.mvb_tau_z_pol(
-                        _lib.ptr(self.antpos), A, float(self.freqs[f]), _lib.ptr(self.crd), self.cap,
-                        _lib.ptr(self.n_above), self.cap, _lib.ptr(self.coh[f]), _lib.ptr(self.kept),
-                        _lib.ptr(self.rot2), _lib.ptr(beam), beam.shape[-1], beam.shape[0],
-                        _lib.ptr(self.bmfunc.beam_index_dev), self.zcalc.mode, self.zscale, _lib.ptr(panel.data),
-                        panel.Mpad, panel.Kcap, sh))
-                else:
-                    chk(L.mvb_tau_z(
-                        _lib.ptr(self.antpos), A, float(self.freqs[f]), _lib.ptr(self.crd), self.cap,
-                        _lib.ptr(self.n_above), self.cap, _lib.ptr(self.sflux[f]), _lib.ptr(self.kept),
-                        _lib.ptr(beam), beam.shape[-1], beam.shape[0], _lib.ptr(self.bmfunc.beam_index_dev), F, X,
-                        self.zcalc.mode, self.zscale, _lib.ptr(panel.data), panel.Mpad, panel.Kcap, sh))
-                panel.n_dev = self.n_above
-                panel.n_host = self.cap
-                panel.scale = self.zscale
-                out = self.vis[f, t]
-                if self.method == "MatMul":
-                    self.matprod.enqueue(panel, out, accumulate=c > 0, stream=stream, k_chunk=self.k_chunk)
-                else:
-                    self.matprod.enqueue(panel, out, accumulate=c > 0, stream=stream)
-                if last and after is not None:
-                    after(f, 1)
+        nf, last = len(self.freqs), self.nchunks - 1
+
+        def part(c0, c1, f0, f1):
+            _lib.check(_lib.lib.mvb_job_enqueue(ctypes.byref(job), t, t + 1, c0, c1, f0, f1, sh))
+
+        if after is None or not nf:
+            return part(0, self.nchunks, 0, nf)
+        if last:
+            part(0, last, 0, nf)
+        for f0 in range(0, nf, self.fgroup):
+            g = min(self.fgroup, nf - f0)
+            part(last, self.nchunks, f0, f0 + g)
+            after(f0, g)
 
     def chunk_prologue(self, t: int, c: int, stream=None) -> torch.Tensor:
         """The kernels of time t and source chunk c that every frequency shares:
@@ -583,6 +615,7 @@ class VisEngine:
                 while steps.get() is not None:
                     pass
 
+        launches = self._launches()
         worker = threading.Thread(target=copier, name="mvb-d2h", daemon=True)
         worker.start()
         try:
@@ -592,7 +625,7 @@ class VisEngine:
                     done.record(main)
                     steps.put((t, f0, g, done))
 
-                self.enqueue_time(t, after=after)
+                self.enqueue_time(t, after=after, launches=launches)
         finally:
             steps.put(None)
             worker.join()

@@ -344,8 +344,8 @@ class B200VectorDot(MatProd):
             self.nbundles = len(plan)
             self._plan_dev = torch.as_tensor(plan, device=self.device)
 
-    def enqueue(self, panel: ZPanel, out: torch.Tensor, accumulate: bool = False, stream=None):
-        c128 = 1 if out.dtype == torch.complex128 else 0
+    def workspace(self, panel: ZPanel) -> torch.Tensor:
+        """Partial-sum workspace for ``panel``'s shape (kept and grown as needed)."""
         if self.kernel == "staged":
             if self._plan_dev is None:
                 self.setup()
@@ -355,6 +355,11 @@ class B200VectorDot(MatProd):
         if self._ws is None or self._ws.numel() < nbytes:
             self._ws = None
             self._ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+        return self._ws
+
+    def enqueue(self, panel: ZPanel, out: torch.Tensor, accumulate: bool = False, stream=None):
+        c128 = 1 if out.dtype == torch.complex128 else 0
+        self.workspace(panel)
         if self.kernel == "staged":
             check(
                 _lib.lib.mvb_vecdot_staged(
