@@ -104,6 +104,8 @@ __device__ __forceinline__ float2 load_grid(const float *g, int64_t o, bool whol
 // The four complex planes of every beam, (nbeam, 4, points) -> (nbeam, points, 4).
 __global__ void beam_pack_kernel(const float2 *__restrict__ grids, int64_t points, int nbeam,
                                  float4 *__restrict__ packed) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t total = (int64_t)nbeam * points;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = i / points, p = i % points;
@@ -123,7 +125,9 @@ __global__ void __launch_bounds__(kBeamThreads)
                        const BeamParams *__restrict__ params, const double *__restrict__ crd, int64_t ld,
                        const int32_t *__restrict__ n_dev, int64_t nsrc, void *__restrict__ out, int out_kind,
                        int64_t nout, int32_t *__restrict__ status) {
-  const int64_t n = n_dev ? min((int64_t)*n_dev, nsrc) : nsrc;
+  pdl_wait();
+  pdl_trigger();
+  const int64_t n = n_dev ? min((int64_t)__ldcg(n_dev), nsrc) : nsrc;
   const bool whole = reinterpret_cast<uintptr_t>(grids) % 8 == 0;
   const int b0 = blockIdx.y * per_y, b1 = min(b0 + per_y, nbeam);
   const int64_t points = (int64_t)nza * naz;
@@ -135,10 +139,10 @@ __global__ void __launch_bounds__(kBeamThreads)
     }
     double az, za;
     if constexpr (AZZA) {
-      az = crd[i];
-      za = crd[ld + i];
+      az = __ldcg(crd + i);
+      za = __ldcg(crd + ld + i);
     } else {
-      az_za_uvbeam(crd[i], crd[ld + i], az, za);
+      az_za_uvbeam(__ldcg(crd + i), __ldcg(crd + ld + i), az, za);
     }
     bool finite = true;
     for (int b = b0; b < b1; ++b) {
@@ -152,8 +156,9 @@ __global__ void __launch_bounds__(kBeamThreads)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-          const float4 v00 = c.in ? __ldg(g + 2 * c.o00 + h) : z4, v01 = c.in ? __ldg(g + 2 * c.o01 + h) : z4;
-          const float4 v10 = c.in ? __ldg(g + 2 * c.o10 + h) : z4, v11 = c.in ? __ldg(g + 2 * c.o11 + h) : z4;
+          // packed by the kernel before
+          const float4 v00 = c.in ? __ldca(g + 2 * c.o00 + h) : z4, v01 = c.in ? __ldca(g + 2 * c.o01 + h) : z4;
+          const float4 v10 = c.in ? __ldca(g + 2 * c.o10 + h) : z4, v11 = c.in ? __ldca(g + 2 * c.o11 + h) : z4;
           v[4 * h + 0] = blend(c, v00.x, v01.x, v10.x, v11.x);
           v[4 * h + 1] = blend(c, v00.y, v01.y, v10.y, v11.y);
           v[4 * h + 2] = blend(c, v00.z, v01.z, v10.z, v11.z);
@@ -197,12 +202,14 @@ __global__ void __launch_bounds__(kBeamThreads)
 __global__ void beam_gaussian_kernel(const double *__restrict__ sigmas, int nbeam, const double *__restrict__ crd,
                                      int64_t ld, const int32_t *__restrict__ n_dev, int64_t nsrc, void *__restrict__ out,
                                      int out_c128, int64_t nout) {
-  const int64_t n = n_dev ? min((int64_t)*n_dev, nsrc) : nsrc;
+  pdl_wait();
+  pdl_trigger();
+  const int64_t n = n_dev ? min((int64_t)__ldcg(n_dev), nsrc) : nsrc;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nout; i += (int64_t)gridDim.x * blockDim.x) {
     double za = 0.0;
     if (i < n) {
       double az;
-      az_za_uvbeam(crd[i], crd[ld + i], az, za);
+      az_za_uvbeam(__ldcg(crd + i), __ldcg(crd + ld + i), az, za);
     }
     for (int b = 0; b < nbeam; ++b) {
       const double s = sigmas[b];
@@ -251,9 +258,8 @@ static int beam_interp_impl(bool azza, const void *grids, int grid_kind, int nbe
   const int out_kind = (out_c128 ? 1 : 0) + (reinterpret_cast<uintptr_t>(out) % (out_c128 ? 16 : 8) ? 2 : 0);
   if (pack) {
     const int64_t blocks = std::min<int64_t>(ceil_div(nbeam * points, 256), (int64_t)nsm * 8);
-    beam_pack_kernel<<<(unsigned)blocks, 256, 0, s>>>(static_cast<const float2 *>(grids), points, nbeam,
-                                                      static_cast<float4 *>(ws));
-    int rc = check_launch("beam_pack_kernel");
+    int rc = launch_chained("beam_pack_kernel", beam_pack_kernel, (unsigned)blocks, 256, 0, s,
+                            static_cast<const float2 *>(grids), points, nbeam, static_cast<float4 *>(ws));
     if (rc) return rc;
     g = static_cast<const float *>(ws);
   }
@@ -263,23 +269,12 @@ static int beam_interp_impl(bool azza, const void *grids, int grid_kind, int nbe
   const dim3 grid((unsigned)xblocks, (unsigned)std::min<int64_t>(ceil_div(nbeam, per_y), 65535));
   const int per = (int)ceil_div(nbeam, grid.y);
 #define MVB_BEAM(KIND, AZZA)                                                                                          \
-  beam_gather_kernel<KIND, AZZA><<<grid, kBeamThreads, 0, s>>>(g, nbeam, per, nax, nfeed, nza, naz, bp, crd, ld, n_dev, \
-                                                               nsrc, out, out_kind, nout, status)
-  if (pack)
-    MVB_BEAM(2, false);
-  else if (grid_kind == 0) {
-    if (azza)
-      MVB_BEAM(0, true);
-    else
-      MVB_BEAM(0, false);
-  } else {
-    if (azza)
-      MVB_BEAM(1, true);
-    else
-      MVB_BEAM(1, false);
-  }
+  launch_chained("beam_gather_kernel", beam_gather_kernel<KIND, AZZA>, grid, kBeamThreads, 0, s, g, nbeam, per, nax,  \
+                 nfeed, nza, naz, bp, crd, ld, n_dev, nsrc, out, out_kind, nout, status)
+  if (pack) return MVB_BEAM(2, false);
+  if (grid_kind == 0) return azza ? MVB_BEAM(0, true) : MVB_BEAM(0, false);
+  return azza ? MVB_BEAM(1, true) : MVB_BEAM(1, false);
 #undef MVB_BEAM
-  return check_launch("beam_gather_kernel");
 }
 
 extern "C" size_t mvb_beam_interp_ws_bytes(int nbeam, int64_t nout) {
@@ -309,7 +304,6 @@ extern "C" int mvb_beam_gaussian(const double *sigmas, int nbeam, const double *
   if (nout == 0) return MVB_OK;
   const int threads = 256;
   const int64_t blocks = std::min<int64_t>(ceil_div(nout, threads), (int64_t)num_sms() * 8);
-  beam_gaussian_kernel<<<(unsigned)blocks, threads, 0, as_stream(stream)>>>(sigmas, nbeam, crd, ld, n_dev, nsrc, out,
-                                                                            out_c128, nout);
-  return check_launch("beam_gaussian_kernel");
+  return launch_chained("beam_gaussian_kernel", beam_gaussian_kernel, (unsigned)blocks, threads, 0, as_stream(stream),
+                        sigmas, nbeam, crd, ld, n_dev, nsrc, out, out_c128, nout);
 }

@@ -37,6 +37,33 @@ inline int check_launch(const char *what) {
 
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Launch of a kernel of the job chain, allowed to start while its predecessor in
+// the stream drains (programmatic dependent launch): block scheduling, barrier and
+// tensor-memory set-up overlap the predecessor's tail.  Such a kernel calls
+// pdl_wait() before it touches global memory -- it returns when every earlier
+// kernel of the stream is complete, since each of them waited too -- and
+// pdl_trigger() once its successor may be scheduled.
+template <typename... KArgs, typename... Args>
+inline int launch_chained(const char *what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                          cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(MVB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  }
+  return MVB_OK;
+}
+
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 __host__ __device__ inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
 
@@ -45,6 +72,22 @@ int num_sms();
 // slots 16..45 are the Hermitian-product variants,
 // 48 and 49 the staged pair kernels.
 int set_smem_once(const void *fn, int bytes, int slot);
+// mvb_herk_grouped with its work-unit counter left as it is (it must be 0), and
+// mvb_herk_reduce_grouped that also clears it for the next product of the same
+// workspace: a job's launch sequence, which clears it once (clear_unit_counter).
+int herk_grouped_chained(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t Kcap,
+                         const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps, void *ws,
+                         size_t ws_bytes, int32_t *status, void *stream);
+int herk_reduce_grouped_chained(void *ws, size_t ws_bytes, int ngroup, int64_t Mpad, int64_t Kcap,
+                                const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int nant, int nfeed,
+                                const int32_t *pairs, int64_t npairs, void *out, size_t out_stride, int out_c128,
+                                double vscale, int accumulate, void *stream);
+int clear_unit_counter(void *ws, size_t ws_bytes, void *stream);
+// mvb_rotate and mvb_horizon_compact of all n sources (no fluxes) with the count in
+// the rotation's pass.
+int rotate_select(const double *src, int64_t n, const double *R, double *topo, double *crd_out, int32_t *idx_out,
+                  int32_t *n_out, int64_t cap, int32_t *status, void *ws, size_t ws_bytes, void *stream);
+
 // Wall-time limit of a pipeline wait in the product and the staged pair kernel
 // (process-wide, set by mvb_set_wait_limit_ns; 4 s by default).
 uint64_t wait_limit_ns();
@@ -82,6 +125,11 @@ __host__ __device__ constexpr int64_t panel_plane_stride(int kb) { return 128 * 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+
+// See launch_chained.  What a predecessor wrote is read with __ldcg / __ldca after
+// the wait, never through the read-only path (a compiler may move such loads).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ uint64_t global_timer_ns() {
   uint64_t t;

@@ -43,8 +43,8 @@
 // panels of one shape (the frequencies of a time step, zstride bytes apart)
 // that share the column count; with ngroup = 1 it is one product.
 // Persistent CTAs (one per SM, 192 KB of shared memory) take units in index
-// order from a counter in the workspace (zeroed on the stream before each
-// launch), so a CTA that drew cheaper diagonal tiles takes more units: with
+// order from a counter in the workspace (0 at each launch), after a
+// first one of their own index, so a CTA that drew cheaper diagonal tiles takes more units: with
 // static round-robin the CTAs' loads differed by up to a tile's work (one
 // panel of 700 rows: 0.92-0.96 of the mean).  Each unit's sums do not depend
 // on which CTA computes it.  Warp roles (576 threads):
@@ -73,6 +73,7 @@
 // (each drain wait bounded by kDrainLimitNs), frees TMEM and returns.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -156,7 +157,7 @@ __device__ __forceinline__ void plan_splits(int64_t kvalid, int n_tiles, int kma
 
 // Valid K columns: (source count) x (columns per source), clamped to the panel.
 __device__ __forceinline__ int64_t valid_k(const int32_t *n_dev, int64_t n_host, int kmul, int64_t Kcap) {
-  int64_t n = n_dev ? (int64_t)*n_dev : n_host;
+  int64_t n = n_dev ? (int64_t)__ldcg(n_dev) : n_host;
   n = n < 0 ? 0 : n;
   return min(n * kmul, Kcap);
 }
@@ -198,6 +199,7 @@ struct HerkTable {
   HerkPanel p[kMaxBatchPanels];
   int n;
 };
+struct NoTable {};  // a launch of one repeated shape does not carry the table's 2.6 KB of parameters
 
 // KD: k-steps accumulated in one TMEM block before it is drained (1, 2 or 4).
 // TABLE: the units come from the table (a batch) instead of one repeated shape.
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
     herk_kernel(const uint8_t *__restrict__ zpanels, int64_t zstride, int ngroup, int T, int n_tiles,
                 const int32_t *__restrict__ n_dev, int64_t n_host, int kmul, int64_t Kcap, int k_chunk, int nsm,
                 float *__restrict__ partials, int32_t *__restrict__ status, int *__restrict__ unit_next,
-                uint64_t wait_ns, const __grid_constant__ HerkTable table) {
+                uint64_t wait_ns, const __grid_constant__ std::conditional_t<TABLE, HerkTable, NoTable> table) {
   using C = HerkCfg<MODE>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[C::STAGES];
@@ -226,6 +228,34 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr bool tabled = TABLE;
+  // barriers and tensor memory, while the kernel before this one may still run
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&dfull_bar[b], 1);
+      mbar_init(&dempty_bar[b], kEpiWarps);
+    }
+    mbar_init(&drain_bar, 1);
+    for (int i = 0; i < kUnitRing; ++i) {
+      mbar_init(&ufull_bar[i], 1);
+      mbar_init(&uempty_bar[i], 1 + kEpiWarps);
+    }
+    abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&tmem_base_sh, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tbase = tmem_base_sh;
+  pdl_wait();
+
   int64_t kvalid = 0, kc = 0;
   int per_panel = 0, n_units;
   if constexpr (tabled) {
@@ -256,7 +286,10 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
     per_panel = n_tiles * nsplit;
     n_units = per_panel * ngroup;
   }
-  if ((int)blockIdx.x >= n_units) return;  // uniform over the CTA
+  if ((int)blockIdx.x >= n_units) {  // uniform over the CTA
+    if (warp == 1) tmem_dealloc(tbase, 512);
+    return;
+  }
 
   // Where unit u is: its panel and block count, tile, columns and partial tile.
   auto place = [&](int u, const uint8_t *&zpanel, float *&partial, int &Tu, int &I, int &J, int64_t &k0,
@@ -293,32 +326,6 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
 
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&dfull_bar[b], 1);
-      mbar_init(&dempty_bar[b], kEpiWarps);
-    }
-    mbar_init(&drain_bar, 1);
-    for (int i = 0; i < kUnitRing; ++i) {
-      mbar_init(&ufull_bar[i], 1);
-      mbar_init(&uempty_bar[i], 1 + kEpiWarps);
-    }
-    abort_flag = 0;
-    fence_mbar_init();
-  }
-  if (warp == 1) {
-    tmem_alloc(&tmem_base_sh, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tbase = tmem_base_sh;
-
   uint64_t issued = 0;            // producer: stages issued
   bool lead = warp == 1 && lane == 0;  // the thread that issues the UMMAs
   if (warp == 0 && lane == 0) {
@@ -332,7 +339,8 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
         abort_flag = 1;
         break;
       }
-      const int u = min(atomicAdd(unit_next, 1), n_units);
+      // (the first is its own index: no atomic before the first load)
+      const int u = uk == 0 ? (int)blockIdx.x : min(atomicAdd(unit_next, 1) + (int)gridDim.x, n_units);
       unit_q[us] = u;
       mbar_arrive(&ufull_bar[us]);
       if (u >= n_units) break;
@@ -666,6 +674,7 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
     }
   }
 
+  pdl_trigger();  // this CTA's units are done
   __syncthreads();
   if (abort_flag) {
     if (warp == 0 && lane == 0) {
@@ -736,7 +745,7 @@ __device__ __forceinline__ void sum_slices(const float4 *const (&p)[NP], int nsp
     for (int u = 0; u < U; ++u)
       if (s + u < nsplit) {
 #pragma unroll
-        for (int k = 0; k < NP; ++k) v[u][k] = __ldg(p[k] + (s + u) * sstride);
+        for (int k = 0; k < NP; ++k) v[u][k] = __ldcg(p[k] + (s + u) * sstride);
       }
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -774,8 +783,11 @@ __global__ void __launch_bounds__(kRedThreads, 2)
     herk_reduce_all_kernel(const float *__restrict__ part, int ngroup, int T, int n_tiles,
                            const int32_t *__restrict__ n_dev, int64_t n_host, int kmul, int64_t Kcap, int k_chunk,
                            int nsm, int A, void *__restrict__ out_base, int64_t out_stride, double vscale,
-                           const float *__restrict__ zscale, int accumulate) {
+                           const float *__restrict__ zscale, int accumulate, int *__restrict__ unit_next) {
   __shared__ FF turn_sm[32][33];
+  pdl_wait();
+  pdl_trigger();
+  if (unit_next && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *unit_next = 0;  // for the next product
   const int t = blockIdx.x / kRedBlocks, rb = blockIdx.x % 4, cb = blockIdx.x / 4 % 4;
   int I, J;
   decode_tile(t, T, I, J);
@@ -840,8 +852,12 @@ __global__ void herk_reduce_pairs_kernel(const float *__restrict__ part, int ngr
                                          const int32_t *__restrict__ n_dev, int64_t n_host, int kmul, int64_t Kcap,
                                          int k_chunk, int nsm, int A, int F, const int32_t *__restrict__ pairs,
                                          int64_t npairs, void *__restrict__ out_base, int64_t out_stride,
-                                         double vscale, const float *__restrict__ zscale, int accumulate) {
+                                         double vscale, const float *__restrict__ zscale, int accumulate,
+                                         int *__restrict__ unit_next) {
   const int64_t total = npairs * F * F;
+  pdl_wait();
+  pdl_trigger();
+  if (unit_next && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *unit_next = 0;  // for the next product
   const int64_t kvalid = valid_k(n_dev, n_host, kmul, Kcap);
   int nsplit;
   int64_t kc;
@@ -878,9 +894,9 @@ __global__ void herk_reduce_pairs_kernel(const float *__restrict__ part, int ngr
       for (int u = 0; u < U; ++u)
         if (s + u < nsplit) {
           const float *ps = p0 + (s + u) * sstride;
-          vr[u] = __ldg(ps + c * 128 + r);
-          vi[u] = __ldg(ps + (128 + c) * 128 + r);
-          if (diag) vt[u] = __ldg(ps + (128 + r) * 128 + c);
+          vr[u] = __ldcg(ps + c * 128 + r);
+          vi[u] = __ldcg(ps + (128 + c) * 128 + r);
+          if (diag) vt[u] = __ldcg(ps + (128 + r) * 128 + c);
         }
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -922,7 +938,7 @@ uint64_t wait_limit_ns() { return g_wait_limit_ns.load(std::memory_order_relaxed
 template <int MODE, int KD>
 static int launch_herk(const void *z, int64_t zstride, int ngroup, int64_t Mpad, int64_t Kcap, const int32_t *n_dev,
                        int64_t n_host, int kmul, int k_chunk, float *partials, int32_t *status, int *unit_next,
-                       cudaStream_t s, const HerkTable &table) {
+                       bool clear_counter, cudaStream_t s, const HerkTable &table) {
   using C = HerkCfg<MODE>;
   const int T = (int)(Mpad / 128);
   const int n_tiles = T * (T + 1) / 2;
@@ -945,18 +961,17 @@ static int launch_herk(const void *z, int64_t zstride, int ngroup, int64_t Mpad,
   if (rc) return rc;
   if (grid <= 0) return MVB_OK;
   const uint64_t wait_ns = wait_limit_ns();
-  // the CTAs take units from this counter, zeroed on the launch's stream
-  cudaError_t e = cudaMemsetAsync(unit_next, 0, sizeof(int), s);
-  if (e != cudaSuccess) return fail(MVB_ERR_CUDA, "herk unit counter: %s", cudaGetErrorString(e));
+  if (clear_counter) {  // the CTAs take units from this counter
+    cudaError_t e = cudaMemsetAsync(unit_next, 0, sizeof(int), s);
+    if (e != cudaSuccess) return fail(MVB_ERR_CUDA, "herk unit counter: %s", cudaGetErrorString(e));
+  }
   if (table.n > 0)
-    herk_kernel<MODE, KD, true><<<grid, kHerkThreads, smem, s>>>(static_cast<const uint8_t *>(z), zstride, ngroup, T,
-                                                                 n_tiles, n_dev, n_host, kmul, Kcap, k_chunk, nsm,
-                                                                 partials, status, unit_next, wait_ns, table);
-  else
-    herk_kernel<MODE, KD, false><<<grid, kHerkThreads, smem, s>>>(static_cast<const uint8_t *>(z), zstride, ngroup, T,
-                                                                  n_tiles, n_dev, n_host, kmul, Kcap, k_chunk, nsm,
-                                                                  partials, status, unit_next, wait_ns, table);
-  return check_launch("herk_kernel");
+    return launch_chained("herk_kernel", herk_kernel<MODE, KD, true>, grid, kHerkThreads, smem, s,
+                          static_cast<const uint8_t *>(z), zstride, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap,
+                          k_chunk, nsm, partials, status, unit_next, wait_ns, table);
+  return launch_chained("herk_kernel", herk_kernel<MODE, KD, false>, grid, kHerkThreads, smem, s,
+                        static_cast<const uint8_t *>(z), zstride, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap,
+                        k_chunk, nsm, partials, status, unit_next, wait_ns, NoTable{});
 }
 
 // Argument checks shared by the product and its reductions (the slice plan
@@ -990,9 +1005,15 @@ static int check_herk_group(const char *who, const void *z, int64_t zstride, int
   return MVB_OK;
 }
 
+// Past every partial tile: each group's share of ws_bytes holds kCounterBytes spare.
+static int *unit_counter(void *ws, size_t ws_bytes) {
+  return reinterpret_cast<int *>(static_cast<uint8_t *>(ws) + ((ws_bytes - 16) & ~size_t(15)));
+}
+
 static int herk_impl(const char *who, const void *z, int64_t zstride, int ngroup, int mode, int64_t Mpad, int64_t Kcap,
                      const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps, void *ws,
-                     size_t ws_bytes, int32_t *status, void *stream, const HerkTable &table = HerkTable{}) {
+                     size_t ws_bytes, int32_t *status, void *stream, const HerkTable &table = HerkTable{},
+                     bool clear_counter = true) {
   if (table.n == 0) {
     int rc = check_herk_group(who, z, zstride, ngroup, mode, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, ws, ws_bytes,
                               status);
@@ -1004,15 +1025,14 @@ static int herk_impl(const char *who, const void *z, int64_t zstride, int ngroup
   const int kd = drain_ksteps ? drain_ksteps : 2;
   cudaStream_t s = as_stream(stream);
   float *part = static_cast<float *>(ws);
-  // past every partial tile: each group's share of ws_bytes holds kCounterBytes spare
-  int *next = reinterpret_cast<int *>(static_cast<uint8_t *>(ws) + ((ws_bytes - 16) & ~size_t(15)));
+  int *next = unit_counter(ws, ws_bytes);
 #define MVB_HERK(M)                                                                                          \
   return kd == 1   ? launch_herk<M, 1>(z, zstride, ngroup, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
-                                       next, s, table)                                                       \
+                                       next, clear_counter, s, table)                                                       \
          : kd == 2 ? launch_herk<M, 2>(z, zstride, ngroup, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
-                                       next, s, table)                                                       \
+                                       next, clear_counter, s, table)                                                       \
                    : launch_herk<M, 4>(z, zstride, ngroup, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
-                                       next, s, table)
+                                       next, clear_counter, s, table)
   switch (mode) {
     case MVB_GEMM_BF16_3: MVB_HERK(MVB_GEMM_BF16_3);
     case MVB_GEMM_BF16_6: MVB_HERK(MVB_GEMM_BF16_6);
@@ -1026,7 +1046,7 @@ static int herk_impl(const char *who, const void *z, int64_t zstride, int ngroup
 static int reduce_impl(const char *who, const void *ws, size_t ws_bytes, int ngroup, int64_t Mpad, int64_t Kcap,
                        const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int nant, int nfeed,
                        const int32_t *pairs, int64_t npairs, void *out, int64_t out_stride, int out_c128,
-                       double vscale, const float *zscale, int accumulate, void *stream) {
+                       double vscale, const float *zscale, int accumulate, void *stream, int *unit_next = nullptr) {
   // the checks of mvb_herk: the slice plan recomputed here is then the product's
   if (!ws || !out || nant <= 0 || (nfeed != 1 && nfeed != 2) || (int64_t)nant * nfeed > Mpad || (pairs && npairs < 0))
     return fail(MVB_ERR_ARG, "%s: bad arguments", who);
@@ -1046,9 +1066,9 @@ static int reduce_impl(const char *who, const void *ws, size_t ws_bytes, int ngr
   if (!pairs) {
     const dim3 grid((unsigned)(n_tiles * kRedBlocks), (unsigned)ngroup);
 #define MVB_RED(OT, FF_)                                                                                           \
-  herk_reduce_all_kernel<OT, FF_><<<grid, kRedThreads, 0, s>>>(part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap, \
-                                                               k_chunk, nsm, nant, out, out_stride, vscale, zscale, \
-                                                               accumulate)
+  return launch_chained(who, herk_reduce_all_kernel<OT, FF_>, grid, kRedThreads, 0, s, part, ngroup, T, n_tiles,   \
+                        n_dev, n_host, kmul, Kcap, k_chunk, nsm, nant, out, out_stride, vscale, zscale, accumulate, \
+                        unit_next)
     if (out_c128) {
       if (nfeed == 2) MVB_RED(double2, 2); else MVB_RED(double2, 1);
     } else {
@@ -1059,16 +1079,31 @@ static int reduce_impl(const char *who, const void *ws, size_t ws_bytes, int ngr
     if (npairs == 0) return MVB_OK;
     const int64_t total = npairs * nfeed * nfeed;
     const dim3 grid((unsigned)std::min<int64_t>(ceil_div(total, 256), (int64_t)nsm * 8), (unsigned)ngroup);
-    if (out_c128)
-      herk_reduce_pairs_kernel<double2><<<grid, 256, 0, s>>>(part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap,
-                                                             k_chunk, nsm, nant, nfeed, pairs, npairs, out, out_stride,
-                                                             vscale, zscale, accumulate);
-    else
-      herk_reduce_pairs_kernel<float2><<<grid, 256, 0, s>>>(part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap,
-                                                            k_chunk, nsm, nant, nfeed, pairs, npairs, out, out_stride,
-                                                            vscale, zscale, accumulate);
+    const auto kernel = out_c128 ? herk_reduce_pairs_kernel<double2> : herk_reduce_pairs_kernel<float2>;
+    return launch_chained(who, kernel, grid, 256, 0, s, part, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap, k_chunk,
+                          nsm, nant, nfeed, pairs, npairs, out, out_stride, vscale, zscale, accumulate, unit_next);
   }
-  return check_launch(who);
+}
+
+int herk_grouped_chained(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t Kcap,
+                         const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps, void *ws,
+                         size_t ws_bytes, int32_t *status, void *stream) {
+  return herk_impl("mvb_herk_grouped", z, (int64_t)z_stride, ngroup, mode, Mpad, Kcap, n_dev, n_host, kmul, k_chunk,
+                   drain_ksteps, ws, ws_bytes, status, stream, HerkTable{}, false);
+}
+
+int herk_reduce_grouped_chained(void *ws, size_t ws_bytes, int ngroup, int64_t Mpad, int64_t Kcap,
+                                const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int nant, int nfeed,
+                                const int32_t *pairs, int64_t npairs, void *out, size_t out_stride, int out_c128,
+                                double vscale, int accumulate, void *stream) {
+  return reduce_impl("mvb_herk_reduce_grouped", ws, ws_bytes, ngroup, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, nant,
+                     nfeed, pairs, npairs, out, (int64_t)out_stride, out_c128, vscale, nullptr, accumulate, stream,
+                     unit_counter(ws, ws_bytes));
+}
+
+int clear_unit_counter(void *ws, size_t ws_bytes, void *stream) {
+  cudaError_t e = cudaMemsetAsync(unit_counter(ws, ws_bytes), 0, sizeof(int), as_stream(stream));
+  return e == cudaSuccess ? MVB_OK : fail(MVB_ERR_CUDA, "herk unit counter: %s", cudaGetErrorString(e));
 }
 
 }  // namespace mvb

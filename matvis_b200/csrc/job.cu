@@ -7,7 +7,8 @@
 // Every call below is one of the library's own entry points.  A small job is a few
 // hundred launches of 2 to 20 us; made one by one through the Python binding they
 // cost 10 to 16 us of host time each (37 antennas x 5,003 sources x 7 frequencies x
-// 5 times: 478 us a run for 290 us of kernels; 361 us from here, one call a run).
+// 5 times: 478 us a run for 290 us of kernels; 361 us from here, one call a run, and
+// 290 us with the kernels launched as a chain: launch_chained).
 #include <algorithm>
 
 #include "common.cuh"
@@ -22,6 +23,9 @@ static int job_prologue(const mvb_job &j, int t, int c, void *stream) {
       if (j.refresh[t] && (rc = mvb_bcrs(j.eci, j.nsrc, j.astrom + 18 * (int64_t)t, j.bcrs, stream))) return rc;
       src = j.bcrs;
     }
+    if (j.nchunks == 1)
+      return rotate_select(src, j.nsrc, j.rot + 9 * (int64_t)t, j.topo, j.crd, j.kept, j.n_above, j.cap, j.status,
+                           j.select_ws, j.select_ws_bytes, stream);
     if ((rc = mvb_rotate(src, j.nsrc, j.rot + 9 * (int64_t)t, j.topo, stream))) return rc;
   }
   const int64_t c0 = std::min<int64_t>(c * j.chunk_size, j.nsrc), c1 = std::min<int64_t>((c + 1) * j.chunk_size, j.nsrc);
@@ -69,10 +73,10 @@ static int job_group(const mvb_job &j, int t, int f0, int g, int accumulate, voi
     return mvb_vecdot(j.z, j.Kcap, j.n_above, j.cap, F, F, j.pairs, j.npairs, j.k_chunk, j.ws, j.ws_bytes, out,
                       j.out_c128, accumulate, stream);
   }
-  if ((rc = mvb_herk_grouped(j.z, j.z_stride, g, j.mode, j.Mpad, j.Kcap, j.n_above, j.cap, F, j.k_chunk,
+  if ((rc = herk_grouped_chained(j.z, j.z_stride, g, j.mode, j.Mpad, j.Kcap, j.n_above, j.cap, F, j.k_chunk,
                              j.drain_ksteps, j.ws, j.ws_bytes, j.status, stream)))
     return rc;
-  return mvb_herk_reduce_grouped(j.ws, j.ws_bytes, g, j.Mpad, j.Kcap, j.n_above, j.cap, F, j.k_chunk, j.nant, F,
+  return herk_reduce_grouped_chained(j.ws, j.ws_bytes, g, j.Mpad, j.Kcap, j.n_above, j.cap, F, j.k_chunk, j.nant, F,
                                  j.pairs, j.npairs, out, (size_t)j.vis_f_stride, j.out_c128,
                                  1.0 / ((double)j.zscale * j.zscale), accumulate, stream);
 }
@@ -88,6 +92,8 @@ extern "C" int mvb_job_enqueue(const mvb_job *job, int t0, int t1, int c0, int c
       (j.mode == MVB_Z_C64 && (j.freq_group != 1 || (!j.plan && !j.pairs && j.npairs))))
     return fail(MVB_ERR_ARG, "%s: bad arguments", who);
   int rc;
+  // the products' work-unit counter: cleared here, then by each reduction
+  if (t0 < t1 && c0 < c1 && f0 < f1 && j.mode != MVB_Z_C64 && (rc = clear_unit_counter(j.ws, j.ws_bytes, stream))) return rc;
   for (int t = t0; t < t1; ++t)
     for (int c = c0; c < c1; ++c) {
       if (f0 == 0) {

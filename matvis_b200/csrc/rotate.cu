@@ -12,6 +12,7 @@
 // (ballot + popc) and a scatter pass in which each block sums the counts of the
 // blocks before it, then ranks its own sources with warp ballots.  No block
 // waits on another, so there is no inter-block spin.
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -22,16 +23,20 @@ struct Rot3 {
   double r[9];
 };
 
+__device__ __forceinline__ double rotate_row(const Rot3 &R, int r, double x, double y, double z) {
+  const double a = __dmul_rn(R.r[3 * r + 0], x);
+  const double b = __dmul_rn(R.r[3 * r + 1], y);
+  const double c = __dmul_rn(R.r[3 * r + 2], z);
+  return __dadd_rn(__dadd_rn(a, b), c);
+}
+
 __global__ void rotate_kernel(const double *__restrict__ eci, int64_t n, Rot3 R, double *__restrict__ topo) {
+  pdl_wait();
+  pdl_trigger();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double x = eci[i], y = eci[n + i], z = eci[2 * n + i];
+    const double x = __ldcg(eci + i), y = __ldcg(eci + n + i), z = __ldcg(eci + 2 * n + i);
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const double a = __dmul_rn(R.r[3 * r + 0], x);
-      const double b = __dmul_rn(R.r[3 * r + 1], y);
-      const double c = __dmul_rn(R.r[3 * r + 2], z);
-      topo[r * n + i] = __dadd_rn(__dadd_rn(a, b), c);
-    }
+    for (int r = 0; r < 3; ++r) topo[r * n + i] = rotate_row(R, r, x, y, z);
   }
 }
 
@@ -39,26 +44,60 @@ constexpr int kCompactThreads = 256;
 constexpr int kCompactPerThread = 4;
 constexpr int kCompactBlock = kCompactThreads * kCompactPerThread;  // sources per block
 
+// Sum of one count per thread over the CTA (every thread gets it).
+__device__ __forceinline__ int block_count(int mine, int *warp_tot) {
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = mine;
+  __syncthreads();
+  int s = 0;
+  for (int w = 0; w < kCompactThreads / 32; ++w) s += warp_tot[w];
+  return s;
+}
+
 __global__ void __launch_bounds__(kCompactThreads) horizon_count_kernel(const double *__restrict__ zrow, int64_t count,
                                                                          int32_t *__restrict__ block_counts) {
   __shared__ int warp_tot[kCompactThreads / 32];
+  pdl_wait();
+  pdl_trigger();
   const int64_t base = (int64_t)blockIdx.x * kCompactBlock;
   int mine = 0;
 #pragma unroll
   for (int j = 0; j < kCompactPerThread; ++j) {
     const int64_t i = base + j * kCompactThreads + threadIdx.x;
-    mine += (i < count && zrow[i] > 0.0) ? 1 : 0;
+    mine += (i < count && __ldcg(zrow + i) > 0.0) ? 1 : 0;
   }
-  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-  if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = mine;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int w = 0; w < kCompactThreads / 32; ++w) s += warp_tot[w];
-    block_counts[blockIdx.x] = s;
-  }
+  const int s = block_count(mine, warp_tot);
+  if (threadIdx.x == 0) block_counts[blockIdx.x] = s;
 }
 
+// rotate_kernel and horizon_count_kernel in one pass over all n sources: a launch
+// and a read of the z row fewer.
+__global__ void __launch_bounds__(kCompactThreads)
+    rotate_count_kernel(const double *__restrict__ src, int64_t n, Rot3 R, double *__restrict__ topo,
+                        int32_t *__restrict__ block_counts) {
+  __shared__ int warp_tot[kCompactThreads / 32];
+  pdl_wait();
+  pdl_trigger();
+  const int64_t base = (int64_t)blockIdx.x * kCompactBlock;
+  int mine = 0;
+#pragma unroll
+  for (int j = 0; j < kCompactPerThread; ++j) {
+    const int64_t i = base + j * kCompactThreads + threadIdx.x;
+    if (i < n) {
+      const double x = __ldcg(src + i), y = __ldcg(src + n + i), z = __ldcg(src + 2 * n + i);
+      topo[i] = rotate_row(R, 0, x, y, z);
+      topo[n + i] = rotate_row(R, 1, x, y, z);
+      const double up = rotate_row(R, 2, x, y, z);
+      topo[2 * n + i] = up;
+      mine += up > 0.0 ? 1 : 0;
+    }
+  }
+  const int s = block_count(mine, warp_tot);
+  if (threadIdx.x == 0) block_counts[blockIdx.x] = s;
+}
+
+// Four consecutive sources a thread, so that one scan of per-thread counts ranks the
+// block (four rounds of 256 sources with three barriers each before).
 __global__ void __launch_bounds__(kCompactThreads)
     horizon_scatter_kernel(const double *__restrict__ topo, int64_t ld, int64_t c0, int64_t count,
                            const int32_t *__restrict__ block_counts, int nblocks, const double *__restrict__ flux,
@@ -67,21 +106,37 @@ __global__ void __launch_bounds__(kCompactThreads)
   __shared__ long long red_before[kCompactThreads / 32];
   __shared__ long long red_total[kCompactThreads / 32];
   __shared__ int warp_cnt[kCompactThreads / 32];
-  __shared__ int warp_off[kCompactThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_wait();
+  pdl_trigger();
+
+  const double *zr = topo + 2 * ld + c0;
+  const int64_t i0 = (int64_t)blockIdx.x * kCompactBlock + threadIdx.x * kCompactPerThread;
+  double z[kCompactPerThread];
+#pragma unroll
+  for (int j = 0; j < kCompactPerThread; ++j) z[j] = i0 + j < count ? __ldcg(zr + i0 + j) : 0.0;
 
   // counts of earlier blocks, and the grand total
   long long before = 0, total = 0;
   for (int b = threadIdx.x; b < nblocks; b += kCompactThreads) {
-    const long long c = block_counts[b];
+    const long long c = __ldcg(block_counts + b);
     total += c;
     if (b < (int)blockIdx.x) before += c;
+  }
+  unsigned keep = 0;
+#pragma unroll
+  for (int j = 0; j < kCompactPerThread; ++j) keep |= (z[j] > 0.0 ? 1u : 0u) << j;
+  int scan = __popc(keep);  // becomes the warp's inclusive scan
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, scan, o);
+    if (lane >= o) scan += v;
   }
   for (int o = 16; o > 0; o >>= 1) {
     before += __shfl_xor_sync(0xffffffffu, before, o);
     total += __shfl_xor_sync(0xffffffffu, total, o);
   }
-  if (lane == 0) {
+  if (lane == 31) {
+    warp_cnt[warp] = scan;
     red_before[warp] = before;
     red_total[warp] = total;
   }
@@ -89,43 +144,22 @@ __global__ void __launch_bounds__(kCompactThreads)
   before = 0;
   total = 0;
   for (int w = 0; w < kCompactThreads / 32; ++w) {
-    before += red_before[w];
+    before += red_before[w] + (w < warp ? warp_cnt[w] : 0);
     total += red_total[w];
   }
-
-  const double *xr = topo + c0;
-  const double *yr = topo + ld + c0;
-  const double *zr = topo + 2 * ld + c0;
-  const int64_t base = (int64_t)blockIdx.x * kCompactBlock;
-  long long run = before;
-  if ((int)blockIdx.x < nblocks) {
-    for (int j = 0; j < kCompactPerThread; ++j) {
-      const int64_t i = base + j * kCompactThreads + threadIdx.x;
-      const bool keep = i < count && zr[i] > 0.0;
-      const unsigned m = __ballot_sync(0xffffffffu, keep);
-      if (lane == 0) warp_cnt[warp] = __popc(m);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        int s = 0;
-        for (int w = 0; w < kCompactThreads / 32; ++w) {
-          warp_off[w] = s;
-          s += warp_cnt[w];
-        }
-      }
-      __syncthreads();
-      if (keep) {
-        const long long pos = run + warp_off[warp] + __popc(m & ((1u << lane) - 1u));
-        if (pos < cap) {
-          crd_out[pos] = xr[i];
-          crd_out[cap + pos] = yr[i];
-          crd_out[2 * cap + pos] = zr[i];
-          idx_out[pos] = (int32_t)(c0 + i);
-          if (flux != nullptr) flux_out[pos] = flux[c0 + i];
-        }
-      }
-      run += warp_off[kCompactThreads / 32 - 1] + warp_cnt[kCompactThreads / 32 - 1];
-      __syncthreads();
+  long long pos = before + scan - __popc(keep);
+  const double *xr = topo + c0, *yr = topo + ld + c0;
+#pragma unroll
+  for (int j = 0; j < kCompactPerThread; ++j) {
+    if (!((keep >> j) & 1u)) continue;
+    if (pos < cap) {
+      crd_out[pos] = __ldcg(xr + i0 + j);
+      crd_out[cap + pos] = __ldcg(yr + i0 + j);
+      crd_out[2 * cap + pos] = z[j];
+      idx_out[pos] = (int32_t)(c0 + i0 + j);
+      if (flux != nullptr) flux_out[pos] = flux[c0 + i0 + j];
     }
+    ++pos;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *n_out = (int32_t)total;
@@ -150,6 +184,8 @@ struct Astrom {
 };
 
 __global__ void bcrs_kernel(const double *__restrict__ eci, int64_t n, Astrom a, double *__restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double p0 = eci[i], p1 = eci[n + i], p2 = eci[2 * n + i];
     const double e0 = a.eh[0], e1 = a.eh[1], e2 = a.eh[2];
@@ -187,6 +223,20 @@ __global__ void bcrs_kernel(const double *__restrict__ eci, int64_t n, Astrom a,
 
 using namespace mvb;
 
+// The count pass (unless the rotation has made it) and the scatter pass.
+static int launch_select(const double *topo, int64_t ld, int64_t c0, int64_t count, const double *flux, double *crd_out,
+                         int32_t *idx_out, double *flux_out, int32_t *n_out, int64_t cap, int32_t *status,
+                         int32_t *counts, bool count_pass, cudaStream_t s) {
+  const int nblocks = (int)ceil_div(count, kCompactBlock);
+  if (nblocks > 0 && count_pass) {
+    int rc = launch_chained("horizon_count_kernel", horizon_count_kernel, nblocks, kCompactThreads, 0, s,
+                            topo + 2 * ld + c0, count, counts);
+    if (rc) return rc;
+  }
+  return launch_chained("horizon_scatter_kernel", horizon_scatter_kernel, std::max(nblocks, 1), kCompactThreads, 0, s,
+                        topo, ld, c0, count, counts, nblocks, flux, crd_out, idx_out, flux_out, n_out, cap, status);
+}
+
 extern "C" int mvb_rotate(const double *eci, int64_t N, const double *R, double *topo, void *stream) {
   if (N < 0 || (N > 0 && (!eci || !topo)) || !R) return fail(MVB_ERR_ARG, "mvb_rotate: bad arguments");
   if (N == 0) return MVB_OK;
@@ -194,8 +244,7 @@ extern "C" int mvb_rotate(const double *eci, int64_t N, const double *R, double 
   for (int i = 0; i < 9; ++i) r.r[i] = R[i];
   const int threads = 256;
   const int64_t blocks = std::min<int64_t>(ceil_div(N, threads), (int64_t)num_sms() * 16);
-  rotate_kernel<<<(unsigned)blocks, threads, 0, as_stream(stream)>>>(eci, N, r, topo);
-  return check_launch("rotate_kernel");
+  return launch_chained("rotate_kernel", rotate_kernel, (unsigned)blocks, threads, 0, as_stream(stream), eci, N, r, topo);
 }
 
 extern "C" int mvb_bcrs(const double *eci, int64_t N, const double *astrom, double *bcrs, void *stream) {
@@ -211,8 +260,7 @@ extern "C" int mvb_bcrs(const double *eci, int64_t N, const double *astrom, doub
   if (!(a.em > 0.0) || !(a.bm1 > 0.0)) return fail(MVB_ERR_ARG, "mvb_bcrs: em and bm1 must be positive");
   const int threads = 256;
   const int64_t blocks = std::min<int64_t>(ceil_div(N, threads), (int64_t)num_sms() * 16);
-  bcrs_kernel<<<(unsigned)blocks, threads, 0, as_stream(stream)>>>(eci, N, a, bcrs);
-  return check_launch("bcrs_kernel");
+  return launch_chained("bcrs_kernel", bcrs_kernel, (unsigned)blocks, threads, 0, as_stream(stream), eci, N, a, bcrs);
 }
 
 extern "C" size_t mvb_horizon_ws_bytes(int64_t count) {
@@ -228,19 +276,29 @@ extern "C" int mvb_horizon_compact(const double *topo, int64_t ld, int64_t c0, i
     return fail(MVB_ERR_ARG, "mvb_horizon_compact: bad arguments");
   if (count > INT32_MAX) return fail(MVB_ERR_ARG, "mvb_horizon_compact: chunk too large");
   if (ws_bytes < mvb_horizon_ws_bytes(count)) return fail(MVB_ERR_ARG, "mvb_horizon_compact: workspace too small");
-  const int nblocks = (int)ceil_div(count, kCompactBlock);
-  int32_t *counts = static_cast<int32_t *>(ws);
+  return launch_select(topo, ld, c0, count, flux, crd_out, idx_out, flux_out, n_out, cap, status,
+                       static_cast<int32_t *>(ws), true, as_stream(stream));
+}
+
+namespace mvb {
+int rotate_select(const double *src, int64_t n, const double *R, double *topo, double *crd_out, int32_t *idx_out,
+                  int32_t *n_out, int64_t cap, int32_t *status, void *ws, size_t ws_bytes, void *stream) {
+  if (n < 0 || n > INT32_MAX || (n > 0 && (!src || !topo)) || !R || !n_out || !ws || cap < 0 ||
+      (cap > 0 && (!crd_out || !idx_out)) || ws_bytes < mvb_horizon_ws_bytes(n))
+    return fail(MVB_ERR_ARG, "rotate_select: bad arguments");
   cudaStream_t s = as_stream(stream);
+  const int nblocks = (int)ceil_div(n, kCompactBlock);
   if (nblocks > 0) {
-    horizon_count_kernel<<<nblocks, kCompactThreads, 0, s>>>(topo + 2 * ld + c0, count, counts);
-    int rc = check_launch("horizon_count_kernel");
+    Rot3 r;
+    for (int i = 0; i < 9; ++i) r.r[i] = R[i];
+    int rc = launch_chained("rotate_count_kernel", rotate_count_kernel, nblocks, kCompactThreads, 0, s, src, n, r, topo,
+                            static_cast<int32_t *>(ws));
     if (rc) return rc;
   }
-  const int grid = std::max(nblocks, 1);
-  horizon_scatter_kernel<<<grid, kCompactThreads, 0, s>>>(topo, ld, c0, count, counts, nblocks, flux, crd_out, idx_out,
-                                                         flux_out, n_out, cap, status);
-  return check_launch("horizon_scatter_kernel");
+  return launch_select(topo, n, 0, n, nullptr, crd_out, idx_out, nullptr, n_out, cap, status,
+                       static_cast<int32_t *>(ws), false, s);
 }
+}  // namespace mvb
 
 // ---------------------------------------------------------------------------
 // Allocation-free variant of mvb_horizon_compact.
@@ -302,14 +360,6 @@ extern "C" int mvb_horizon_compact_static(const double *topo, int64_t ld, int64_
   if (rc) return rc;
   // Every count the scatter pass reads is written by the count pass first, so
   // nothing in the shared array has to start at zero.
-  cudaStream_t s = as_stream(stream);
-  if (nblocks > 0) {
-    horizon_count_kernel<<<(unsigned)nblocks, kCompactThreads, 0, s>>>(topo + 2 * ld + c0, count, counts);
-    rc = check_launch("horizon_count_kernel");
-    if (rc) return rc;
-  }
-  const int grid = (int)std::max<int64_t>(nblocks, 1);
-  horizon_scatter_kernel<<<grid, kCompactThreads, 0, s>>>(topo, ld, c0, count, counts, (int)nblocks, flux, crd_out,
-                                                         idx_out, flux_out, n_out, cap, status);
-  return check_launch("horizon_scatter_kernel");
+  return launch_select(topo, ld, c0, count, flux, crd_out, idx_out, flux_out, n_out, cap, status, counts, true,
+                       as_stream(stream));
 }

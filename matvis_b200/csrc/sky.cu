@@ -76,12 +76,14 @@ __device__ __forceinline__ void coherency_rotation_one(double ra, double dec, do
 __global__ void coherency_rotation_kernel(const double *__restrict__ radec, int64_t N, const int32_t *__restrict__ kept,
                                           const double *__restrict__ crd, int64_t ld, const int32_t *__restrict__ n_dev,
                                           int64_t cap, Mat3 ravg, double2 *__restrict__ rot) {
-  const int64_t n = n_dev ? min((int64_t)*n_dev, cap) : cap;
+  pdl_wait();
+  pdl_trigger();
+  const int64_t n = n_dev ? min((int64_t)__ldcg(n_dev), cap) : cap;
   for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t src = kept ? kept[s] : s;
+    const int64_t src = kept ? __ldcg(kept + s) : s;
     if (src < 0 || src >= N) continue;
     double c, sn;
-    coherency_rotation_one(radec[src], radec[N + src], crd[s], crd[ld + s], ravg, c, sn);
+    coherency_rotation_one(radec[src], radec[N + src], __ldcg(crd + s), __ldcg(crd + ld + s), ravg, c, sn);
     rot[s] = make_double2(c, sn);
   }
 }
@@ -134,9 +136,8 @@ extern "C" int mvb_coherency_rotation(const double *radec, int64_t N, const int3
   for (int k = 0; k < 9; ++k) m.m[k] = r_avg[k];
   const int threads = 128;
   const int64_t blocks = std::min<int64_t>(ceil_div(cap, threads), (int64_t)num_sms() * 8);
-  coherency_rotation_kernel<<<(unsigned)blocks, threads, 0, as_stream(stream)>>>(
-      radec, N, kept, crd, ld, n_dev, cap, m, reinterpret_cast<double2 *>(rot));
-  return check_launch("coherency_rotation_kernel");
+  return launch_chained("coherency_rotation_kernel", coherency_rotation_kernel, (unsigned)blocks, threads, 0,
+                        as_stream(stream), radec, N, kept, crd, ld, n_dev, cap, m, reinterpret_cast<double2 *>(rot));
 }
 
 extern "C" int mvb_rotate_coherency(const double *rot, const int32_t *kept, const int32_t *n_dev, const void *coh,

@@ -288,7 +288,9 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
   static_assert(!POL || (X == 2 && F == 2), "the polarised sky needs two feeds and two beam axes");
   constexpr int NS = kTauZCols / X;        // sources per thread
   constexpr int BS = kTauZGroups * NS;     // sources per CTA
-  const int64_t n = p.n_dev ? min((int64_t)*p.n_dev, p.nsrc) : p.nsrc;
+  pdl_wait();
+  pdl_trigger();
+  const int64_t n = p.n_dev ? min((int64_t)__ldcg(p.n_dev), p.nsrc) : p.nsrc;
   const int64_t s_end = round_up(n * X, kKAlign) / X;  // zero-fill up to here: a multiple of BS
   const int64_t sb = (int64_t)blockIdx.x * BS;
   if (sb >= s_end) return;  // uniform per CTA
@@ -307,20 +309,20 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
   const int sl = threadIdx.x % BS, lane0 = threadIdx.x / BS;
   const int64_t s = sb + sl;
   const bool live = s < n;
-  const int64_t src = live && p.sidx ? __ldg(p.sidx + s) : s;
+  const int64_t src = live && p.sidx ? __ldcg(p.sidx + s) : s;
   constexpr int NC = (3 + PER - 1) / PER, NB = kTauZMaxBFX / PER, NG = kTauZMaxFreq / PER;
   double c_in[NC];
 #pragma unroll
-  for (int i = 0; i < NC; ++i) c_in[i] = live && lane0 + i * PER < 3 ? __ldg(p.crd + (lane0 + i * PER) * p.ld + s) : 0.0;
+  for (int i = 0; i < NC; ++i) c_in[i] = live && lane0 + i * PER < 3 ? __ldcg(p.crd + (lane0 + i * PER) * p.ld + s) : 0.0;
   const int nq = p.staged ? p.nbeam * F * X : 0;
   float2 b_in[NB];
 #pragma unroll
   for (int i = 0; i < NB; ++i)
-    b_in[i] = live && lane0 + i * PER < nq ? __ldg(p.beam + (int64_t)(lane0 + i * PER) * p.beam_ld + s)
+    b_in[i] = live && lane0 + i * PER < nq ? __ldcg(p.beam + (int64_t)(lane0 + i * PER) * p.beam_ld + s)
                                            : make_float2(0.f, 0.f);
   if (threadIdx.x < gn) foc_sm[threadIdx.x] = p.freqs ? __ldg(p.freqs + g0 + threadIdx.x) * kInvC : p.f_over_c;
   if constexpr (POL) {
-    const double2 rot = live ? __ldg(p.rot + s) : make_double2(0.0, 0.0);
+    const double2 rot = live ? __ldcg(p.rot + s) : make_double2(0.0, 0.0);
     for (int g = lane0; g < gn; g += PER) {
       float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
       if (live) l = coherency_factor(__ldg(p.coh + (g0 + g) * p.coh_ld + src), rot);
@@ -388,7 +390,7 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
 #pragma unroll
         for (int k = 0; k < kTauZCols; ++k) {
           const int64_t s = sb + sg * NS + k / X;
-          const float2 v1 = s < n ? __ldg(p.beam + (int64_t)((b * F + f) * X + k % X) * p.beam_ld + s)
+          const float2 v1 = s < n ? __ldca(p.beam + (int64_t)((b * F + f) * X + k % X) * p.beam_ld + s)
                                   : make_float2(0.f, 0.f);
           v[k] = make_float2(v1.x * p.scale_beam, v1.y * p.scale_beam);
         }
@@ -793,28 +795,27 @@ extern "C" int mvb_exptau(const double *antpos, int A, double freq, const double
 }
 
 template <int MODE, bool POL, bool GROUP>
-static void launch_tau_z_form(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
+static int launch_tau_z_form(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
   if constexpr (POL) {
-    tau_z_kernel<MODE, 2, 2, true, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+    return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 2, 2, true, GROUP>, grid, kTauZThreads, smem, s, p);
   } else if (X == 2) {
     if (F == 2)
-      tau_z_kernel<MODE, 2, 2, false, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+      return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 2, 2, false, GROUP>, grid, kTauZThreads, smem, s, p);
     else
-      tau_z_kernel<MODE, 2, 1, false, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+      return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 2, 1, false, GROUP>, grid, kTauZThreads, smem, s, p);
   } else {
     if (F == 2)
-      tau_z_kernel<MODE, 1, 2, false, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+      return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 1, 2, false, GROUP>, grid, kTauZThreads, smem, s, p);
     else
-      tau_z_kernel<MODE, 1, 1, false, GROUP><<<grid, kTauZThreads, smem, s>>>(p);
+      return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 1, 1, false, GROUP>, grid, kTauZThreads, smem, s, p);
   }
 }
 
 template <int MODE, bool POL>
-static void launch_tau_z_mode(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
+static int launch_tau_z_mode(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
   if (p.per_z > 1)
-    launch_tau_z_form<MODE, POL, true>(p, F, X, grid, smem, s);
-  else
-    launch_tau_z_form<MODE, POL, false>(p, F, X, grid, smem, s);
+    return launch_tau_z_form<MODE, POL, true>(p, F, X, grid, smem, s);
+  return launch_tau_z_form<MODE, POL, false>(p, F, X, grid, smem, s);
 }
 
 // The launch of both fused writers (arguments checked by the callers).
@@ -876,13 +877,12 @@ static int launch_tau_z(TauZArgs p, const double *antpos, int A, double freq, co
                       (p.staged ? (size_t)nbeam * F * kTauZBeamRow * sizeof(float2) : 0);
   cudaStream_t s = as_stream(stream);
   switch (mode) {
-    case MVB_GEMM_BF16_3: launch_tau_z_mode<MVB_GEMM_BF16_3, POL>(p, F, X, grid, smem, s); break;
-    case MVB_GEMM_BF16_6: launch_tau_z_mode<MVB_GEMM_BF16_6, POL>(p, F, X, grid, smem, s); break;
-    case MVB_GEMM_TF32_3: launch_tau_z_mode<MVB_GEMM_TF32_3, POL>(p, F, X, grid, smem, s); break;
-    case MVB_GEMM_F16_3: launch_tau_z_mode<MVB_GEMM_F16_3, POL>(p, F, X, grid, smem, s); break;
-    default: launch_tau_z_mode<MVB_Z_C64, POL>(p, F, X, grid, smem, s); break;
+    case MVB_GEMM_BF16_3: return launch_tau_z_mode<MVB_GEMM_BF16_3, POL>(p, F, X, grid, smem, s);
+    case MVB_GEMM_BF16_6: return launch_tau_z_mode<MVB_GEMM_BF16_6, POL>(p, F, X, grid, smem, s);
+    case MVB_GEMM_TF32_3: return launch_tau_z_mode<MVB_GEMM_TF32_3, POL>(p, F, X, grid, smem, s);
+    case MVB_GEMM_F16_3: return launch_tau_z_mode<MVB_GEMM_F16_3, POL>(p, F, X, grid, smem, s);
+    default: return launch_tau_z_mode<MVB_Z_C64, POL>(p, F, X, grid, smem, s);
   }
-  return check_launch("tau_z_kernel");
 }
 
 // Fused phase + Z writer for nfreq frequencies: freqs_dev == nullptr means one

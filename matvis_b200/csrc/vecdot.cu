@@ -29,7 +29,7 @@
 namespace mvb {
 
 __device__ __forceinline__ int64_t vd_valid_k(const int32_t *n_dev, int64_t n_host, int kmul, int64_t Kcap) {
-  int64_t n = n_dev ? (int64_t)*n_dev : n_host;
+  int64_t n = n_dev ? (int64_t)__ldcg(n_dev) : n_host;
   n = n < 0 ? 0 : n;
   return min(n * kmul, Kcap);
 }
