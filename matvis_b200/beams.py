@@ -163,12 +163,12 @@ class B200BeamInterpolator(BeamInterpolator):
                 raise ValueError("all gridded beams must share one (nza, naz) grid shape")
             nza, naz = shapes.pop()
             if self.polarized:
-                grids = np.stack([b.data[: self.nax, : self.nfeed] for b in self.beam_list]).astype(np.complex64)
+                grids = np.stack([b.data[: self.nax, : self.nfeed] for b in self.beam_list]).astype(np.complex64, copy=False)
                 if grids.shape[1:3] != (self.nax, self.nfeed):
                     raise ValueError("polarized gridded beams need nax = nfeed = 2")
                 self.grid_kind = 0
             else:
-                grids = np.stack([b.power_grid() for b in self.beam_list]).astype(np.float32)
+                grids = np.stack([b.power_grid() for b in self.beam_list]).astype(np.float32, copy=False)
                 self.grid_kind = 1
             self.nza, self.naz = nza, naz
             params = np.array([[b.daz, b.dza, b.azmin] for b in self.beam_list], dtype=np.float64)

@@ -13,7 +13,7 @@ from concurrent.futures import ThreadPoolExecutor
 import numpy as np
 
 #: below this many sources one numpy pass beats handing the work to threads
-_PAR_MIN = 1 << 17
+_PAR_MIN = 1 << 15
 #: chunk granule (elements): a multiple of every SIMD width, so each chunk is
 #: split into vector body and tail exactly as the whole array would be
 _PAR_GRANULE = 8192

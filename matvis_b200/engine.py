@@ -123,6 +123,36 @@ def _pinned(src: np.ndarray) -> torch.Tensor:
     return t
 
 
+#: results up to this many bytes are copied to the host in one piece
+SMALL_RESULT = 1 << 20
+
+
+class _PageToucher:
+    """Touches the pages of a (Nf, Nt, ...) result array on host threads, a group of
+    frequencies of a time step at a time in the order a job completes them."""
+
+    def __init__(self, out: np.ndarray, group: int):
+        self._out = out
+        self._page = max(4096 // out.itemsize, 1)
+        nf, nt = out.shape[:2]
+        self._pool = ThreadPoolExecutor(min(os.cpu_count() or 1, 8))
+        self._done = {(t, f0): self._pool.submit(self._touch, t, f0, min(group, nf - f0))
+                      for t in range(nt) for f0 in range(0, nf, group)}
+
+    def _touch(self, t: int, f0: int, g: int):
+        for f in range(f0, f0 + g):
+            self._out[f, t].reshape(-1)[::self._page] = 0
+
+    def wait(self, t: int, f0: int, g: int):
+        """Returns once group f0 of time t is touched (nothing writes it afterwards)."""
+        fut = self._done.pop((t, f0), None)
+        if fut is not None:
+            fut.result()
+
+    def close(self):
+        self._pool.shutdown(wait=True, cancel_futures=True)
+
+
 def _repack_coherency(c: np.ndarray) -> tuple[np.ndarray, np.ndarray]:
     """(N, Nf, 2, 2) complex coherency -> (Nf, N, 4) float32 [C00, C11, Re C01,
     Im C01] and the (N, Nf) float64 trace max(C00 + C11, 0); source chunks on
@@ -574,28 +604,55 @@ class VisEngine:
 
         As soon as the kernels of a group of frequencies of a time step have
         run, a helper thread copies those visibilities into ``out`` on its own
-        stream, so the device -> host copy, and the first touch of freshly
-        allocated host pages (slower than the copy itself), overlap the compute
-        that follows; only the last group's copy runs after the compute.
+        stream, so the device -> host copy overlaps the compute that follows;
+        only the last group's copy runs after the compute.  The first touch of
+        freshly allocated host pages is slower than the copy itself (the kernel
+        clears them at about 10 GB/s a core): a few threads do it, from before the
+        job's buffers are made, in the order of the copies.  A result of at most
+        ``SMALL_RESULT`` bytes is copied in one piece after the run.
         """
-        if not self._uploaded:
-            self.upload()
-        shape = tuple(self.vis.shape)
         dtype = np.complex64 if self.ctype == torch.complex64 else np.complex128
-        if out is None:
-            out = np.empty(shape, dtype=dtype)
-        elif out.shape != shape or out.dtype != dtype or not out.flags.c_contiguous:
-            raise ValueError(f"out must be a C-contiguous {dtype.__name__} array of shape {shape}")
+
+        def destination(shape):
+            if out is None:
+                return np.empty(shape, dtype=dtype)
+            if out.shape != shape or out.dtype != dtype or not out.flags.c_contiguous:
+                raise ValueError(f"out must be a C-contiguous {dtype.__name__} array of shape {shape}")
+            return out
+
+        res = touch = None
+        try:
+            if not self._allocated and self.spec.antpairs is None:
+                res = destination((len(self.freqs), len(self.lsts), self.nant**2, self.nfeed, self.nfeed))
+                if res.nbytes > SMALL_RESULT:
+                    touch = _PageToucher(res, self.fgroup)
+            if not self._uploaded:
+                self.upload()
+            if res is None:
+                res = destination(tuple(self.vis.shape))
+                if res.nbytes > SMALL_RESULT:
+                    touch = _PageToucher(res, self.fgroup)
+            self.status.zero_()
+            if touch is None:
+                self.enqueue()
+                torch.from_numpy(res).copy_(self.vis)  # pageable destination: returns when done
+            else:
+                self._run_copying(res, touch)
+        finally:
+            if touch is not None:
+                touch.close()
+        _lib.check_status_word(self.status, "VisEngine")
+        return res
+
+    def _run_copying(self, out: np.ndarray, touch: "_PageToucher"):
+        """Enqueue the job a frequency group at a time, a helper thread copying each
+        group's visibilities once its kernels have run."""
         host = torch.from_numpy(out)
-        nf, nt = shape[:2]
         dev = self.vis.device
-        self.status.zero_()
         main = torch.cuda.current_stream(dev)
         side = torch.cuda.Stream(device=dev)
         steps: queue.Queue = queue.Queue()
         errors: list[BaseException] = []
-
-        page = 4096 // out.itemsize
 
         def copier():
             try:
@@ -603,10 +660,7 @@ class VisEngine:
                 with torch.cuda.stream(side):
                     while (item := steps.get()) is not None:
                         t, f0, g, done = item
-                        # touch the destination pages while the group still computes, so
-                        # that the copy after it is not held up by first-touch page faults
-                        for f in range(f0, f0 + g):
-                            out[f, t].reshape(-1)[::page] = 0
+                        touch.wait(t, f0, g)
                         side.wait_event(done)
                         for f in range(f0, f0 + g):
                             host[f, t].copy_(self.vis[f, t])
@@ -619,7 +673,7 @@ class VisEngine:
         worker = threading.Thread(target=copier, name="mvb-d2h", daemon=True)
         worker.start()
         try:
-            for t in range(nt):
+            for t in range(len(self.lsts)):
                 def after(f0, g, t=t):
                     done = torch.cuda.Event()
                     done.record(main)
@@ -632,8 +686,6 @@ class VisEngine:
         main.synchronize()
         if errors:
             raise errors[0]
-        _lib.check_status_word(self.status, "VisEngine")
-        return out
 
     def capture(self):
         """Capture the launch sequence as one CUDA graph (run once uncaptured first)."""

@@ -36,9 +36,10 @@ import torch
 
 from . import _lib
 from ._utils import get_desired_chunks
-from .beams import beams_at_frequency
+from .beams import beams_at_frequency, is_chromatic
 from .coordinates import latitude_of, lsts_of, point_source_crd_eq, radec_of
-from .engine import JobSpec, VisEngine, _norm_matprod, fit_freq_group, plan_job
+from .engine import (JobSpec, VisEngine, _norm_matprod, _resolve_product, fit_freq_group, freq_group_of,
+                     plan_job)
 
 
 logger = logging.getLogger(__name__)
@@ -76,6 +77,12 @@ def _check_coord_method(coord_method, params=None):
     if coord_method != "CoordinateRotationLST":
         raise ValueError(f"unknown coord_method {coord_method!r}")
     return {}
+
+
+def _plan(spec: JobSpec, budget: float) -> tuple[JobSpec, int, int]:
+    """(spec with its frequency group, frequencies per batch, source chunks) for ``budget`` bytes."""
+    spec = fit_freq_group(spec, budget)
+    return (spec, *plan_job(spec, budget))
 
 
 def simulate(
@@ -204,11 +211,15 @@ def simulate_vis(
     # one batched job (the reference re-interpolates per frequency, wrapper.py:180-199)
     spec = JobSpec(fluxes=fluxes, freqs=freqs, beams=list(beams), **common)
     dev = _lib.require_cuda(device)
-    # memory the caching allocator holds but does not use is free for this job too
-    free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-    budget = min(max_memory, free) * memory_buffer
-    spec = fit_freq_group(spec, budget)
-    nfb, nchunks = plan_job(spec, budget)
+    free = torch.cuda.mem_get_info(dev)[0]
+    want = spec
+    spec, nfb, nchunks = _plan(want, min(max_memory, free) * memory_buffer)
+    if freqs.size and (nfb < freqs.size or nchunks != want.nchunks or spec.freq_group < freq_group_of(
+            want, _resolve_product(want)[0], is_chromatic(want.beams))):
+        # memory the caching allocator holds but does not use is free for this job too
+        # (only looked up where the plan could change: it takes 0.2 ms)
+        free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+        spec, nfb, nchunks = _plan(want, min(max_memory, free) * memory_buffer)
     if nfb >= freqs.size and nchunks == spec.nchunks:
         vis = VisEngine(spec, device=dev).run_to_host()
         return vis if polarized else vis[..., 0, 0]
