@@ -257,6 +257,14 @@ int mvb_herk(const void *z, int mode, int64_t Mpad, int64_t Kcap, const int32_t 
 int mvb_herk_grouped(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t Kcap,
                      const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps, void *ws,
                      size_t ws_bytes, int32_t *status, void *stream);
+/* mvb_herk_grouped for panels whose first `rows` rows are live (Mpad - 128 < rows <=
+ * Mpad): the last block may be taken as its first 64 or 96 rows, where no more are
+ * live; the others are then not read, multiplied or stored, and the workspace holds
+ * nothing for them.  mvb_herk_reduce[_grouped] with nant * nfeed <= rows reads what is
+ * there; its visibilities are those of mvb_herk_grouped. */
+int mvb_herk_grouped_rows(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t rows,
+                          int64_t Kcap, const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk,
+                          int drain_ksteps, void *ws, size_t ws_bytes, int32_t *status, void *stream);
 /* One group of mvb_herk_batch: ngroup panels of one shape, z_stride bytes apart,
  * with the arguments mvb_herk_grouped takes for them. */
 typedef struct {

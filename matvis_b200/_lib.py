@@ -101,6 +101,8 @@ _SIGNATURES = {
     "mvb_set_wait_limit_ns": (ctypes.c_uint64, [ctypes.c_uint64]),
     "mvb_herk_grouped": (c_int, [_p, c_size_t, c_int, c_int, c_int64, c_int64, _p, c_int64, c_int, c_int, c_int, _p,
                                  c_size_t, _p, _p]),
+    "mvb_herk_grouped_rows": (c_int, [_p, c_size_t, c_int, c_int, c_int64, c_int64, c_int64, _p, c_int64, c_int, c_int,
+                                      c_int, _p, c_size_t, _p, _p]),
     "mvb_herk_batch": (c_int, [_p, c_int, c_int, c_int, _p]),
     "mvb_herk_reduce_grouped": (
         c_int,

@@ -69,15 +69,15 @@ __host__ __device__ inline int64_t round_up(int64_t a, int64_t b) { return ceil_
 
 int num_sms();
 // Sets a kernel's max dynamic shared memory once per (device, slot < 64);
-// slots 16..45 are the Hermitian-product variants,
+// slots 16..45 and 50..59 are the Hermitian-product variants,
 // 48 and 49 the staged pair kernels.
 int set_smem_once(const void *fn, int bytes, int slot);
-// mvb_herk_grouped with its work-unit counter left as it is (it must be 0), and
+// mvb_herk_grouped_rows with its work-unit counter left as it is (it must be 0), and
 // mvb_herk_reduce_grouped that also clears it for the next product of the same
 // workspace: a job's launch sequence, which clears it once (clear_unit_counter).
-int herk_grouped_chained(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t Kcap,
-                         const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps, void *ws,
-                         size_t ws_bytes, int32_t *status, void *stream);
+int herk_grouped_chained(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t rows,
+                         int64_t Kcap, const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps,
+                         void *ws, size_t ws_bytes, int32_t *status, void *stream);
 int herk_reduce_grouped_chained(void *ws, size_t ws_bytes, int ngroup, int64_t Mpad, int64_t Kcap,
                                 const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int nant, int nfeed,
                                 const int32_t *pairs, int64_t npairs, void *out, size_t out_stride, int out_c128,

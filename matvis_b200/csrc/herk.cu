@@ -22,6 +22,10 @@
 // forms from the partial tile's two triangles.  Three of the four real
 // 128 x 128 products on 6 of the 21 tiles of a 700-row panel: 7 % fewer
 // tensor-core cycles per slice.
+// Where the caller states the live rows and at most 96 (64) of the last block's 128
+// are, that block's tiles have 96 (64) columns: less to read, multiply and store, the
+// same sums in the same order (700 x 196,608, eight panels: job 10.96 -> 10.72 ms, of
+// which lower power is part; 90 rows of one block: 1,095 -> 1,088 us; 74: 287 -> 285).
 //
 // Accuracy.  The tensor core rounds its FP32 accumulator toward zero at every
 // UMMA, so a long in-TMEM sum drifts by about one ulp per instruction (3e-5
@@ -180,6 +184,32 @@ __device__ __forceinline__ void umma(uint32_t d, uint64_t a, uint64_t b, uint32_
     umma_bf16(d, a, b, idesc, acc);
 }
 
+// One k-step of one split product into the block at d: the two products of the Zi
+// rows first, so that the block's real and imaginary halves each start from Zi
+// terms, then the Zr rows'.  A full off-diagonal tile takes Zr against [Zr; Zi] as
+// one N = 256 instruction, a diagonal one only its real half (see the file's head).
+// NC < 128: a tile of the last block column, NC columns live; off the diagonal
+// Zr takes two instructions (the live rows of the two planes are not adjacent).  An
+// instruction of N columns takes max(N / 2, 32 + N / 4) cycles (the operands' 4 KB +
+// 32 N bytes at 128 bytes a cycle): 192 and 224 a k-step at 64 and 96 columns instead
+// of 256.
+template <int MODE, int NC>
+__device__ __forceinline__ void umma_kstep(uint32_t d, uint64_t a_re, uint64_t a_im, uint64_t b_re, uint64_t b_im,
+                                           uint32_t id_re, bool diag, uint32_t acc) {
+  using C = HerkCfg<MODE>;
+  if constexpr (NC == 128) {
+    umma<MODE>(d, a_im, b_im, C::ID128, acc);
+    umma<MODE>(d + 128, a_im, b_re, C::ID128N, acc);
+    umma<MODE>(d, a_re, b_re, id_re, 1u);
+  } else {
+    constexpr uint32_t id = umma_idesc(C::FMT, NC, 0), id_neg = umma_idesc(C::FMT, NC, 1);
+    umma<MODE>(d, a_im, b_im, id, acc);
+    umma<MODE>(d + 128, a_im, b_re, id_neg, acc);
+    umma<MODE>(d, a_re, b_re, id, 1u);
+    if (!diag) umma<MODE>(d + 128, a_re, b_im, id, 1u);
+  }
+}
+
 // A launch's work units come either from one panel shape repeated ngroup
 // times (the frequencies of a job's time step), or from a table of panels of
 // different shapes (the panel groups of several jobs, mvb_herk_batch).  A table
@@ -203,7 +233,8 @@ struct NoTable {};  // a launch of one repeated shape does not carry the table's
 
 // KD: k-steps accumulated in one TMEM block before it is drained (1, 2 or 4).
 // TABLE: the units come from the table (a batch) instead of one repeated shape.
-template <int MODE, int KD, bool TABLE>
+// TAIL > 0: the last block is narrow, its first TAIL rows.
+template <int MODE, int KD, bool TABLE, int TAIL>
 __global__ void __launch_bounds__(kHerkThreads, 1)
     herk_kernel(const uint8_t *__restrict__ zpanels, int64_t zstride, int ngroup, int T, int n_tiles,
                 const int32_t *__restrict__ n_dev, int64_t n_host, int kmul, int64_t Kcap, int k_chunk, int nsm,
@@ -291,8 +322,9 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
     return;
   }
 
-  // Where unit u is: its panel and block count, tile, columns and partial tile.
-  auto place = [&](int u, const uint8_t *&zpanel, float *&partial, int &Tu, int &I, int &J, int64_t &k0,
+  // Where unit u is: its panel and block count, tile, the tile's columns (TAIL in
+  // a narrow last block, else 128), its k range and its partial tile.
+  auto place = [&](int u, const uint8_t *&zpanel, float *&partial, int &Tu, int &I, int &J, int &nc, int64_t &k0,
                    int64_t &klen) {
     if constexpr (tabled) {
       int q = 0;
@@ -315,6 +347,7 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
       k0 = (int64_t)(r / n_tiles) * kc;
       klen = min(kc, kvalid - k0);
     }
+    nc = TAIL > 0 && J == Tu - 1 ? TAIL : 128;
   };
   // a bounded wait ran out: every status word of the launch learns it
   auto flag_timeout = [&]() {
@@ -346,12 +379,13 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
       if (u >= n_units) break;
       const uint8_t *zpanel;
       float *partial;
-      int Tu, I, J;
+      int Tu, I, J, nc;
       int64_t k0, klen;
-      place(u, zpanel, partial, Tu, I, J, k0, klen);
+      place(u, zpanel, partial, Tu, I, J, nc, k0, klen);
       const int nkb = (int)((klen + C::KB - 1) / C::KB);
       const bool diag = I == J;
-      const uint32_t bytes = diag ? C::OPER_BYTES : 2 * C::OPER_BYTES;
+      const uint32_t b_bytes = TAIL ? 2 * C::P * 64u * (uint32_t)nc : C::OPER_BYTES;  // block J's rows of every plane
+      const uint32_t bytes = diag ? b_bytes : C::OPER_BYTES + b_bytes;
       for (int kbi = 0; kbi < nkb; ++kbi) {
         if (!mbar_wait(&empty_bar[st], ph ^ 1, wait_ns)) {
           flag_timeout();
@@ -363,9 +397,20 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
         // k-block index: k0 is a multiple of 64 elements, a k-block 64 bytes;
         // operand (kb, R) starts at ((kb T + R) 2P) planes of 8 KB
         const int64_t kb = (k0 + (int64_t)kbi * C::KB) / C::KB;
-        bulk_load(a, zpanel + (kb * Tu + I) * (int64_t)C::OPER_BYTES, C::OPER_BYTES, &full_bar[st]);
-        if (!diag)
-          bulk_load(a + C::OPER_BYTES, zpanel + (kb * Tu + J) * (int64_t)C::OPER_BYTES, C::OPER_BYTES, &full_bar[st]);
+        if constexpr (TAIL > 0) {
+          if (!diag) bulk_load(a, zpanel + (kb * Tu + I) * (int64_t)C::OPER_BYTES, C::OPER_BYTES, &full_bar[st]);
+          uint8_t *b = diag ? a : a + C::OPER_BYTES;
+          const uint8_t *zb = zpanel + (kb * Tu + J) * (int64_t)C::OPER_BYTES;
+          if (nc == 128)
+            bulk_load(b, zb, C::OPER_BYTES, &full_bar[st]);
+          else
+            for (int pl = 0; pl < 2 * C::P; ++pl)
+              bulk_load(b + pl * kPlaneBytes, zb + pl * kPlaneBytes, 64u * (uint32_t)nc, &full_bar[st]);
+        } else {
+          bulk_load(a, zpanel + (kb * Tu + I) * (int64_t)C::OPER_BYTES, C::OPER_BYTES, &full_bar[st]);
+          if (!diag)
+            bulk_load(a + C::OPER_BYTES, zpanel + (kb * Tu + J) * (int64_t)C::OPER_BYTES, C::OPER_BYTES, &full_bar[st]);
+        }
         ++issued;
         if (++st == C::STAGES) {
           st = 0;
@@ -395,6 +440,7 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
     uint32_t st = 0, ph = 0, buf = 0, dph = 0, uk = 0;
     int nks = 0;
     bool diag = false, ok = true;
+    bool narrow_unit = false;  // the unit's tile has TAIL columns
     auto wait_all = [&](uint64_t *bar, uint32_t parity) {
       return __all_sync(0xffffffffu, mbar_wait(bar, parity, wait_ns)) != 0;
     };
@@ -412,67 +458,79 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
       if (u >= n_units) return false;
       const uint8_t *zpanel;
       float *partial;
-      int Tu, I, J;
+      int Tu, I, J, nc;
       int64_t k0, klen;
-      place(u, zpanel, partial, Tu, I, J, k0, klen);
+      place(u, zpanel, partial, Tu, I, J, nc, k0, klen);
       nks = __shfl_sync(0xffffffffu, (int)((klen + C::KSTEP - 1) / C::KSTEP), 0);
       diag = __shfl_sync(0xffffffffu, I == J ? 1 : 0, 0) != 0;
+      if constexpr (TAIL > 0) narrow_unit = __shfl_sync(0xffffffffu, nc, 0) < 128;
       return true;
     };
     bool have = next_unit();
     int ks = 0;
     if (have) ok = wait_all(&dempty_bar[0], 1u) && wait_all(&full_bar[0], 0u);
-    while (have && ok) {
-      tc_fence_after();
-      const int nk = min(2, nks - ks);
-      const uint32_t d = tbase + buf * 256;
-      const uint64_t a0 = umma_desc_sw64(smem_u32(smem) + st * C::STAGE_BYTES);
-      const uint64_t b0 = diag ? a0 : a0 + (C::OPER_BYTES >> 4);
-      const uint32_t id_re = diag ? C::ID128 : C::ID256;
-      const uint32_t st2 = st + 1 == C::STAGES ? 0 : st + 1, ph2 = st2 == 0 ? ph ^ 1u : ph;
-      const uint32_t dph2 = dph ^ (1u << buf);
+    // the blocks of consecutive units of one kind of tile
+    auto issue_blocks = [&](auto narrow) {
+      constexpr bool NARROW = decltype(narrow)::value;
+      constexpr int NC = NARROW ? TAIL : 128;
+      while (have && ok && (!TAIL || narrow_unit == NARROW)) {
+        tc_fence_after();
+        const int nk = min(2, nks - ks);
+        const uint32_t d = tbase + buf * 256;
+        const uint64_t a0 = umma_desc_sw64(smem_u32(smem) + st * C::STAGE_BYTES);
+        const uint64_t b0 = diag ? a0 : a0 + (C::OPER_BYTES >> 4);
+        const uint32_t id_re = diag ? C::ID128 : C::ID256;
+        const bool dg = NARROW && diag;  // (next_unit changes it)
+        const uint32_t st2 = st + 1 == C::STAGES ? 0 : st + 1, ph2 = st2 == 0 ? ph ^ 1u : ph;
+        const uint32_t dph2 = dph ^ (1u << buf);
 #pragma unroll
-      for (int q = 0; q < C::NPROD; ++q) {
-        uint32_t pa, pb;
-        product_terms(C::NPROD, q, pa, pb);
+        for (int q = 0; q < C::NPROD; ++q) {
+          uint32_t pa, pb;
+          product_terms(C::NPROD, q, pa, pb);
 #pragma unroll
-        for (int kk = 0; kk < 2; ++kk) {
-          // the next block, while the pipe still has the products before the last one
-          // queued; the two waits apart, each covered by the UMMAs around it
-          if (q == C::NPROD - 1 && kk == 0) {
-            ks += 2;
-            if (ks >= nks) {
-              have = next_unit();
-              ks = 0;
+          for (int kk = 0; kk < 2; ++kk) {
+            // the next block, while the pipe still has the products before the last one
+            // queued; the two waits apart, each covered by the UMMAs around it
+            if (NARROW ? (q == C::NPROD - 2 && kk == 1) : (q == C::NPROD - 1 && kk == 0)) {
+              ks += 2;
+              if (ks >= nks) {
+                have = next_unit();
+                ks = 0;
+              }
+              if (have) ok = wait_all(&full_bar[st2], ph2);
+            } else if (q == C::NPROD - 1 && kk == (NARROW ? 0 : 1) && have && ok) {
+              ok = wait_all(&dempty_bar[buf ^ 1u], ((dph2 >> (buf ^ 1u)) & 1u) ^ 1u);
             }
-            if (have) ok = wait_all(&full_bar[st2], ph2);
-          } else if (q == C::NPROD - 1 && have && ok) {
-            ok = wait_all(&dempty_bar[buf ^ 1u], ((dph2 >> (buf ^ 1u)) & 1u) ^ 1u);
+            if (lead && kk < nk) {
+              const uint64_t a_re = a0 + ((2 * pa * kPlaneBytes + kk * 32) >> 4);
+              const uint64_t a_im = a0 + (((2 * pa + 1) * kPlaneBytes + kk * 32) >> 4);
+              const uint64_t b_re = b0 + ((2 * pb * kPlaneBytes + kk * 32) >> 4);
+              const uint64_t b_im = b0 + (((2 * pb + 1) * kPlaneBytes + kk * 32) >> 4);
+              umma_kstep<MODE, NC>(d, a_re, a_im, b_re, b_im, id_re, dg, (q > 0 || kk > 0) ? 1u : 0u);
+            }
+            __syncwarp();
           }
-          if (lead && kk < nk) {
-            const uint64_t a_re = a0 + ((2 * pa * kPlaneBytes + kk * 32) >> 4);
-            const uint64_t a_im = a0 + (((2 * pa + 1) * kPlaneBytes + kk * 32) >> 4);
-            const uint64_t b_re = b0 + ((2 * pb * kPlaneBytes + kk * 32) >> 4);
-            const uint64_t b_im = b0 + (((2 * pb + 1) * kPlaneBytes + kk * 32) >> 4);
-            // the two N = 128 products first: the block's real and imaginary
-            // halves each start from Zi terms, then take the Zr terms
-            const uint32_t acc = (q > 0 || kk > 0) ? 1u : 0u;
-            umma<MODE>(d, a_im, b_im, C::ID128, acc);
-            umma<MODE>(d + 128, a_im, b_re, C::ID128N, acc);
-            umma<MODE>(d, a_re, b_re, id_re, 1u);
-          }
-          __syncwarp();
         }
+        if (lead) {
+          tc_commit(&empty_bar[st]);  // the stage is consumed
+          tc_commit(&dfull_bar[buf]);  // the block is complete
+        }
+        __syncwarp();
+        st = st2;
+        ph = ph2;
+        dph = dph2;
+        buf ^= 1u;
       }
-      if (lead) {
-        tc_commit(&empty_bar[st]);  // the stage is consumed
-        tc_commit(&dfull_bar[buf]);  // the block is complete
+    };
+    if constexpr (TAIL > 0) {
+      while (have && ok) {
+        if (narrow_unit)
+          issue_blocks(std::true_type{});
+        else
+          issue_blocks(std::false_type{});
       }
-      __syncwarp();
-      st = st2;
-      ph = ph2;
-      dph = dph2;
-      buf ^= 1u;
+    } else {
+      issue_blocks(std::false_type{});
     }
     if (!ok) {
       if (lane == 0) flag_timeout();
@@ -493,9 +551,9 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
       if (u >= n_units) break;
       const uint8_t *zpanel;
       float *partial;
-      int Tu, I, J;
+      int Tu, I, J, nc;
       int64_t k0, klen;
-      place(u, zpanel, partial, Tu, I, J, k0, klen);
+      place(u, zpanel, partial, Tu, I, J, nc, k0, klen);
       const int nks = (int)((klen + C::KSTEP - 1) / C::KSTEP);
       const bool diag = I == J;
       bool ok = true;
@@ -541,12 +599,8 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
               const uint64_t a_im = umma_desc_sw64(a_base + (2 * pa + 1) * kPlaneBytes);
               const uint64_t b_re = umma_desc_sw64(b_base + (2 * pb) * kPlaneBytes);
               const uint64_t b_im = umma_desc_sw64(b_base + (2 * pb + 1) * kPlaneBytes);
-              // the two N = 128 products first: the block's real and imaginary
-              // halves each start from Zi terms, then take the Zr terms
-              const uint32_t acc = (q > 0 || kk > 0) ? 1u : 0u;
-              umma<MODE>(d, a_im, b_im, C::ID128, acc);
-              umma<MODE>(d + 128, a_im, b_re, C::ID128N, acc);
-              umma<MODE>(d, a_re, b_re, diag ? C::ID128 : C::ID256, 1u);
+              umma_kstep<MODE, 128>(d, a_re, a_im, b_re, b_im, diag ? C::ID128 : C::ID256, diag,
+                                       (q > 0 || kk > 0) ? 1u : 0u);
             }
           }
 #pragma unroll
@@ -586,10 +640,8 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
           const uint64_t a_im = umma_desc_sw64(a_base + (2 * pa + 1) * kPlaneBytes);
           const uint64_t b_re = umma_desc_sw64(b_base + (2 * pb) * kPlaneBytes);
           const uint64_t b_im = umma_desc_sw64(b_base + (2 * pb + 1) * kPlaneBytes);
-          const uint32_t acc = (ks % KD != 0 || q > 0) ? 1u : 0u;
-          umma<MODE>(d, a_im, b_im, C::ID128, acc);
-          umma<MODE>(d + 128, a_im, b_re, C::ID128N, acc);
-          umma<MODE>(d, a_re, b_re, diag ? C::ID128 : C::ID256, 1u);
+          umma_kstep<MODE, 128>(d, a_re, a_im, b_re, b_im, diag ? C::ID128 : C::ID256, diag,
+                                   (ks % KD != 0 || q > 0) ? 1u : 0u);
         }
         if ((ks & 1) == 1 || ks == nks - 1) {  // the stage is consumed
           tc_commit(&empty_bar[st]);
@@ -634,10 +686,14 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
       if (u >= n_units) break;
       const uint8_t *zpanel;
       float *partial;
-      int Tu, I, J;
+      int Tu, I, J, nc;
       int64_t k0, klen;
-      place(u, zpanel, partial, Tu, I, J, k0, klen);
+      place(u, zpanel, partial, Tu, I, J, nc, k0, klen);
       const int nks = (int)((klen + C::KSTEP - 1) / C::KSTEP);
+      // live columns of this warp's quarter; none of a quadrant of padding rows (which
+      // only the last diagonal tile has: its rows are its columns)
+      const int mine = !TAIL ? 64 : I == J && quad * 32 >= nc ? 0 : max(0, nc - (quarter & 1) * 64);
+      const bool live = !TAIL || I != J || row < nc;
       bool ok = true;
       for (int g0 = 0; g0 < nks; g0 += KD) {
         // every lane waits; the vote keeps the warp converged for tcgen05.ld
@@ -648,6 +704,7 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
         constexpr int W = KD == 2 ? 8 : 16;  // columns per load: 16 spill beside the KD = 2 issuer
 #pragma unroll
         for (int c = 0; c < 64 / W; ++c) {
+          if (TAIL && c * W >= mine) break;
           uint32_t v[W];
           tmem_ld<W>(taddr + c * W, v);
           tmem_ld_wait();
@@ -668,7 +725,7 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
       float *dst = partial + (size_t)quarter * 64 * 128;
 #pragma unroll
       for (int j = 0; j < 64; ++j) {
-        dst[j * 128 + row] = acc[j];
+        if (live && j < mine) dst[j * 128 + row] = acc[j];
         acc[j] = 0.f;
       }
     }
@@ -936,9 +993,9 @@ uint64_t wait_limit_ns() { return g_wait_limit_ns.load(std::memory_order_relaxed
 
 // table.n > 0: the units come from the table (z, ngroup, shape and status arguments unused).
 template <int MODE, int KD>
-static int launch_herk(const void *z, int64_t zstride, int ngroup, int64_t Mpad, int64_t Kcap, const int32_t *n_dev,
-                       int64_t n_host, int kmul, int k_chunk, float *partials, int32_t *status, int *unit_next,
-                       bool clear_counter, cudaStream_t s, const HerkTable &table) {
+static int launch_herk(const void *z, int64_t zstride, int ngroup, int64_t Mpad, int rows, int64_t Kcap,
+                       const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, float *partials, int32_t *status,
+                       int *unit_next, bool clear_counter, cudaStream_t s, const HerkTable &table) {
   using C = HerkCfg<MODE>;
   const int T = (int)(Mpad / 128);
   const int n_tiles = T * (T + 1) / 2;
@@ -953,10 +1010,22 @@ static int launch_herk(const void *z, int64_t zstride, int ngroup, int64_t Mpad,
   }
   const int grid = (int)std::min<int64_t>(max_units, nsm);
   const size_t smem = (size_t)C::STAGES * C::STAGE_BYTES + 1024;
-  // slots 16 + 3 * MODE + {0, 1, 2} for KD = {1, 2, 4}, 15 more for the table forms
-  const int slot = 16 + 3 * MODE + (KD == 4 ? 2 : KD - 1) + (table.n > 0 ? 15 : 0);
-  const void *fn = table.n > 0 ? reinterpret_cast<const void *>(herk_kernel<MODE, KD, true>)
-                               : reinterpret_cast<const void *>(herk_kernel<MODE, KD, false>);
+  // The last block of one repeated shape as its live rows rounded up to 64 or 96, under
+  // the default drain.  The forms' waits and drains are the more expensive ones for full
+  // tiles, so a shape without a narrow block keeps the plain form (384 rows: 1.5 % more
+  // cycles in the narrow one).
+  constexpr int kTail64 = KD == 2 ? 64 : 0, kTail96 = KD == 2 ? 96 : 0;
+  const int last = (int)(rows - (Mpad - 128));
+  const int tail = KD != 2 || table.n > 0 || last > 96 ? 0 : last > 64 ? 96 : 64;
+  // slots 16 + 3 * MODE + {0, 1, 2} for KD = {1, 2, 4}, 15 more for the table forms; 50 + MODE and 55 + MODE for
+  // the narrow ones
+  const int slot = tail == 96   ? 55 + MODE
+                   : tail == 64 ? 50 + MODE
+                                : 16 + 3 * MODE + (KD == 4 ? 2 : KD - 1) + (table.n > 0 ? 15 : 0);
+  const void *fn = table.n > 0  ? reinterpret_cast<const void *>(herk_kernel<MODE, KD, true, 0>)
+                   : tail == 96 ? reinterpret_cast<const void *>(herk_kernel<MODE, KD, false, kTail96>)
+                   : tail == 64 ? reinterpret_cast<const void *>(herk_kernel<MODE, KD, false, kTail64>)
+                                : reinterpret_cast<const void *>(herk_kernel<MODE, KD, false, 0>);
   int rc = set_smem_once(fn, (int)smem, slot);
   if (rc) return rc;
   if (grid <= 0) return MVB_OK;
@@ -965,13 +1034,15 @@ static int launch_herk(const void *z, int64_t zstride, int ngroup, int64_t Mpad,
     cudaError_t e = cudaMemsetAsync(unit_next, 0, sizeof(int), s);
     if (e != cudaSuccess) return fail(MVB_ERR_CUDA, "herk unit counter: %s", cudaGetErrorString(e));
   }
-  if (table.n > 0)
-    return launch_chained("herk_kernel", herk_kernel<MODE, KD, true>, grid, kHerkThreads, smem, s,
-                          static_cast<const uint8_t *>(z), zstride, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap,
-                          k_chunk, nsm, partials, status, unit_next, wait_ns, table);
-  return launch_chained("herk_kernel", herk_kernel<MODE, KD, false>, grid, kHerkThreads, smem, s,
-                        static_cast<const uint8_t *>(z), zstride, ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap,
-                        k_chunk, nsm, partials, status, unit_next, wait_ns, NoTable{});
+  auto launch = [&](auto kernel, auto units) {
+    return launch_chained("herk_kernel", kernel, grid, kHerkThreads, smem, s, static_cast<const uint8_t *>(z), zstride,
+                          ngroup, T, n_tiles, n_dev, n_host, kmul, Kcap, k_chunk, nsm, partials, status, unit_next,
+                          wait_ns, units);
+  };
+  if (table.n > 0) return launch(herk_kernel<MODE, KD, true, 0>, table);
+  if (tail == 96) return launch(herk_kernel<MODE, KD, false, kTail96>, NoTable{});
+  if (tail == 64) return launch(herk_kernel<MODE, KD, false, kTail64>, NoTable{});
+  return launch(herk_kernel<MODE, KD, false, 0>, NoTable{});
 }
 
 // Argument checks shared by the product and its reductions (the slice plan
@@ -1013,8 +1084,10 @@ static int *unit_counter(void *ws, size_t ws_bytes) {
 static int herk_impl(const char *who, const void *z, int64_t zstride, int ngroup, int mode, int64_t Mpad, int64_t Kcap,
                      const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps, void *ws,
                      size_t ws_bytes, int32_t *status, void *stream, const HerkTable &table = HerkTable{},
-                     bool clear_counter = true) {
+                     bool clear_counter = true, int64_t live_rows = 0) {
+  const int rows = (int)(live_rows ? live_rows : Mpad);
   if (table.n == 0) {
+    if (rows > Mpad || rows <= Mpad - 128) return fail(MVB_ERR_ARG, "%s: rows do not end in the last block", who);
     int rc = check_herk_group(who, z, zstride, ngroup, mode, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, ws, ws_bytes,
                               status);
     if (rc) return rc;
@@ -1027,11 +1100,11 @@ static int herk_impl(const char *who, const void *z, int64_t zstride, int ngroup
   float *part = static_cast<float *>(ws);
   int *next = unit_counter(ws, ws_bytes);
 #define MVB_HERK(M)                                                                                          \
-  return kd == 1   ? launch_herk<M, 1>(z, zstride, ngroup, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
+  return kd == 1   ? launch_herk<M, 1>(z, zstride, ngroup, Mpad, rows, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
                                        next, clear_counter, s, table)                                                       \
-         : kd == 2 ? launch_herk<M, 2>(z, zstride, ngroup, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
+         : kd == 2 ? launch_herk<M, 2>(z, zstride, ngroup, Mpad, rows, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
                                        next, clear_counter, s, table)                                                       \
-                   : launch_herk<M, 4>(z, zstride, ngroup, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
+                   : launch_herk<M, 4>(z, zstride, ngroup, Mpad, rows, Kcap, n_dev, n_host, kmul, k_chunk, part, status, \
                                        next, clear_counter, s, table)
   switch (mode) {
     case MVB_GEMM_BF16_3: MVB_HERK(MVB_GEMM_BF16_3);
@@ -1085,11 +1158,11 @@ static int reduce_impl(const char *who, const void *ws, size_t ws_bytes, int ngr
   }
 }
 
-int herk_grouped_chained(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t Kcap,
-                         const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps, void *ws,
-                         size_t ws_bytes, int32_t *status, void *stream) {
+int herk_grouped_chained(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t rows,
+                         int64_t Kcap, const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk, int drain_ksteps,
+                         void *ws, size_t ws_bytes, int32_t *status, void *stream) {
   return herk_impl("mvb_herk_grouped", z, (int64_t)z_stride, ngroup, mode, Mpad, Kcap, n_dev, n_host, kmul, k_chunk,
-                   drain_ksteps, ws, ws_bytes, status, stream, HerkTable{}, false);
+                   drain_ksteps, ws, ws_bytes, status, stream, HerkTable{}, false, rows);
 }
 
 int herk_reduce_grouped_chained(void *ws, size_t ws_bytes, int ngroup, int64_t Mpad, int64_t Kcap,
@@ -1134,6 +1207,15 @@ extern "C" int mvb_herk_grouped(const void *z, size_t z_stride, int ngroup, int 
   if (z_stride > (size_t)INT64_MAX) return fail(MVB_ERR_ARG, "mvb_herk_grouped: bad arguments");
   return herk_impl("mvb_herk_grouped", z, (int64_t)z_stride, ngroup, mode, Mpad, Kcap, n_dev, n_host, kmul, k_chunk,
                    drain_ksteps, ws, ws_bytes, status, stream);
+}
+
+extern "C" int mvb_herk_grouped_rows(const void *z, size_t z_stride, int ngroup, int mode, int64_t Mpad, int64_t rows,
+                                     int64_t Kcap, const int32_t *n_dev, int64_t n_host, int kmul, int k_chunk,
+                                     int drain_ksteps, void *ws, size_t ws_bytes, int32_t *status, void *stream) {
+  const char *who = "mvb_herk_grouped_rows";
+  if (z_stride > (size_t)INT64_MAX || rows <= 0) return fail(MVB_ERR_ARG, "%s: bad arguments", who);
+  return herk_impl(who, z, (int64_t)z_stride, ngroup, mode, Mpad, Kcap, n_dev, n_host, kmul, k_chunk, drain_ksteps, ws,
+                   ws_bytes, status, stream, HerkTable{}, true, rows);
 }
 
 extern "C" int mvb_herk_batch(const mvb_herk_group *groups, int ngroups, int mode, int drain_ksteps, void *stream) {

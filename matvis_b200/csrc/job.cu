@@ -73,8 +73,8 @@ static int job_group(const mvb_job &j, int t, int f0, int g, int accumulate, voi
     return mvb_vecdot(j.z, j.Kcap, j.n_above, j.cap, F, F, j.pairs, j.npairs, j.k_chunk, j.ws, j.ws_bytes, out,
                       j.out_c128, accumulate, stream);
   }
-  if ((rc = herk_grouped_chained(j.z, j.z_stride, g, j.mode, j.Mpad, j.Kcap, j.n_above, j.cap, F, j.k_chunk,
-                             j.drain_ksteps, j.ws, j.ws_bytes, j.status, stream)))
+  if ((rc = herk_grouped_chained(j.z, j.z_stride, g, j.mode, j.Mpad, (int64_t)j.nant * F, j.Kcap, j.n_above, j.cap, F,
+                             j.k_chunk, j.drain_ksteps, j.ws, j.ws_bytes, j.status, stream)))
     return rc;
   return herk_reduce_grouped_chained(j.ws, j.ws_bytes, g, j.Mpad, j.Kcap, j.n_above, j.cap, F, j.k_chunk, j.nant, F,
                                  j.pairs, j.npairs, out, (size_t)j.vis_f_stride, j.out_c128,

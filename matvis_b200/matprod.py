@@ -206,6 +206,11 @@ class B200MatMul(MatProd):
             self._ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         return self._ws
 
+    def _live_rows(self, panel: ZPanel) -> int:
+        """The panel's rows that the reduction reads (all of it if they end before its last block)."""
+        m = self.nant * self.nfeed
+        return m if panel.Mpad - _lib.TILE < m <= panel.Mpad else panel.Mpad
+
     def enqueue_grouped(self, panels: list[ZPanel], out: torch.Tensor, accumulate: bool = False, stream=None,
                         k_chunk=None):
         """Products of consecutive panels of one allocation (``ZPanel.group``) in
@@ -222,9 +227,9 @@ class B200MatMul(MatProd):
         ws = self.workspace(p0, kc, ng)
         sh = stream_handle(stream)
         check(
-            _lib.lib.mvb_herk_grouped(
-                ptr(p0.data), stride, ng, self.mode, p0.Mpad, p0.Kcap, ptr(p0.n_dev), p0.n_host, p0.nax, kc,
-                self.drain_ksteps, ptr(ws), ws.numel(), ptr(self.status), sh,
+            _lib.lib.mvb_herk_grouped_rows(
+                ptr(p0.data), stride, ng, self.mode, p0.Mpad, self._live_rows(p0), p0.Kcap, ptr(p0.n_dev), p0.n_host,
+                p0.nax, kc, self.drain_ksteps, ptr(ws), ws.numel(), ptr(self.status), sh,
             )
         )
         self.reduce_grouped(panels, out, accumulate=accumulate, stream=stream, k_chunk=kc)
@@ -274,9 +279,9 @@ class B200MatMul(MatProd):
         sh = stream_handle(stream)
         kmul = panel.nax
         check(
-            _lib.lib.mvb_herk(
-                ptr(panel.data), self.mode, panel.Mpad, panel.Kcap, ptr(panel.n_dev), panel.n_host, kmul, kc,
-                self.drain_ksteps, ptr(ws), ws.numel(), ptr(self.status), sh,
+            _lib.lib.mvb_herk_grouped_rows(
+                ptr(panel.data), 0, 1, self.mode, panel.Mpad, self._live_rows(panel), panel.Kcap, ptr(panel.n_dev),
+                panel.n_host, kmul, kc, self.drain_ksteps, ptr(ws), ws.numel(), ptr(self.status), sh,
             )
         )
         pairs = None if self.all_pairs else self._pairs_dev
