@@ -159,6 +159,17 @@ __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *m
       : "memory");
 }
 
+// One or two columns (H = 2 or 4 floats) of a row in shared memory.
+template <int H>
+__device__ __forceinline__ void vd_load(uint32_t addr, float (&v)[H]) {
+  if constexpr (H == 4)
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                 : "r"(addr));
+  else
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "r"(addr));
+}
+
 // Units are (k-slice, bundle group); groups fastest so the CTAs of one slice
 // read its columns from L2 together, and rotating with the slice so that a
 // CTA's units cycle through the groups.  Compute thread t of a unit runs bundle
@@ -248,8 +259,19 @@ __global__ void __launch_bounds__(kVdCtaThreads, 1)
   // Row r of a stage starts at r rowbytes in a 1024-aligned buffer, so the
   // swizzled offset of its 16-byte unit holding columns (c, c + 1) is
   // (r rowbytes + m_r) ^ (8 c), m_r < rowbytes the row's swizzle mask: each row
-  // read is kept as that one offset.
-  int64_t g = 0;  // stages consumed
+  // read is kept as that one address in the current stage's buffer.
+  // What bounds it: instruction issue.  A bundle's two columns cost 96 FMAs and 8
+  // 16-byte loads (F = 2; 41 of 52 cycles a warp measured, against 32 of shared-memory
+  // bandwidth), so the rest is kept small: whole 16-column stages unrolled with constant
+  // column offsets (one XOR a load), the stage and its phase counted instead of divided
+  // out, the addresses moved on once a stage.  350 antennas x 2 feeds, 5,000 pairs,
+  // K = 1,000,000: 5,710 -> 5,195 us; K = 40,000: 272 -> 228; F = 1, K = 100,000:
+  // 271 -> 206; 64 antennas, F = 1, 1,000 pairs, K = 40,000: 67 -> 52.  Did not help:
+  // paired FP32 FMAs (half the FMAs to issue, the same time), each antenna's loads
+  // issued before the sums of the one before, a panel stored stage by stage
+  // (64 bundles, where the copies bound it, 1,290 -> 800 us; 1,792 bundles the same).
+  const uint32_t buf0 = smem_u32(stage0), buf_end = buf0 + (uint32_t)(nstage * stage_bytes);
+  uint32_t buf = buf0, b = 0, ph = 0;  // the next stage's buffer and its full barrier's phase
   for (int64_t u = blockIdx.x; u < nunits; u += gridDim.x) {
     const int64_t slice = u / ngroups;
     const int s0 = (int)((u % ngroups + slice) % ngroups) * group_size;
@@ -273,7 +295,7 @@ __global__ void __launch_bounds__(kVdCtaThreads, 1)
 #pragma unroll
         for (int x = 0; x < F; ++x) {
           const uint32_t off = (uint32_t)((F * a + (x ^ ba)) * rowbytes);
-          r[x] = off + ((((off >> 7) & swz)) << 4);  // row offset with its swizzle mask
+          r[x] = buf + off + ((((off >> 7) & swz)) << 4);  // row address with its swizzle mask
         }
       };
       rows(lo.x, ri);
@@ -289,49 +311,30 @@ __global__ void __launch_bounds__(kVdCtaThreads, 1)
       for (int e = 0; e < E; ++e) acc2[q][e] = acc1[q][e] = 0.f;
 
     const int nst = (int)((k1 - k0 + kb - 1) / kb);
-    const int per16 = 16 / kb;  // stages per 16-column block
+    int left = (int)(k1 - k0), in16 = 0;  // columns of the unit, and of the 16-column block so far
     bool stop = false;
-    for (int st = 0; st < nst; ++st, ++g) {
-      const int b = (int)(g % nstage);
-      if (abort_flag || !mbar_wait(&full_bar[b], (uint32_t)((g / nstage) & 1), wait_ns)) {
+    for (int st = 0; st < nst; ++st) {
+      if (abort_flag || !mbar_wait(&full_bar[b], ph, wait_ns)) {
         if (lane == 0 && status && !abort_flag) atomicOr(status, MVB_DEV_TIMEOUT);
         abort_flag = 1;
         stop = true;
         break;
       }
-      const uint8_t *buf = stage0 + (size_t)b * stage_bytes;
       // columns of this stage inside [k0, k1): all but the kvalid tail
-      const int ncols = (int)min((int64_t)kb, k1 - (k0 + (int64_t)st * kb));
+      const int ncols = min(kb, left);
+      left -= kb;
       // acc[y][x] += Zj[y] conj(Zi[x]): y, x the feeds in load order;
       // H = 4 (columns c, c + 1) or 2 (the odd last column)
       auto step = [&](uint32_t c8, auto hw) {
         constexpr int H = decltype(hw)::value;
         float vi[F][H];
 #pragma unroll
-        for (int x = 0; x < F; ++x) {
-          const uint8_t *ad = buf + (ri[x] ^ c8);
-          if constexpr (H == 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(ad);
-            vi[x][0] = v.x, vi[x][1] = v.y, vi[x][2] = v.z, vi[x][3] = v.w;
-          } else {
-            const float2 v = *reinterpret_cast<const float2 *>(ad);
-            vi[x][0] = v.x, vi[x][1] = v.y;
-          }
-        }
+        for (int x = 0; x < F; ++x) vd_load<H>(ri[x] ^ c8, vi[x]);
 #pragma unroll
         for (int q = 0; q < S; ++q) {
           float vj[F][H];
 #pragma unroll
-          for (int y = 0; y < F; ++y) {
-            const uint8_t *ad = buf + (rj[q][y] ^ c8);
-            if constexpr (H == 4) {
-              const float4 v = *reinterpret_cast<const float4 *>(ad);
-              vj[y][0] = v.x, vj[y][1] = v.y, vj[y][2] = v.z, vj[y][3] = v.w;
-            } else {
-              const float2 v = *reinterpret_cast<const float2 *>(ad);
-              vj[y][0] = v.x, vj[y][1] = v.y;
-            }
-          }
+          for (int y = 0; y < F; ++y) vd_load<H>(rj[q][y] ^ c8, vj[y]);
 #pragma unroll
           for (int y = 0; y < F; ++y)
 #pragma unroll
@@ -346,10 +349,17 @@ __global__ void __launch_bounds__(kVdCtaThreads, 1)
         }
       };
       if (live) {
+        if (ncols == 16) {
+#pragma unroll
+          for (uint32_t c8 = 0; c8 < 128; c8 += 16) step(c8, std::integral_constant<int, 4>{});
+        } else {
 #pragma unroll 1
-        for (int c = 0; c + 1 < ncols; c += 2) step((uint32_t)(c * 8), std::integral_constant<int, 4>{});
+          for (int c = 0; c + 1 < ncols; c += 2) step((uint32_t)(c * 8), std::integral_constant<int, 4>{});
+        }
         if (ncols & 1) step((uint32_t)((ncols - 1) * 8), std::integral_constant<int, 2>{});
-        if ((st + 1) % per16 == 0 || st + 1 == nst) {
+        in16 += kb;
+        if (in16 == 16 || left <= 0) {
+          in16 = 0;
 #pragma unroll
           for (int q = 0; q < S; ++q)
 #pragma unroll
@@ -361,6 +371,20 @@ __global__ void __launch_bounds__(kVdCtaThreads, 1)
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty_bar[b]);  // this warp is done with the stage
+      uint32_t next = buf + (uint32_t)stage_bytes;
+      ++b;
+      if (next == buf_end) {
+        next = buf0;
+        b = 0;
+        ph ^= 1u;
+      }
+#pragma unroll
+      for (int x = 0; x < F; ++x) {
+        ri[x] += next - buf;
+#pragma unroll
+        for (int q = 0; q < S; ++q) rj[q][x] += next - buf;
+      }
+      buf = next;
     }
     if (stop) break;
     if (live) {
