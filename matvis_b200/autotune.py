@@ -36,7 +36,7 @@ KD_CANDIDATES = (1, 2, 4)
 #: (196,608 sources, 350 antennas, complex128 output, k_chunk 4096) per split
 #: mode and drain interval; product time per slice in the comment (one B200)
 MEASURED_ERROR = {
-    _lib.GEMM_F16_3: {1: 2.00e-7, 2: 3.04e-7, 4: 5.62e-7},   # 1.32 / 1.16 / 1.29 ms
+    _lib.GEMM_F16_3: {1: 2.00e-7, 2: 3.04e-7, 4: 5.62e-7},   # 1.67 / 1.11 / 1.34 ms
     _lib.GEMM_TF32_3: {1: 1.75e-7, 2: 2.42e-7, 4: 3.83e-7},  # 2.61 / 2.14 / 2.56 ms
     _lib.GEMM_BF16_6: {1: 1.23e-7, 2: 1.66e-7, 4: 3.39e-7},  # 2.06 / 1.92 / 2.26 ms
     _lib.GEMM_BF16_3: {1: 3.5e-6, 2: 3.5e-6, 4: 3.5e-6},     # the 2-term bf16 split itself misses the bar

@@ -5,12 +5,15 @@ inside it, rotation -> horizon selection -> beam -> tau -> Z -> product per time
 and chunk with a device synchronisation after each stage (cpu/cpu.py:247-272,
 gpu/gpu.py:197-254).  Here one job is one stream of launches:
 
-    for t:      mvb_rotate -> (per chunk) mvb_horizon_compact -> mvb_beam_*
+    for t:      rotation and horizon selection -> (per chunk) beam
       for each group of G frequencies:
-                mvb_tau_z_grouped -> mvb_herk_grouped -> mvb_herk_reduce_grouped
+                tau/Z -> Hermitian product -> reduction
                 (G panels, one launch each; a beamfits beam, which changes with
-                frequency, or a pair list on mvb_vecdot goes one frequency at a time:
-                [mvb_beam_*] -> mvb_tau_z -> mvb_herk + mvb_herk_reduce or mvb_vecdot)
+                frequency, or a pair list on per-pair sums goes one frequency at a time:
+                [beam] -> tau/Z -> product + reduction or pair sums)
+
+enqueued by one native call for a range of times and groups (mvb_job_enqueue),
+each kernel launched while the one before it drains.
 
 Rotation, selection and (for an achromatic beam) beam interpolation depend on
 time only and are done once per time for all frequencies.  The above-horizon count never leaves the device:
@@ -46,8 +49,8 @@ from .autotune import KD_CANDIDATES, tune_product
 from .matprod import B200MatMul, B200VectorDot, choose_k_chunk, pair_product
 
 #: k-slice of the Hermitian product without autotuning: the tuner's choice for
-#: the HERA-350-like slice in fp16x3 (product + reduction 1.36 ms at 4096
-#: columns; shorter slices mean more partial tiles to reduce).  The number of
+#: the HERA-350-like slice in fp16x3 (product + reduction 1.12 ms at 4096
+#: columns, 1.19 at 2048; shorter slices mean more partial tiles to reduce).  The number of
 #: slices is still fitted to whole waves of SMs on the device.
 DEFAULT_K_CHUNK = 4096
 
