@@ -416,8 +416,10 @@ class VisEngine:
         mp, p0, bm = self.matprod, self.panels[0], self.bmfunc
         herk = self.method == "MatMul"
         ws = mp.workspace(p0, self.k_chunk, self.fgroup) if herk else mp.workspace(p0)
+        # dense: the native code indexes them (a caller's frequencies may be a strided view)
         rot = np.ascontiguousarray(self.rot, dtype=np.float64)
-        keep = [rot, ws, self.freqs]
+        freqs = np.ascontiguousarray(self.freqs, dtype=np.float64)
+        keep = [rot, ws, freqs]
 
         def at(x):
             return None if x is None else x.data_ptr()
@@ -432,7 +434,7 @@ class VisEngine:
             antpos=at(self.antpos), topo=at(self.topo), rot=rot.ctypes.data, crd=at(self.crd), kept=at(self.kept),
             n_above=at(self.n_above), status=at(self.status), select_ws=at(self.ws_compact),
             select_ws_bytes=self.ws_compact.numel(), nbeam=bm.nbeam, chromatic=int(self.chromatic),
-            beam=at(bm.interpolated_beam), beam_idx=at(bm.beam_index_dev), freqs=self.freqs.ctypes.data,
+            beam=at(bm.interpolated_beam), beam_idx=at(bm.beam_index_dev), freqs=freqs.ctypes.data,
             freqs_dev=at(self.freqs_dev), mode=self.zcalc.mode, zscale=self.zscale, z=at(p0.data),
             z_stride=p0.nbytes, Mpad=p0.Mpad, Kcap=p0.Kcap, k_chunk=self.k_chunk if herk else mp.k_chunk,
             ws=at(ws), ws_bytes=ws.numel(), npairs=self.npairs, vis=at(self.vis),
