@@ -161,7 +161,12 @@ int mvb_exptau(const double *antpos, int A, double freq, const double *crd, int6
  *   ((k / KB) * (Mpad / 128) + m / 128) * 2P * 128 * KB + pl * 128 * KB
  *   + (m % 128) * KB + ((c / E) ^ ((m % 128 / 2) % 4)) * E + c % E,
  * c = k % KB, E = KB / 4 elements per chunk.
- * Mpad is a multiple of 128, Kcap of 64.  Bytes: 2P x Mpad x Kcap x element size. */
+ * Mpad is a multiple of 128, Kcap of 64.  Bytes: 2P x Mpad x Kcap x element size.
+ * A 32-byte aligned panel takes the widest stores.  The phase / Z writers accept 8
+ * bytes at 16 bits and 16 at 32 and for a plain Z (with narrower stores); mvb_z_pack
+ * less (4 for bf16, 2 fp16, 8 tf32, 16 plain); mvb_z_from_exptau 8 bytes x X at 16
+ * bits, 16 x X for tf32, 32 for a plain Z.  Less than that is MVB_ERR_ARG; the
+ * Hermitian product needs 16. */
 size_t mvb_zpanel_bytes(int mode, int64_t Mpad, int64_t Kcap);
 /* sflux[f * N + s] = (float) sqrt(0.5 * flux[s * nf + f]) (cpu/cpu.py:188): the
  * per-frequency sqrt(0.5 I) rows the Z writers read, from the caller's

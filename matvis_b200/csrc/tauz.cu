@@ -282,10 +282,12 @@ __device__ __forceinline__ float4 coherency_factor(float4 c, double2 r) {
 // L[x, y, s], so that Z Z^H gives exptau_j conj(exptau_i) E_j C' E_i^H per source.
 // grid.x: blocks of 64 columns, grid.y: blocks of kTauZAnts antennas, grid.z: per_z
 // frequencies each, frequency g: fluxes sflux + g sflux_ld (coh + g coh_ld), panel
-// z + g zstride bytes.
-template <int MODE, int X, int F, bool POL, bool GROUP>
+// z + g zstride bytes.  WIDE: every panel is aligned to the stores of eight columns
+// (store_align); otherwise eight columns go out in two halves, the same bytes.
+template <int MODE, int X, int F, bool POL, bool GROUP, bool WIDE>
 __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GROUP)) tau_z_kernel(const __grid_constant__ TauZArgs p) {
   static_assert(!POL || (X == 2 && F == 2), "the polarised sky needs two feeds and two beam axes");
+  static_assert(!GROUP || WIDE, "narrow stores: one frequency per CTA");
   constexpr int NS = kTauZCols / X;        // sources per thread
   constexpr int BS = kTauZGroups * NS;     // sources per CTA
   pdl_wait();
@@ -444,15 +446,18 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
         }
         const int64_t m = (int64_t)a * F + f;
         if constexpr (MODE == MVB_Z_C64) {
-          // the row's 8 values start 64-byte aligned (Kcap a multiple of 64): whole
-          // 32-byte sectors, four values each
+          // the row's 8 values start a multiple of 64 bytes into the panel (Kcap a
+          // multiple of 64): whole 32-byte sectors, four values each
           float2 *zp = reinterpret_cast<float2 *>(zg) + m * p.Kcap + k0;
 #pragma unroll
           for (int i = 0; i < kTauZCols; i += 4) {
             const uint32_t w[8] = {__float_as_uint(vr[i]),     __float_as_uint(vi[i]),     __float_as_uint(vr[i + 1]),
                                    __float_as_uint(vi[i + 1]), __float_as_uint(vr[i + 2]), __float_as_uint(vi[i + 2]),
                                    __float_as_uint(vr[i + 3]), __float_as_uint(vi[i + 3])};
-            store_sector(zp + i, w);
+            if constexpr (WIDE)
+              store_sector(zp + i, w);
+            else
+              store_words<8>(zp + i, w);
           }
         } else {
           // 8 consecutive k from a multiple of 8: inside one k-block
@@ -460,8 +465,17 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
           constexpr int NPL = MODE == MVB_GEMM_BF16_6 ? 6 : 4;
           const int64_t off = panel_off(m, k0, p.Mpad, KB, NPL);
           const int64_t off2 = panel_off(m, k0 + kTauZCols / 2, p.Mpad, KB, NPL);
-          put_split<MODE, kTauZCols>(zg, panel_plane_stride(KB), off, off2, 0, vr, 1.f);
-          put_split<MODE, kTauZCols>(zg, panel_plane_stride(KB), off, off2, 1, vi, 1.f);
+          if constexpr (WIDE) {
+            put_split<MODE, kTauZCols>(zg, panel_plane_stride(KB), off, off2, 0, vr, 1.f);
+            put_split<MODE, kTauZCols>(zg, panel_plane_stride(KB), off, off2, 1, vi, 1.f);
+          } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int64_t o = h ? off2 : off;
+              put_split<MODE, kTauZCols / 2>(zg, panel_plane_stride(KB), o, o, 0, vr + h * (kTauZCols / 2), 1.f);
+              put_split<MODE, kTauZCols / 2>(zg, panel_plane_stride(KB), o, o, 1, vi + h * (kTauZCols / 2), 1.f);
+            }
+          }
         }
       }
     }
@@ -794,38 +808,53 @@ extern "C" int mvb_exptau(const double *antpos, int A, double freq, const double
   return check_launch("exptau_kernel");
 }
 
-template <int MODE, bool POL, bool GROUP>
+template <int MODE, bool POL, bool GROUP, bool WIDE>
 static int launch_tau_z_form(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
+  auto launch = [&](auto kernel) { return launch_chained("tau_z_kernel", kernel, grid, kTauZThreads, smem, s, p); };
   if constexpr (POL) {
-    return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 2, 2, true, GROUP>, grid, kTauZThreads, smem, s, p);
+    return launch(tau_z_kernel<MODE, 2, 2, true, GROUP, WIDE>);
   } else if (X == 2) {
-    if (F == 2)
-      return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 2, 2, false, GROUP>, grid, kTauZThreads, smem, s, p);
-    else
-      return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 2, 1, false, GROUP>, grid, kTauZThreads, smem, s, p);
+    return F == 2 ? launch(tau_z_kernel<MODE, 2, 2, false, GROUP, WIDE>)
+                  : launch(tau_z_kernel<MODE, 2, 1, false, GROUP, WIDE>);
   } else {
-    if (F == 2)
-      return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 1, 2, false, GROUP>, grid, kTauZThreads, smem, s, p);
-    else
-      return launch_chained("tau_z_kernel", tau_z_kernel<MODE, 1, 1, false, GROUP>, grid, kTauZThreads, smem, s, p);
+    return F == 2 ? launch(tau_z_kernel<MODE, 1, 2, false, GROUP, WIDE>)
+                  : launch(tau_z_kernel<MODE, 1, 1, false, GROUP, WIDE>);
   }
 }
 
 template <int MODE, bool POL>
-static int launch_tau_z_mode(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
-  if (p.per_z > 1)
-    return launch_tau_z_form<MODE, POL, true>(p, F, X, grid, smem, s);
-  return launch_tau_z_form<MODE, POL, false>(p, F, X, grid, smem, s);
+static int launch_tau_z_mode(const TauZArgs &p, bool wide, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
+  if (!wide) return launch_tau_z_form<MODE, POL, false, false>(p, F, X, grid, smem, s);
+  if (p.per_z > 1) return launch_tau_z_form<MODE, POL, true, true>(p, F, X, grid, smem, s);
+  return launch_tau_z_form<MODE, POL, false, true>(p, F, X, grid, smem, s);
+}
+
+// Alignment of a panel that the stores of `cols` consecutive columns of a mode need:
+// 8 columns are 16 bytes at 16 bits and whole sectors at 32 and in a complex64 Z; 4
+// are 8 bytes, 16, and a sector again (which the fused writer halves).
+static int store_align(int mode, int cols) {
+  if (mode == MVB_Z_C64) return 32;
+  return cols * (mode == MVB_GEMM_TF32_3 ? 4 : 2);
+}
+
+static int check_align(const char *who, const void *z, int bytes) {
+  if (reinterpret_cast<uintptr_t>(z) % bytes) return fail(MVB_ERR_ARG, "%s: panel not %d-byte aligned", who, bytes);
+  return MVB_OK;
 }
 
 // The launch of both fused writers (arguments checked by the callers).
 template <bool POL>
-static int launch_tau_z(TauZArgs p, const double *antpos, int A, double freq, const double *freqs_dev, int nfreq,
+static int launch_tau_z(const char *who, TauZArgs p, const double *antpos, int A, double freq, const double *freqs_dev, int nfreq,
                         const double *crd, int64_t ld, const int32_t *n_dev, int64_t nsrc, const int32_t *sidx,
                         const void *beam, int64_t beam_ld, int nbeam, const int32_t *beam_idx, int F, int X, int mode,
                         float zscale, void *z, int64_t z_stride, int64_t Mpad, int64_t Kcap, void *stream) {
   const int64_t cols = round_up(nsrc * X, kKAlign);
   if (cols == 0) return MVB_OK;
+  // The package's own panels are aligned to the wide stores; a C caller's may lie on
+  // (or be spaced by) less, and then go out a frequency per CTA in half-wide stores.
+  const int align = store_align(mode, kTauZCols);
+  const bool wide = reinterpret_cast<uintptr_t>(z) % align == 0 && (nfreq == 1 || z_stride % align == 0);
+  if (int rc = wide ? MVB_OK : check_align(who, z, mode == MVB_Z_C64 ? 16 : store_align(mode, kTauZCols / 2))) return rc;
   p.antpos = antpos;
   p.crd = crd;
   p.freqs = freqs_dev;
@@ -866,7 +895,7 @@ static int launch_tau_z(TauZArgs p, const double *antpos, int A, double freq, co
   const int64_t units = xblocks * ceil_div(A, kTauZAntLanes) * nfreq;
   const int64_t share = std::max<int64_t>(1, units / ((int64_t)num_sms() * kTauZCtasPerSm));
   const int64_t parts = ceil_div(nfreq, std::min<int64_t>({share, (int64_t)kTauZMaxFreq, (int64_t)nfreq}));
-  p.per_z = (int)ceil_div(nfreq, parts);
+  p.per_z = wide ? (int)ceil_div(nfreq, parts) : 1;
   const int64_t lanes = std::min<int64_t>(std::max<int64_t>(share / p.per_z, 1), kTauZAnts / kTauZAntLanes);
   const int64_t ablocks = ceil_div(A, lanes * kTauZAntLanes);
   p.ants = (int)round_up(ceil_div(A, ablocks), kTauZAntLanes);  // even shares, whole lanes
@@ -877,11 +906,11 @@ static int launch_tau_z(TauZArgs p, const double *antpos, int A, double freq, co
                       (p.staged ? (size_t)nbeam * F * kTauZBeamRow * sizeof(float2) : 0);
   cudaStream_t s = as_stream(stream);
   switch (mode) {
-    case MVB_GEMM_BF16_3: return launch_tau_z_mode<MVB_GEMM_BF16_3, POL>(p, F, X, grid, smem, s);
-    case MVB_GEMM_BF16_6: return launch_tau_z_mode<MVB_GEMM_BF16_6, POL>(p, F, X, grid, smem, s);
-    case MVB_GEMM_TF32_3: return launch_tau_z_mode<MVB_GEMM_TF32_3, POL>(p, F, X, grid, smem, s);
-    case MVB_GEMM_F16_3: return launch_tau_z_mode<MVB_GEMM_F16_3, POL>(p, F, X, grid, smem, s);
-    default: return launch_tau_z_mode<MVB_Z_C64, POL>(p, F, X, grid, smem, s);
+    case MVB_GEMM_BF16_3: return launch_tau_z_mode<MVB_GEMM_BF16_3, POL>(p, wide, F, X, grid, smem, s);
+    case MVB_GEMM_BF16_6: return launch_tau_z_mode<MVB_GEMM_BF16_6, POL>(p, wide, F, X, grid, smem, s);
+    case MVB_GEMM_TF32_3: return launch_tau_z_mode<MVB_GEMM_TF32_3, POL>(p, wide, F, X, grid, smem, s);
+    case MVB_GEMM_F16_3: return launch_tau_z_mode<MVB_GEMM_F16_3, POL>(p, wide, F, X, grid, smem, s);
+    default: return launch_tau_z_mode<MVB_Z_C64, POL>(p, wide, F, X, grid, smem, s);
   }
 }
 
@@ -904,7 +933,7 @@ static int tau_z_impl(const char *who, const double *antpos, int A, double freq,
   TauZArgs p{};
   p.sflux = sflux;
   p.sflux_ld = sflux_ld;
-  return launch_tau_z<false>(p, antpos, A, freq, freqs_dev, nfreq, crd, ld, n_dev, nsrc, sidx, beam, beam_ld, nbeam,
+  return launch_tau_z<false>(who, p, antpos, A, freq, freqs_dev, nfreq, crd, ld, n_dev, nsrc, sidx, beam, beam_ld, nbeam,
                              beam_idx, F, X, mode, zscale, z, z_stride, Mpad, Kcap, stream);
 }
 
@@ -931,6 +960,9 @@ static int z_pack_impl(const char *who, const void *zsrc, int z_c128, int64_t M,
                        cudaStream_t s) {
   const int64_t cols = round_up(K, kKAlign);
   if (M == 0 || cols == 0) return MVB_OK;
+  // the narrowest stores: 16 bytes of a complex64 Z, pairs of float32 or bf16, single fp16
+  int rc = check_align(who, z, mode == MVB_Z_C64 ? 16 : mode == MVB_GEMM_TF32_3 ? 8 : mode == MVB_GEMM_F16_3 ? 2 : 4);
+  if (rc) return rc;
   const int64_t xblocks = ceil_div(cols, kPackGroups * (z_c128 ? kPackCols<double2> : kPackCols<float2>));
   // four rows a lane (a 64-row block) where that still leaves eight CTAs per SM
   constexpr int lanes = kPackThreads / kPackGroups;
@@ -1009,7 +1041,7 @@ static int tau_z_pol_impl(const char *who, const double *antpos, int A, double f
   p.coh = reinterpret_cast<const float4 *>(coh);
   p.coh_ld = coh_ld;
   p.rot = reinterpret_cast<const double2 *>(rot);
-  return launch_tau_z<true>(p, antpos, A, freq, freqs_dev, nfreq, crd, ld, n_dev, nsrc, sidx, beam, beam_ld, nbeam,
+  return launch_tau_z<true>(who, p, antpos, A, freq, freqs_dev, nfreq, crd, ld, n_dev, nsrc, sidx, beam, beam_ld, nbeam,
                             beam_idx, F, X, mode, zscale, z, z_stride, Mpad, Kcap, stream);
 }
 
@@ -1044,6 +1076,8 @@ extern "C" int mvb_z_from_exptau(const void *exptau, int e_c128, int64_t e_ld, i
   if (round_up(nsrc * X, kKAlign) > Kcap) return fail(MVB_ERR_ARG, "mvb_z_from_exptau: Kcap too small");
   const int64_t s_max = round_up(nsrc * X, kKAlign) / X;
   if (s_max == 0) return MVB_OK;
+  rc = check_align("mvb_z_from_exptau", z, store_align(mode, kZExtSrc * X));
+  if (rc) return rc;
   dim3 grid((unsigned)ceil_div(s_max, kZExtBlockSrc), (unsigned)ceil_div(A, kTauZAnts));
   const bool staged = nbeam * F * X <= kTauZMaxBFX;
   const size_t smem = staged ? (size_t)nbeam * F * X * kZExtRow * sizeof(float2) : 0;
