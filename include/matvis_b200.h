@@ -465,7 +465,10 @@ typedef struct {
  * multiple of freq_group): for each time and chunk, if f0 = 0, the rotation (chunk
  * 0), selection, beam and frame rotation, then the frequency groups' tau/Z, product
  * and reduction -- the entry points above in the order of the reference's loops
- * (wrapper.py:180-199, cpu/cpu.py:247-272).  Nothing is kept from the call. */
+ * (wrapper.py:180-199, cpu/cpu.py:247-272).  No host array is kept from the call.
+ * With f0 > 0 the call continues the one time and chunk of the call before it, from
+ * the selection and beam in the job's buffers; with c0 > 0 the one time, from its
+ * rotation: such ranges over more than one time (or, f0 > 0, chunk) are MVB_ERR_ARG. */
 int mvb_job_enqueue(const mvb_job *job, int t0, int t1, int c0, int c1, int f0, int f1, void *stream);
 
 /* ---- Redundant-baseline pair selection (host memory, no device work) ------- */

@@ -91,6 +91,11 @@ extern "C" int mvb_job_enqueue(const mvb_job *job, int t0, int t1, int c0, int c
       (t0 < t1 && f0 < f1 && (!j.freqs || !j.freqs_dev || !j.vis)) || (j.chromatic && (j.freq_group != 1 || j.sigmas)) ||
       (j.mode == MVB_Z_C64 && (j.freq_group != 1 || (!j.plan && !j.pairs && j.npairs))))
     return fail(MVB_ERR_ARG, "%s: bad arguments", who);
+  // Frequencies after the first group continue one (time, chunk), chunks after the first
+  // one time: more than one would take the sky or the rotation the last call left.
+  const int nt = std::max(t1 - t0, 0), nc = std::max(c1 - c0, 0);
+  if ((f0 > 0 && f0 < f1 && (int64_t)nt * nc > 1) || (c0 > 0 && nt > 1 && nc > 0))
+    return fail(MVB_ERR_ARG, "%s: a later frequency or chunk of more than one time or chunk", who);
   int rc;
   // the products' work-unit counter: cleared here, then by each reduction
   if (t0 < t1 && c0 < c1 && f0 < f1 && j.mode != MVB_Z_C64 && (rc = clear_unit_counter(j.ws, j.ws_bytes, stream))) return rc;
