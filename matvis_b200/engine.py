@@ -482,6 +482,7 @@ class VisEngine:
         frequencies f0 .. f0 + g - 1 of this time are enqueued (for a results
         copy that can start as soon as they have run).  ``launches``: the
         ``_launches()`` of this job, if the caller already has them."""
+        t = range(len(self.lsts))[t]  # an array's index: from the end if negative
         job, _keep = launches or self._launches()
         sh = _lib.stream_handle(stream)
         nf, last = len(self.freqs), self.nchunks - 1
