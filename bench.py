@@ -610,7 +610,7 @@ def run_b200(args, rank, world, local_rank):
             "autotune": eng.tuned,
         },
         "roofline": roofline,
-        "gpu_launches": eng.launches_per_run() * args.steps,
+        "gpu_launches": eng.launched * args.steps,
         "clocks": clocks,
     }
 

@@ -62,6 +62,9 @@ extern "C" {
 int mvb_version(void);
 /* Message for the last non-OK status returned on the calling host thread. */
 const char *mvb_last_error(void);
+/* Kernels launched so far through this library by the calling host thread (a graph's
+ * replays are not seen: take the difference over its capture). */
+int64_t mvb_launches(void);
 /* Number of SMs and compute capability of the current device. */
 int mvb_device_info(int *sm_count, int *cc_major, int *cc_minor);
 

@@ -44,6 +44,7 @@ _p = c_void_p
 _SIGNATURES = {
     "mvb_version": (c_int, []),
     "mvb_last_error": (ctypes.c_char_p, []),
+    "mvb_launches": (c_int64, []),
     "mvb_device_info": (c_int, [_p, _p, _p]),
     "mvb_rotate": (c_int, [_p, c_int64, _p, _p, _p]),
     "mvb_bcrs": (c_int, [_p, c_int64, _p, _p, _p]),

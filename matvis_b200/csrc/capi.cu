@@ -10,6 +10,11 @@ std::string &last_error() {
   return msg;
 }
 
+int64_t &launch_count() {
+  static thread_local int64_t n = 0;
+  return n;
+}
+
 // SM count of the current device, cached per device ordinal.
 int num_sms() {
   static int cache[64] = {0};
@@ -28,6 +33,8 @@ int num_sms() {
 extern "C" int mvb_version(void) { return 1; }
 
 extern "C" const char *mvb_last_error(void) { return mvb::last_error().c_str(); }
+
+extern "C" int64_t mvb_launches(void) { return mvb::launch_count(); }
 
 extern "C" int mvb_device_info(int *sm_count, int *cc_major, int *cc_minor) {
   int dev = 0;

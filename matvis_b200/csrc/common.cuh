@@ -18,6 +18,7 @@ namespace mvb {
 // host-side status
 // ---------------------------------------------------------------------------
 std::string &last_error();
+int64_t &launch_count();  // kernels launched by this host thread
 
 inline int fail(int code, const char *fmt, ...) {
   char buf[512];
@@ -29,9 +30,11 @@ inline int fail(int code, const char *fmt, ...) {
   return code;
 }
 
+// Called once after each <<< >>> launch.
 inline int check_launch(const char *what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MVB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  ++launch_count();
   return MVB_OK;
 }
 
@@ -61,6 +64,7 @@ inline int launch_chained(const char *what, void (*kernel)(KArgs...), dim3 grid,
     cudaGetLastError();
     return fail(MVB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   }
+  ++launch_count();
   return MVB_OK;
 }
 

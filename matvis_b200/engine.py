@@ -281,6 +281,8 @@ class VisEngine:
             zmax = smax * bmax * (2.0 if self.pol_sky else 1.0)
             self.zscale = _lib.f16_scale(zmax * (1 + 2**-10))
         self._graph = None
+        #: kernels of the latest ``enqueue`` (of the captured graph, after capture())
+        self.launched = 0
         self._allocated = False
         self._uploaded = False
         #: the autotuner's decision for this job (set by capture())
@@ -470,10 +472,13 @@ class VisEngine:
         return j, keep
 
     def enqueue(self, stream=None):
-        """Enqueue every kernel of the job on ``stream`` (no host synchronisation)."""
+        """Enqueue every kernel of the job on ``stream`` (no host synchronisation);
+        ``launched`` then holds how many there were."""
         job, _keep = self._launches()
+        before = _lib.lib.mvb_launches()
         _lib.check(_lib.lib.mvb_job_enqueue(ctypes.byref(job), 0, len(self.lsts), 0, self.nchunks, 0, len(self.freqs),
                                             _lib.stream_handle(stream)))
+        self.launched = _lib.lib.mvb_launches() - before
 
     def enqueue_time(self, t: int, stream=None, after=None, launches=None):
         """Enqueue the kernels of time index t (all chunks and frequencies).
@@ -580,6 +585,9 @@ class VisEngine:
         return n + (ws.numel() if ws is not None else 0)
 
     def launches_per_run(self) -> int:
+        """At most this many kernel launches a run: what it is split into by hand
+        (rotation and horizon count apart, a gridded beam laid out and gathered).  The
+        number made is less where one kernel does two of these; ``launched`` has it."""
         # per frequency (or per group of fgroup frequencies): tau/Z, then the product
         # and its reduction (mvb_herk[_grouped] + reduce, or vecdot_kernel + its slice reduction)
         per_f = 3

@@ -266,10 +266,6 @@ class VisServer:
                 eng = job.engine
                 ngroups = len(eng.lsts) * eng.nchunks * -(-len(eng.freqs) // max(eng.fgroup, 1))
                 job.group_terms = estimate_terms(job.spec) / max(ngroups, 1)
-                self.launches += eng.launches_per_run()
-                if self.batch_products and eng.batchable:
-                    # its product launches are shared ones, counted as they are made
-                    self.launches -= len(eng.lsts) * eng.nchunks * -(-len(eng.freqs) // max(eng.fgroup, 1))
                 self._active.append(job)
         self.max_concurrent = max(self.max_concurrent, len(self._active))
 
@@ -397,7 +393,6 @@ class VisServer:
                 done.record(bs)
                 self._turn.append(done)
                 self.batch_launches += 1
-                self.launches += 1
                 self.batched_groups += len(take)
                 for job, g, _ in take:
                     if self._reduce_and_step(job, g, done):
@@ -465,7 +460,9 @@ class VisServer:
     def poll(self):
         """One scheduling turn: admit, advance every active job by a time step, retire."""
         self._admit()
+        before = _lib.lib.mvb_launches()
         self._advance()
+        self.launches += _lib.lib.mvb_launches() - before
         self._retire()
 
     def run_until_idle(self, timeout_s: float = 3600.0):
