@@ -18,8 +18,8 @@ on the job's own Z panel; frequencies per grouped launch sized to memory.
 
 ``tune_product`` times every candidate pair (a few launches each, CUDA events
 on a side stream) -- the product together with its reduction when the caller
-passes ``run`` -- and caches the winner per (mode, Mpad, K bucket, device) for
-the life of the process; ``cached_choice`` hands it to later jobs of the same
+passes ``run`` -- and caches the winner per (mode, Mpad, width of the last row
+block, K bucket, device) for the life of the process; ``cached_choice`` hands it to later jobs of the same
 shape that are not captured (``simulate_vis``).  ``last_choice`` reports the
 latest decision.
 """
@@ -55,6 +55,13 @@ def _bucket(k: int) -> int:
     return b
 
 
+def _tail(rows: int | None, Mpad: int) -> int:
+    """Columns of the product's last row block for a panel of ``rows`` live rows: 64 or
+    96 where no more are live, 0 for a full block (the product has a form for each)."""
+    last = 0 if rows is None else rows - (Mpad - _lib.TILE)
+    return 0 if last <= 0 or last > 96 else 64 if last <= 64 else 96
+
+
 def drain_candidates(mode: int, kd_candidates=KD_CANDIDATES) -> list[int]:
     """Drain intervals whose measured error fits ERROR_BUDGET (0 = the mode's
     default, always allowed); the lowest-error one if none does."""
@@ -75,7 +82,8 @@ def tune_product(panel, mode: int, status: torch.Tensor, run=None, reps: int = 3
     kvalid = panel.n_host * panel.nax if panel.n_dev is None else int(panel.n_dev.item()) * panel.nax
     kcs = [c for c in kc_candidates if c <= max(kvalid, kc_candidates[0])] or [kc_candidates[0]]
     kds = drain_candidates(mode, kd_candidates)
-    key = (mode, panel.Mpad, _bucket(max(kvalid, 1)), torch.cuda.current_device(), tuple(kcs), tuple(kds))
+    tail = _tail(panel.M, panel.Mpad)
+    key = (mode, panel.Mpad, tail, _bucket(max(kvalid, 1)), torch.cuda.current_device(), tuple(kcs), tuple(kds))
     if key in _cache:
         return _cache[key]
     ws = None
@@ -96,9 +104,10 @@ def tune_product(panel, mode: int, status: torch.Tensor, run=None, reps: int = 3
                     if run is not None:
                         run(c, kd, s)
                         continue
-                    _lib.check(_lib.lib.mvb_herk(_lib.ptr(panel.data), mode, panel.Mpad, panel.Kcap,
-                                                 _lib.ptr(panel.n_dev), panel.n_host, panel.nax, c, kd, _lib.ptr(ws),
-                                                 ws.numel(), _lib.ptr(status), _lib.stream_handle(s)))
+                    _lib.check(_lib.lib.mvb_herk_grouped_rows(
+                        _lib.ptr(panel.data), 0, 1, mode, panel.Mpad, panel.M if tail else panel.Mpad, panel.Kcap,
+                        _lib.ptr(panel.n_dev), panel.n_host, panel.nax, c, kd, _lib.ptr(ws), ws.numel(),
+                        _lib.ptr(status), _lib.stream_handle(s)))
                 e1.record(s)
                 e1.synchronize()
                 ms = e0.elapsed_time(e1) / reps
@@ -112,12 +121,13 @@ def tune_product(panel, mode: int, status: torch.Tensor, run=None, reps: int = 3
     return best
 
 
-def cached_choice(mode: int, Mpad: int, kvalid: int, device: int) -> tuple[int, int] | None:
+def cached_choice(mode: int, Mpad: int, kvalid: int, device: int, rows: int | None = None) -> tuple[int, int] | None:
     """A (k_chunk, drain_ksteps) already tuned in this process for this shape
-    (mode, Mpad, K bucket, device), or None."""
-    b = _bucket(max(int(kvalid), 1))
+    (mode, Mpad, width of the last block, K bucket, device), or None; ``rows``: the
+    panel's live rows (None: all Mpad)."""
+    want = (mode, Mpad, _tail(rows, Mpad), _bucket(max(int(kvalid), 1)), device)
     for key, choice in _cache.items():
-        if key[:4] == (mode, Mpad, b, device):
+        if key[:5] == want:
             return choice
     return None
 

@@ -357,7 +357,7 @@ class VisEngine:
                 # a choice the autotuner made earlier in this process for this shape
                 # (about half the sky above the horizon)
                 hit = autotune.cached_choice(self.matprod.mode, panel.Mpad, self.nsrc // 2 * self.nax,
-                                             torch.device(dev).index or 0)
+                                             torch.device(dev).index or 0, rows=panel.M)
                 if hit is not None:
                     self.k_chunk, self.matprod.drain_ksteps = hit
                     self.tuned = {"k_chunk": hit[0], "drain_ksteps": hit[1], "cached": True}
