@@ -209,9 +209,10 @@ struct PanelWriter {
 
 // ---------------------------------------------------------------------------
 // Fused writer.  CTA = 128 threads over 64 panel columns (32 sources at X = 2, 64
-// at X = 1) x 64 antennas x `per_z` frequencies: thread bits 0..2 pick a group of
-// 8 consecutive columns (16-byte stores per plane at 16 bits), bits 3..6 one of 16
-// antenna lanes, each lane taking every 16th antenna of the block.  A CTA writes 2
+// at X = 1) x 64 antennas x `per_z` frequencies: thread bits 0..2 pick a group of 8
+// consecutive columns (16-byte stores per plane at 16 bits), bits 3..6 one of 16
+// antenna lanes, each lane taking every 16th antenna of the block (one frequency at
+// X = 1: 32 columns, groups of 4).  A CTA writes 2
 // or 4 k-blocks of 128 rows per frequency, so the Z lines it has open at any time
 // fit, summed over the resident CTAs, well inside L2 (a wider k-range per CTA left
 // partially written lines to be evicted); a warp's store writes 16 whole 32-byte
@@ -230,19 +231,32 @@ struct PanelWriter {
 // lane factored the coherency again).  The results are bit-identical.
 // ---------------------------------------------------------------------------
 constexpr int kTauZThreads = 128;
-constexpr int kTauZCols = 8;                // consecutive columns per thread
+constexpr int kTauZCols = 8;                // consecutive columns per thread (tau_z_cols: 4 in one form)
 constexpr int kTauZGroups = 8;              // column groups per CTA
 constexpr int kTauZAntLanes = kTauZThreads / kTauZGroups;
 constexpr int kTauZAnts = 64;               // antennas per CTA
 constexpr int kTauZMaxBFX = 16;             // beam planes staged in shared memory, else read through L1
 constexpr int kTauZMaxFreq = 8;             // frequencies per CTA
 constexpr int kTauZCtasPerSm = 8;           // CTAs per SM that a small launch is cut into
-constexpr int kTauZBeamRow = kTauZCols * kTauZGroups;  // staged values of one (beam, feed)
+
+// Columns per thread.  One frequency at one beam axis takes four: eight sources'
+// paths and fluxes do not stay in registers, and nothing else of them is shared.
+// 512 antennas x 60,000 sources, fp16x3: 82 us with four, 121 with eight (20 beams,
+// read through L1: 91 and 176); 100 x 60,000 as a complex64 Z: 17 and 28.
+__host__ __device__ constexpr int tau_z_cols(int X, bool group) { return X == 1 && !group ? 4 : kTauZCols; }
+
+// Whether frequencies share a CTA.  A two-feed, two-axis tf32x3 panel is 16 bytes a
+// value and bound by its stores: fewer and longer CTAs only cost their last wave.  350
+// antennas x 6,000 slots x 12, half live: 122 us one frequency per CTA, 141 shared;
+// x 40,000 x 3: 221 and 220; polarised sky, x 15,000 x 8: 233 and 270.
+__host__ __device__ constexpr bool tau_z_groups(int mode, int F, int X) {
+  return !(mode == MVB_GEMM_TF32_3 && F * X == 4);
+}
 
 // Resident CTAs per SM that the registers are held to (the best of 4, 5, 6, 8 and
 // no bound, by form: the polarised group form keeps 32 beam values a thread).
-constexpr int tau_z_min_blocks(int mode, int X, int F, bool group) {
-  return X * F == 4 ? (!group ? 6 : (mode == MVB_GEMM_TF32_3 ? 5 : 4)) : (X == 1 && F == 2 ? 5 : 6);
+constexpr int tau_z_min_blocks(int X, int F, bool group) {
+  return X * F == 4 ? (group ? 4 : 6) : (X == 1 && F == 2 ? 5 : 6);
 }
 
 struct TauZArgs {
@@ -280,15 +294,17 @@ __device__ __forceinline__ float4 coherency_factor(float4 c, double2 r) {
 // (coh[sidx[s]] at this frequency) and frame rotation R (rot[s] = cos X, sin X);
 // with C' = R^T C R = L L^H, Z[a, f, (s, y)] = exptau(a, s) sum_x beam[f, x, s]
 // L[x, y, s], so that Z Z^H gives exptau_j conj(exptau_i) E_j C' E_i^H per source.
-// grid.x: blocks of 64 columns, grid.y: blocks of kTauZAnts antennas, grid.z: per_z
+// grid.x: blocks of ROW columns, grid.y: blocks of kTauZAnts antennas, grid.z: per_z
 // frequencies each, frequency g: fluxes sflux + g sflux_ld (coh + g coh_ld), panel
 // z + g zstride bytes.  WIDE: every panel is aligned to the stores of eight columns
 // (store_align); otherwise eight columns go out in two halves, the same bytes.
 template <int MODE, int X, int F, bool POL, bool GROUP, bool WIDE>
-__global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GROUP)) tau_z_kernel(const __grid_constant__ TauZArgs p) {
+__global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(X, F, GROUP)) tau_z_kernel(const __grid_constant__ TauZArgs p) {
   static_assert(!POL || (X == 2 && F == 2), "the polarised sky needs two feeds and two beam axes");
   static_assert(!GROUP || WIDE, "narrow stores: one frequency per CTA");
-  constexpr int NS = kTauZCols / X;        // sources per thread
+  constexpr int COLS = tau_z_cols(X, GROUP);
+  constexpr int ROW = COLS * kTauZGroups;  // columns of the CTA: staged values of one (beam, feed)
+  constexpr int NS = COLS / X;             // sources per thread
   constexpr int BS = kTauZGroups * NS;     // sources per CTA
   pdl_wait();
   pdl_trigger();
@@ -348,7 +364,7 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
     const int q = lane0 + i * PER;
     if (q < nq) {
       const int k = (sl % NS) * X + q % X;  // the thread's column
-      beam_sm[(q / X) * kTauZBeamRow + ((k >> 1) * kTauZGroups + sl / NS) * 2 + (k & 1)] =
+      beam_sm[(q / X) * ROW + ((k >> 1) * kTauZGroups + sl / NS) * 2 + (k & 1)] =
           make_float2(b_in[i].x * p.scale_beam, b_in[i].y * p.scale_beam);
     }
   }
@@ -378,19 +394,19 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
     for (int j = 0; j < NS; ++j)
       path[j] = KEEP ? dx * cx[KEEP ? j : 0] + dy * cy[KEEP ? j : 0] + dz * cz[KEEP ? j : 0]
                      : dx * crd_sm[0][sg * NS + j] + dy * crd_sm[1][sg * NS + j] + dz * crd_sm[2][sg * NS + j];
-    float2 bv[GROUP ? F : 1][kTauZCols];
-    auto load_beam = [&](int f, float2(&v)[kTauZCols]) {
+    float2 bv[GROUP ? F : 1][COLS];
+    auto load_beam = [&](int f, float2(&v)[COLS]) {
       if (p.staged) {
-        const float4 *src = reinterpret_cast<const float4 *>(beam_sm + (b * F + f) * kTauZBeamRow) + sg;
+        const float4 *src = reinterpret_cast<const float4 *>(beam_sm + (b * F + f) * ROW) + sg;
 #pragma unroll
-        for (int k = 0; k < kTauZCols; k += 2) {
+        for (int k = 0; k < COLS; k += 2) {
           const float4 v2 = src[(k >> 1) * kTauZGroups];
           v[k] = make_float2(v2.x, v2.y);
           v[k + 1] = make_float2(v2.z, v2.w);
         }
       } else {
 #pragma unroll
-        for (int k = 0; k < kTauZCols; ++k) {
+        for (int k = 0; k < COLS; ++k) {
           const int64_t s = sb + sg * NS + k / X;
           const float2 v1 = s < n ? __ldca(p.beam + (int64_t)((b * F + f) * X + k % X) * p.beam_ld + s)
                                   : make_float2(0.f, 0.f);
@@ -424,10 +440,10 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
       uint8_t *zg = static_cast<uint8_t *>(p.z) + (g0 + g) * p.zstride;
 #pragma unroll
       for (int f = 0; f < F; ++f) {
-        float vr[kTauZCols], vi[kTauZCols];
+        float vr[COLS], vi[COLS];
         if constexpr (!GROUP) load_beam(f, bv[0]);
 #pragma unroll
-        for (int k = 0; k < kTauZCols; ++k) {
+        for (int k = 0; k < COLS; ++k) {
           const float2 v = bv[GROUP ? f : 0][k];
           vr[k] = er[k / X] * v.x - ei[k / X] * v.y;
           vi[k] = er[k / X] * v.y + ei[k / X] * v.x;
@@ -446,11 +462,11 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
         }
         const int64_t m = (int64_t)a * F + f;
         if constexpr (MODE == MVB_Z_C64) {
-          // the row's 8 values start a multiple of 64 bytes into the panel (Kcap a
+          // the row's values start a multiple of 32 bytes into the panel (Kcap a
           // multiple of 64): whole 32-byte sectors, four values each
           float2 *zp = reinterpret_cast<float2 *>(zg) + m * p.Kcap + k0;
 #pragma unroll
-          for (int i = 0; i < kTauZCols; i += 4) {
+          for (int i = 0; i < COLS; i += 4) {
             const uint32_t w[8] = {__float_as_uint(vr[i]),     __float_as_uint(vi[i]),     __float_as_uint(vr[i + 1]),
                                    __float_as_uint(vi[i + 1]), __float_as_uint(vr[i + 2]), __float_as_uint(vi[i + 2]),
                                    __float_as_uint(vr[i + 3]), __float_as_uint(vi[i + 3])};
@@ -460,20 +476,20 @@ __global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GRO
               store_words<8>(zp + i, w);
           }
         } else {
-          // 8 consecutive k from a multiple of 8: inside one k-block
+          // COLS consecutive k from a multiple of COLS: inside one k-block
           constexpr int KB = kKBlockBytes / (MODE == MVB_GEMM_TF32_3 ? 4 : 2);
           constexpr int NPL = MODE == MVB_GEMM_BF16_6 ? 6 : 4;
           const int64_t off = panel_off(m, k0, p.Mpad, KB, NPL);
-          const int64_t off2 = panel_off(m, k0 + kTauZCols / 2, p.Mpad, KB, NPL);
-          if constexpr (WIDE) {
-            put_split<MODE, kTauZCols>(zg, panel_plane_stride(KB), off, off2, 0, vr, 1.f);
-            put_split<MODE, kTauZCols>(zg, panel_plane_stride(KB), off, off2, 1, vi, 1.f);
+          const int64_t off2 = panel_off(m, k0 + COLS / 2, p.Mpad, KB, NPL);
+          if constexpr (WIDE || COLS == 4) {
+            put_split<MODE, COLS>(zg, panel_plane_stride(KB), off, off2, 0, vr, 1.f);
+            put_split<MODE, COLS>(zg, panel_plane_stride(KB), off, off2, 1, vi, 1.f);
           } else {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               const int64_t o = h ? off2 : off;
-              put_split<MODE, kTauZCols / 2>(zg, panel_plane_stride(KB), o, o, 0, vr + h * (kTauZCols / 2), 1.f);
-              put_split<MODE, kTauZCols / 2>(zg, panel_plane_stride(KB), o, o, 1, vi + h * (kTauZCols / 2), 1.f);
+              put_split<MODE, 4>(zg, panel_plane_stride(KB), o, o, 0, vr + 4 * h, 1.f);
+              put_split<MODE, 4>(zg, panel_plane_stride(KB), o, o, 1, vi + 4 * h, 1.f);
             }
           }
         }
@@ -811,10 +827,11 @@ extern "C" int mvb_exptau(const double *antpos, int A, double freq, const double
 template <int MODE, bool POL, bool GROUP, bool WIDE>
 static int launch_tau_z_form(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
   auto launch = [&](auto kernel) { return launch_chained("tau_z_kernel", kernel, grid, kTauZThreads, smem, s, p); };
+  constexpr bool G4 = GROUP && tau_z_groups(MODE, 2, 2);
   if constexpr (POL) {
-    return launch(tau_z_kernel<MODE, 2, 2, true, GROUP, WIDE>);
+    return launch(tau_z_kernel<MODE, 2, 2, true, G4, WIDE>);
   } else if (X == 2) {
-    return F == 2 ? launch(tau_z_kernel<MODE, 2, 2, false, GROUP, WIDE>)
+    return F == 2 ? launch(tau_z_kernel<MODE, 2, 2, false, G4, WIDE>)
                   : launch(tau_z_kernel<MODE, 2, 1, false, GROUP, WIDE>);
   } else {
     return F == 2 ? launch(tau_z_kernel<MODE, 1, 2, false, GROUP, WIDE>)
@@ -825,6 +842,7 @@ static int launch_tau_z_form(const TauZArgs &p, int F, int X, dim3 grid, size_t 
 template <int MODE, bool POL>
 static int launch_tau_z_mode(const TauZArgs &p, bool wide, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
   if (!wide) return launch_tau_z_form<MODE, POL, false, false>(p, F, X, grid, smem, s);
+  // (tau_z_cols: the launch's shape goes with this choice)
   if (p.per_z > 1) return launch_tau_z_form<MODE, POL, true, true>(p, F, X, grid, smem, s);
   return launch_tau_z_form<MODE, POL, false, true>(p, F, X, grid, smem, s);
 }
@@ -895,15 +913,20 @@ static int launch_tau_z(const char *who, TauZArgs p, const double *antpos, int A
   const int64_t units = xblocks * ceil_div(A, kTauZAntLanes) * nfreq;
   const int64_t share = std::max<int64_t>(1, units / ((int64_t)num_sms() * kTauZCtasPerSm));
   const int64_t parts = ceil_div(nfreq, std::min<int64_t>({share, (int64_t)kTauZMaxFreq, (int64_t)nfreq}));
-  p.per_z = wide ? (int)ceil_div(nfreq, parts) : 1;
-  const int64_t lanes = std::min<int64_t>(std::max<int64_t>(share / p.per_z, 1), kTauZAnts / kTauZAntLanes);
+  const int per = (int)ceil_div(nfreq, parts);
+  // At one beam axis two frequencies do not repay the eight-column form (tau_z_cols):
+  // 350 antennas x 15,000 slots x 2, half live, tf32x3: 20.6 us one by one, 27.0 together.
+  p.per_z = wide && tau_z_groups(mode, F, X) && !(X == 1 && per == 2) ? per : 1;
+  const int tcols = tau_z_cols(X, p.per_z > 1);  // (a launch of one frequency per CTA: the form that is not GROUP)
+  const int64_t lanes =
+      std::min<int64_t>(std::max<int64_t>(share * (kTauZCols / tcols) / p.per_z, 1), kTauZAnts / kTauZAntLanes);
   const int64_t ablocks = ceil_div(A, lanes * kTauZAntLanes);
   p.ants = (int)round_up(ceil_div(A, ablocks), kTauZAntLanes);  // even shares, whole lanes
-  const dim3 grid((unsigned)(cols / (kTauZCols * kTauZGroups)), (unsigned)ceil_div(A, p.ants),
+  const dim3 grid((unsigned)(cols / (tcols * kTauZGroups)), (unsigned)ceil_div(A, p.ants),
                   (unsigned)ceil_div(nfreq, p.per_z));
-  const int bs = kTauZCols / X * kTauZGroups;
+  const int bs = tcols / X * kTauZGroups;
   const size_t smem = (size_t)p.per_z * bs * (POL ? sizeof(float4) : sizeof(float)) +
-                      (p.staged ? (size_t)nbeam * F * kTauZBeamRow * sizeof(float2) : 0);
+                      (p.staged ? (size_t)nbeam * F * tcols * kTauZGroups * sizeof(float2) : 0);
   cudaStream_t s = as_stream(stream);
   switch (mode) {
     case MVB_GEMM_BF16_3: return launch_tau_z_mode<MVB_GEMM_BF16_3, POL>(p, wide, F, X, grid, smem, s);
