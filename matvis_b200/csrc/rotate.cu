@@ -96,8 +96,11 @@ __global__ void __launch_bounds__(kCompactThreads)
   if (threadIdx.x == 0) block_counts[blockIdx.x] = s;
 }
 
-// Four consecutive sources a thread, so that one scan of per-thread counts ranks the
-// block (four rounds of 256 sources with three barriers each before).
+// A warp takes 128 consecutive sources in four rounds of 32, so that its loads and
+// stores are whole lines and its ballots rank them; one barrier then adds the counts
+// of the warps and blocks before it (four rounds of 256 sources with three barriers
+// each: 10.0 us at 100,000 sources, 37.6 at 3,000,000; four consecutive sources a
+// thread: 5.8 and 41.1; this: 6.0 and 37.4; 1,000,000: 16.6, 16.6 and 12.1).
 __global__ void __launch_bounds__(kCompactThreads)
     horizon_scatter_kernel(const double *__restrict__ topo, int64_t ld, int64_t c0, int64_t count,
                            const int32_t *__restrict__ block_counts, int nblocks, const double *__restrict__ flux,
@@ -111,10 +114,10 @@ __global__ void __launch_bounds__(kCompactThreads)
   pdl_trigger();
 
   const double *zr = topo + 2 * ld + c0;
-  const int64_t i0 = (int64_t)blockIdx.x * kCompactBlock + threadIdx.x * kCompactPerThread;
+  const int64_t i0 = (int64_t)blockIdx.x * kCompactBlock + warp * (32 * kCompactPerThread) + lane;
   double z[kCompactPerThread];
 #pragma unroll
-  for (int j = 0; j < kCompactPerThread; ++j) z[j] = i0 + j < count ? __ldcg(zr + i0 + j) : 0.0;
+  for (int j = 0; j < kCompactPerThread; ++j) z[j] = i0 + 32 * j < count ? __ldcg(zr + i0 + 32 * j) : 0.0;
 
   // counts of earlier blocks, and the grand total
   long long before = 0, total = 0;
@@ -123,20 +126,19 @@ __global__ void __launch_bounds__(kCompactThreads)
     total += c;
     if (b < (int)blockIdx.x) before += c;
   }
-  unsigned keep = 0;
+  unsigned keep[kCompactPerThread];
+  int kept = 0;  // of the warp
 #pragma unroll
-  for (int j = 0; j < kCompactPerThread; ++j) keep |= (z[j] > 0.0 ? 1u : 0u) << j;
-  int scan = __popc(keep);  // becomes the warp's inclusive scan
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, scan, o);
-    if (lane >= o) scan += v;
+  for (int j = 0; j < kCompactPerThread; ++j) {
+    keep[j] = __ballot_sync(0xffffffffu, z[j] > 0.0);
+    kept += __popc(keep[j]);
   }
   for (int o = 16; o > 0; o >>= 1) {
     before += __shfl_xor_sync(0xffffffffu, before, o);
     total += __shfl_xor_sync(0xffffffffu, total, o);
   }
-  if (lane == 31) {
-    warp_cnt[warp] = scan;
+  if (lane == 0) {
+    warp_cnt[warp] = kept;
     red_before[warp] = before;
     red_total[warp] = total;
   }
@@ -147,19 +149,19 @@ __global__ void __launch_bounds__(kCompactThreads)
     before += red_before[w] + (w < warp ? warp_cnt[w] : 0);
     total += red_total[w];
   }
-  long long pos = before + scan - __popc(keep);
+  long long first = before;  // slot of the round's first kept source
   const double *xr = topo + c0, *yr = topo + ld + c0;
 #pragma unroll
   for (int j = 0; j < kCompactPerThread; ++j) {
-    if (!((keep >> j) & 1u)) continue;
-    if (pos < cap) {
-      crd_out[pos] = __ldcg(xr + i0 + j);
-      crd_out[cap + pos] = __ldcg(yr + i0 + j);
-      crd_out[2 * cap + pos] = z[j];
-      idx_out[pos] = (int32_t)(c0 + i0 + j);
-      if (flux != nullptr) flux_out[pos] = flux[c0 + i0 + j];
-    }
-    ++pos;
+    const long long pos = first + __popc(keep[j] & ((1u << lane) - 1u));
+    first += __popc(keep[j]);
+    if (!((keep[j] >> lane) & 1u) || pos >= cap) continue;
+    const int64_t i = i0 + 32 * j;
+    crd_out[pos] = __ldcg(xr + i);
+    crd_out[cap + pos] = __ldcg(yr + i);
+    crd_out[2 * cap + pos] = z[j];
+    idx_out[pos] = (int32_t)(c0 + i);
+    if (flux != nullptr) flux_out[pos] = flux[c0 + i];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *n_out = (int32_t)total;
