@@ -658,8 +658,7 @@ __device__ __forceinline__ void load_row(const CT *__restrict__ row, int64_t k, 
 }
 
 // Packs a caller complex matrix (M, K) into a panel.  CTA = 256 threads: 16 groups
-// of C columns (8 of complex64, 4 of complex128: 64 bytes, beyond which a load
-// instruction touches a line per lane) x 16 row lanes x `lane_rows` rows each, so
+// of C columns (pack_cols) x 16 row lanes x `lane_rows` rows each, so
 // stores fill 8 or 16 bytes of a plane row.  It is bound by HBM; the row blocks run
 // last to first, so that those a maximum pass has just read come from L2.  With
 // `absmax` the fp16 scale is formed here from that pass's result and written to
@@ -671,15 +670,21 @@ __device__ __forceinline__ void load_row(const CT *__restrict__ row, int64_t k, 
 constexpr int kPackThreads = 256;
 constexpr int kPackGroups = 16;
 
-template <typename CT>
-constexpr int kPackCols = 64 / (int)sizeof(CT);
+// Columns per thread: 8 of complex64 and 4 of complex128, 64 bytes, beyond which a load
+// instruction touches a line per lane.  Rows of an odd pitch are loaded value by value,
+// for which 64 bytes a lane are too far apart: 4 of complex64 (fp16x3 writes more per
+// value than it loads and keeps 8).  700 x 50,001 complex64 to a plain Z: 92 us with 4,
+// 100 with 8; 90 x 50,001 from L2: 11.7 and 16.3; 700 x 50,001 to fp16x3: 106 and 104.
+constexpr int pack_cols(int mode, int value_bytes, bool vec) {
+  return value_bytes == 16 || (!vec && mode != MVB_GEMM_F16_3) ? 4 : 8;
+}
 
-template <int MODE, typename CT>
+template <int MODE, typename CT, int C>
 __global__ void __launch_bounds__(kPackThreads)
     z_pack_kernel(const CT *__restrict__ zs, int64_t M, int64_t K, int64_t ldz, float zscale,
                   const float *__restrict__ absmax, float *__restrict__ scale_out, void *__restrict__ z, int64_t Mpad,
                   int64_t Kcap, int lane_rows, bool vec, int align) {
-  constexpr int C = kPackCols<CT>, LANES = kPackThreads / kPackGroups;
+  constexpr int LANES = kPackThreads / kPackGroups;
   if (absmax) {
     zscale = panel_scale(*absmax);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scale_out = zscale;
@@ -986,21 +991,23 @@ static int z_pack_impl(const char *who, const void *zsrc, int z_c128, int64_t M,
   // the narrowest stores: 16 bytes of a complex64 Z, pairs of float32 or bf16, single fp16
   int rc = check_align(who, z, mode == MVB_Z_C64 ? 16 : mode == MVB_GEMM_TF32_3 ? 8 : mode == MVB_GEMM_F16_3 ? 2 : 4);
   if (rc) return rc;
-  const int64_t xblocks = ceil_div(cols, kPackGroups * (z_c128 ? kPackCols<double2> : kPackCols<float2>));
+  const bool vec = reinterpret_cast<uintptr_t>(zsrc) % 16 == 0 && (z_c128 || ldz % 2 == 0);
+  const int64_t xblocks = ceil_div(cols, kPackGroups * pack_cols(mode, z_c128 ? 16 : 8, vec));
   // four rows a lane (a 64-row block) where that still leaves eight CTAs per SM
   constexpr int lanes = kPackThreads / kPackGroups;
   const int lane_rows = xblocks * ceil_div(M, 4 * lanes) >= (int64_t)num_sms() * 8 ? 4 : 1;
   const dim3 grid((unsigned)xblocks, (unsigned)std::min<int64_t>(ceil_div(M, (int64_t)lane_rows * lanes), 65535));
-  const bool vec = reinterpret_cast<uintptr_t>(zsrc) % 16 == 0 && (z_c128 || ldz % 2 == 0);
   const int align = reinterpret_cast<uintptr_t>(z) % 32 == 0 ? 2 : (reinterpret_cast<uintptr_t>(z) % 16 == 0 ? 1 : 0);
-#define MVB_PACK(M_, CT)                                                                                            \
-  z_pack_kernel<M_, CT><<<grid, kPackThreads, 0, s>>>(static_cast<const CT *>(zsrc), M, K, ldz, zscale, absmax,     \
+#define MVB_PACK(M_, CT, VEC)                                                                                       \
+  z_pack_kernel<M_, CT, pack_cols(M_, sizeof(CT), VEC)><<<grid, kPackThreads, 0, s>>>(static_cast<const CT *>(zsrc), M, K, ldz, zscale, absmax,     \
                                                       scale_out, z, Mpad, Kcap, lane_rows, vec, align)
 #define MVB_PACK2(M_) \
   if (z_c128)         \
-    MVB_PACK(M_, double2); \
+    MVB_PACK(M_, double2, true); \
+  else if (vec)       \
+    MVB_PACK(M_, float2, true); \
   else                \
-    MVB_PACK(M_, float2)
+    MVB_PACK(M_, float2, false)
   switch (mode) {
     case MVB_GEMM_BF16_3: MVB_PACK2(MVB_GEMM_BF16_3); break;
     case MVB_GEMM_BF16_6: MVB_PACK2(MVB_GEMM_BF16_6); break;
