@@ -245,18 +245,20 @@ constexpr int kTauZCtasPerSm = 8;           // CTAs per SM that a small launch i
 // read through L1: 91 and 176); 100 x 60,000 as a complex64 Z: 17 and 28.
 __host__ __device__ constexpr int tau_z_cols(int X, bool group) { return X == 1 && !group ? 4 : kTauZCols; }
 
-// Whether frequencies share a CTA.  A two-feed, two-axis tf32x3 panel is 16 bytes a
-// value and bound by its stores: fewer and longer CTAs only cost their last wave.  350
-// antennas x 6,000 slots x 12, half live: 122 us one frequency per CTA, 141 shared;
-// x 40,000 x 3: 221 and 220; polarised sky, x 15,000 x 8: 233 and 270.
-__host__ __device__ constexpr bool tau_z_groups(int mode, int F, int X) {
-  return !(mode == MVB_GEMM_TF32_3 && F * X == 4);
-}
+// CTAs per SM that a two-feed, two-axis tf32x3 or bf16x6 launch has to keep for
+// frequencies to share them.  Those panels are 16 and 12 bytes a value and bound by
+// their stores, and fewer, longer CTAs cost their last wave: tf32x3, 350 antennas x
+// 6,000 slots x 12, half live, 141 us shared (15 CTAs per SM), 122 one by one; x 15,000 x
+// 3 168 and 164 (19); x 40,000 x 3 438 and 455 (51); bf16x6, 512 x 9,000 x 12 437 and
+// 408 (30); 350 x 40,000 x 6 620 and 658 (51).  A polarised sky's factors are shared
+// too: bf16x6 always pays (x 40,000 x 6 635 and 733), tf32x3 never (x 40,000 x 3 263 and
+// 245).
+constexpr int kTauZWideCtasPerSm = 40;
 
 // Resident CTAs per SM that the registers are held to (the best of 4, 5, 6, 8 and
 // no bound, by form: the polarised group form keeps 32 beam values a thread).
-constexpr int tau_z_min_blocks(int X, int F, bool group) {
-  return X * F == 4 ? (group ? 4 : 6) : (X == 1 && F == 2 ? 5 : 6);
+constexpr int tau_z_min_blocks(int mode, int X, int F, bool group) {
+  return X * F == 4 ? (!group ? 6 : (mode == MVB_GEMM_TF32_3 ? 5 : 4)) : (X == 1 && F == 2 ? 5 : 6);
 }
 
 struct TauZArgs {
@@ -299,7 +301,7 @@ __device__ __forceinline__ float4 coherency_factor(float4 c, double2 r) {
 // z + g zstride bytes.  WIDE: every panel is aligned to the stores of eight columns
 // (store_align); otherwise eight columns go out in two halves, the same bytes.
 template <int MODE, int X, int F, bool POL, bool GROUP, bool WIDE>
-__global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(X, F, GROUP)) tau_z_kernel(const __grid_constant__ TauZArgs p) {
+__global__ void __launch_bounds__(kTauZThreads, tau_z_min_blocks(MODE, X, F, GROUP)) tau_z_kernel(const __grid_constant__ TauZArgs p) {
   static_assert(!POL || (X == 2 && F == 2), "the polarised sky needs two feeds and two beam axes");
   static_assert(!GROUP || WIDE, "narrow stores: one frequency per CTA");
   constexpr int COLS = tau_z_cols(X, GROUP);
@@ -832,11 +834,10 @@ extern "C" int mvb_exptau(const double *antpos, int A, double freq, const double
 template <int MODE, bool POL, bool GROUP, bool WIDE>
 static int launch_tau_z_form(const TauZArgs &p, int F, int X, dim3 grid, size_t smem, cudaStream_t s) {
   auto launch = [&](auto kernel) { return launch_chained("tau_z_kernel", kernel, grid, kTauZThreads, smem, s, p); };
-  constexpr bool G4 = GROUP && tau_z_groups(MODE, 2, 2);
   if constexpr (POL) {
-    return launch(tau_z_kernel<MODE, 2, 2, true, G4, WIDE>);
+    return launch(tau_z_kernel<MODE, 2, 2, true, GROUP && MODE != MVB_GEMM_TF32_3, WIDE>);
   } else if (X == 2) {
-    return F == 2 ? launch(tau_z_kernel<MODE, 2, 2, false, G4, WIDE>)
+    return F == 2 ? launch(tau_z_kernel<MODE, 2, 2, false, GROUP, WIDE>)
                   : launch(tau_z_kernel<MODE, 2, 1, false, GROUP, WIDE>);
   } else {
     return F == 2 ? launch(tau_z_kernel<MODE, 1, 2, false, GROUP, WIDE>)
@@ -921,7 +922,11 @@ static int launch_tau_z(const char *who, TauZArgs p, const double *antpos, int A
   const int per = (int)ceil_div(nfreq, parts);
   // At one beam axis two frequencies do not repay the eight-column form (tau_z_cols):
   // 350 antennas x 15,000 slots x 2, half live, tf32x3: 20.6 us one by one, 27.0 together.
-  p.per_z = wide && tau_z_groups(mode, F, X) && !(X == 1 && per == 2) ? per : 1;
+  bool group = wide && !(X == 1 && per == 2);
+  if (POL && mode == MVB_GEMM_TF32_3) group = false;
+  if (!POL && X * F == 4 && (mode == MVB_GEMM_TF32_3 || mode == MVB_GEMM_BF16_6))
+    group = group && xblocks * ceil_div(A, kTauZAnts) * ceil_div(nfreq, per) >= (int64_t)num_sms() * kTauZWideCtasPerSm;
+  p.per_z = group ? per : 1;
   const int tcols = tau_z_cols(X, p.per_z > 1);  // (a launch of one frequency per CTA: the form that is not GROUP)
   const int64_t lanes =
       std::min<int64_t>(std::max<int64_t>(share * (kTauZCols / tcols) / p.per_z, 1), kTauZAnts / kTauZAntLanes);

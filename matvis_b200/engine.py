@@ -281,7 +281,7 @@ class VisEngine:
             zmax = smax * bmax * (2.0 if self.pol_sky else 1.0)
             self.zscale = _lib.f16_scale(zmax * (1 + 2**-10))
         self._graph = None
-        #: kernels of the latest ``enqueue`` (of the captured graph, after capture())
+        #: kernels of the captured graph (counted by capture())
         self.launched = 0
         self._allocated = False
         self._uploaded = False
@@ -472,13 +472,10 @@ class VisEngine:
         return j, keep
 
     def enqueue(self, stream=None):
-        """Enqueue every kernel of the job on ``stream`` (no host synchronisation);
-        ``launched`` then holds how many there were."""
+        """Enqueue every kernel of the job on ``stream`` (no host synchronisation)."""
         job, _keep = self._launches()
-        before = _lib.lib.mvb_launches()
         _lib.check(_lib.lib.mvb_job_enqueue(ctypes.byref(job), 0, len(self.lsts), 0, self.nchunks, 0, len(self.freqs),
                                             _lib.stream_handle(stream)))
-        self.launched = _lib.lib.mvb_launches() - before
 
     def enqueue_time(self, t: int, stream=None, after=None, launches=None):
         """Enqueue the kernels of time index t (all chunks and frequencies).
@@ -587,7 +584,8 @@ class VisEngine:
     def launches_per_run(self) -> int:
         """At most this many kernel launches a run: what it is split into by hand
         (rotation and horizon count apart, a gridded beam laid out and gathered).  The
-        number made is less where one kernel does two of these; ``launched`` has it."""
+        number made is less where one kernel does two of these: capture() counts it, and
+        ``mvb_launches`` counts any call's."""
         # per frequency (or per group of fgroup frequencies): tau/Z, then the product
         # and its reduction (mvb_herk[_grouped] + reduce, or vecdot_kernel + its slice reduction)
         per_f = 3
@@ -731,7 +729,9 @@ class VisEngine:
         s.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(s):
             with torch.cuda.graph(g, stream=s):
+                before = _lib.lib.mvb_launches()
                 self.enqueue(stream=s)
+                self.launched = _lib.lib.mvb_launches() - before
         torch.cuda.current_stream().wait_stream(s)
         self._graph = g
         return g

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from matvis_b200 import workloads as wl
+from matvis_b200 import _lib, workloads as wl
 from matvis_b200.beam_models import GaussianBeam
 from matvis_b200.engine import VisEngine, job_from_arrays
 from matvis_b200.serve import VisServer
@@ -39,8 +39,11 @@ def test_engine_counts_its_launches(kw):
     eng = VisEngine(_spec(**kw))
     eng.upload()
     eng.enqueue()
-    assert _kernels(eng.enqueue) == eng.launched > 0
-    assert eng.launched <= eng.launches_per_run()
+    before = _lib.lib.mvb_launches()
+    n = _kernels(eng.enqueue)
+    assert n == _lib.lib.mvb_launches() - before > 0
+    eng.capture()
+    assert n == eng.launched == _kernels(eng.run) <= eng.launches_per_run()
 
 
 @pytest.mark.parametrize("batch", [True, False])
