@@ -98,9 +98,11 @@ __global__ void __launch_bounds__(kCompactThreads)
 
 // A warp takes 128 consecutive sources in four rounds of 32, so that its loads and
 // stores are whole lines and its ballots rank them; one barrier then adds the counts
-// of the warps and blocks before it (four rounds of 256 sources with three barriers
-// each: 10.0 us at 100,000 sources, 37.6 at 3,000,000; four consecutive sources a
-// thread: 5.8 and 41.1; this: 6.0 and 37.4; 1,000,000: 16.6, 16.6 and 12.1).
+// of the warps and blocks before it, while the kept sources' other coordinates load.
+// Count and scatter at 100,000 / 1,000,000 / 3,000,000 sources: four rounds of 256
+// sources with three barriers each 10.0 / 16.6 / 37.6 us; four consecutive sources a
+// thread 5.8 / 16.6 / 41.1; this 6.4 / 9.5 / 24.1 (a 37-antenna job of five times, whose
+// chain waits for it, 287 -> 279 us).
 __global__ void __launch_bounds__(kCompactThreads)
     horizon_scatter_kernel(const double *__restrict__ topo, int64_t ld, int64_t c0, int64_t count,
                            const int32_t *__restrict__ block_counts, int nblocks, const double *__restrict__ flux,
@@ -126,6 +128,14 @@ __global__ void __launch_bounds__(kCompactThreads)
     total += c;
     if (b < (int)blockIdx.x) before += c;
   }
+  // the other coordinates are on their way while the ranks are formed
+  const double *xr = topo + c0, *yr = topo + ld + c0;
+  double x[kCompactPerThread], y[kCompactPerThread];
+#pragma unroll
+  for (int j = 0; j < kCompactPerThread; ++j) {
+    x[j] = z[j] > 0.0 ? __ldcg(xr + i0 + 32 * j) : 0.0;
+    y[j] = z[j] > 0.0 ? __ldcg(yr + i0 + 32 * j) : 0.0;
+  }
   unsigned keep[kCompactPerThread];
   int kept = 0;  // of the warp
 #pragma unroll
@@ -150,15 +160,14 @@ __global__ void __launch_bounds__(kCompactThreads)
     total += red_total[w];
   }
   long long first = before;  // slot of the round's first kept source
-  const double *xr = topo + c0, *yr = topo + ld + c0;
 #pragma unroll
   for (int j = 0; j < kCompactPerThread; ++j) {
     const long long pos = first + __popc(keep[j] & ((1u << lane) - 1u));
     first += __popc(keep[j]);
     if (!((keep[j] >> lane) & 1u) || pos >= cap) continue;
     const int64_t i = i0 + 32 * j;
-    crd_out[pos] = __ldcg(xr + i);
-    crd_out[cap + pos] = __ldcg(yr + i);
+    crd_out[pos] = x[j];
+    crd_out[cap + pos] = y[j];
     crd_out[2 * cap + pos] = z[j];
     idx_out[pos] = (int32_t)(c0 + i);
     if (flux != nullptr) flux_out[pos] = flux[c0 + i];
