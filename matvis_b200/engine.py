@@ -138,7 +138,11 @@ class _PageToucher:
         self._out = out
         self._page = max(4096 // out.itemsize, 1)
         nf, nt = out.shape[:2]
-        self._pool = ThreadPoolExecutor(min(os.cpu_count() or 1, 8))
+        # two threads keep ahead of the copies; more of them contend, with one another for
+        # the address space and with the calling thread for the interpreter (median of a
+        # call with 0.3 MB a slice, 164 MB in all: 47 ms with 2 threads, 61 with 8, 52 with
+        # the copying thread alone; 2.9 MB a slice: 17, 17 to 25, 30)
+        self._pool = ThreadPoolExecutor(min(os.cpu_count() or 1, 2))
         self._done = {(t, f0): self._pool.submit(self._touch, t, f0, min(group, nf - f0))
                       for t in range(nt) for f0 in range(0, nf, group)}
 
@@ -619,7 +623,7 @@ class VisEngine:
         stream, so the device -> host copy overlaps the compute that follows;
         only the last group's copy runs after the compute.  The first touch of
         freshly allocated host pages is slower than the copy itself (the kernel
-        clears them at about 10 GB/s a core): a few threads do it, from before the
+        clears them at about 10 GB/s a core): two threads do it, from before the
         job's buffers are made, in the order of the copies.  A result of at most
         ``SMALL_RESULT`` bytes is copied in one piece after the run.
         """
