@@ -125,9 +125,8 @@ int mvb_horizon_compact_static(const double *topo, int64_t ld, int64_t c0, int64
  * 0 complex64 E-field, 1 float32 power (sqrt applied after interpolation).
  * params: nbeam x 3 doubles (daz, dza, azmin).  Output (nbeam, nfeed, nax, nout)
  * complex64 (out_c128 = 0) or complex128 (1); sources i >= n (n = *n_dev if
- * n_dev != NULL, else nsrc) are written as 0.  Grids of up to 200 KB per real
- * plane are staged in shared memory.  If status != NULL, a non-finite result
- * sets MVB_DEV_NONFINITE.  Replaces BeamInterpolator.__call__ /
+ * n_dev != NULL, else nsrc) are written as 0.  If status != NULL, a non-finite
+ * result sets MVB_DEV_NONFINITE.  Replaces BeamInterpolator.__call__ /
  * GPUBeamInterpolator._interp (core/beams.py:184-208, gpu/beams.py:103-200). */
 int mvb_beam_interp(const void *grids, int grid_kind, int nbeam, int nax, int nfeed, int nza, int naz,
                     const double *params, const double *crd, int64_t ld, const int32_t *n_dev, int64_t nsrc,

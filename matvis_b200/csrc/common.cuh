@@ -45,7 +45,8 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 // tensor-memory set-up overlap the predecessor's tail.  Such a kernel calls
 // pdl_wait() before it touches global memory -- it returns when every earlier
 // kernel of the stream is complete, since each of them waited too -- and
-// pdl_trigger() once its successor may be scheduled.
+// pdl_trigger() once its successor may be scheduled (the first thread of each CTA that
+// calls it counts; it says nothing about what the others have done).
 template <typename... KArgs, typename... Args>
 inline int launch_chained(const char *what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                           cudaStream_t s, Args... args) {

@@ -731,7 +731,10 @@ __global__ void __launch_bounds__(kHerkThreads, 1)
     }
   }
 
-  pdl_trigger();  // this CTA's units are done
+  // Takes effect with the first thread that gets here, the producer's, while the CTA's
+  // last stages are still multiplied and stored: a dependent may be scheduled from then
+  // on, and reads nothing of this launch before its pdl_wait().
+  pdl_trigger();
   __syncthreads();
   if (abort_flag) {
     if (warp == 0 && lane == 0) {

@@ -48,10 +48,11 @@ from . import autotune
 from .autotune import KD_CANDIDATES, tune_product
 from .matprod import B200MatMul, B200VectorDot, choose_k_chunk, pair_product
 
-#: k-slice of the Hermitian product without autotuning: the tuner's choice for
-#: the HERA-350-like slice in fp16x3 (product + reduction 1.12 ms at 4096
-#: columns, 1.19 at 2048; shorter slices mean more partial tiles to reduce).  The number of
-#: slices is still fitted to whole waves of SMs on the device.
+#: k-slice of the Hermitian product without autotuning.  On the HERA-350-like slice in
+#: fp16x3 product and reduction take 1.04 / 0.99 / 0.97 ms at 2048 / 4096 / 8192 columns
+#: (shorter slices mean more partial tiles to reduce); the tuner, which times a job's own
+#: panel, takes 8192 there, and half of that serves shorter panels without it.  The number
+#: of slices is still fitted to whole waves of SMs on the device.
 DEFAULT_K_CHUNK = 4096
 
 #: Frequencies per grouped launch (tau/Z, product and reduction of that many
@@ -789,7 +790,7 @@ def estimate_device_bytes(spec: JobSpec) -> int:
     nbeam = len(spec.beams)
     pol_sky = np.ndim(spec.fluxes) == 4
     extra = (16 * Nf * N + 16 * N + 16 * cap) if pol_sky else 0  # coherency, ra/dec, frame rotations
-    beam = 8 * nbeam * F * X * cap + 16 * nbeam * cap  # interpolated beams, per-source grid coordinates
+    beam = 8 * nbeam * F * X * cap + 16 * nbeam * cap  # interpolated beams, room for the packed grids
     return int(24 * N + 8 * 3 * A + 4 * Nf * N + 24 * N + 28 * cap + beam + panel + ws
                + Nf * Nt * npairs * F * F * csize + extra)
 

@@ -38,13 +38,17 @@ def choose_k_chunk(n_tiles: int, kvalid: int, num_sms: int = 148, lo: int = 1024
     return int(min(max(kc, lo), hi))
 
 
-#: Per-column costs measured on one B200 on a config-3 slice (K = 1.0e6 columns,
-#: the seeded 5,000 pairs at F = 2): mvb_vecdot_staged took 5.64 ms, i.e.
-#: 2.8e-13 s per (pair x F^2 x column), mvb_vecdot (one warp per pair, for
-#: arrays too large to stage) 11.83 ms, 5.9e-13 s; mvb_herk in fp16x3 took
-#: 6.51 ms for 21 tiles of 128 x 128, i.e. 1.03e-10 s per (tile x split product
-#: x column), with TF32 operands at half that rate.  Break-even at F = 2, 21
-#: tiles: ~5,750 pairs (staged).
+#: Per-column costs whose ratio sets the line between the two kernels: seconds per
+#: (pair x F^2 x column) of mvb_vecdot_staged and mvb_vecdot (one warp per pair, for
+#: arrays too large to stage), and per (tile x split product x column) of mvb_herk in
+#: fp16x3, TF32 operands at half that rate.  The line at 350 two-feed antennas (21
+#: tiles) is ~5,790 pairs.  Measured with both kernels in seconds-long runs (the product
+#: is then at the power cap: 9.4e-11; 5,000 pairs 2.6e-13): break-even at 5,690 pairs
+#: counted from the time of 5,000 and 5,860 from that of 6,500 (K = 1.0e6; 4,980 at K =
+#: 1.0e5).  A single product after a pause is faster (8.1e-11): 4,860 to 5,020, so that
+#: between those lists and the line a lone snapshot loses up to 15 % on per-pair sums.
+#: 128 two-feed antennas (3 tiles, K = 4.0e5): 750 pairs sustained, 630 alone; the line
+#: lies at 830.
 VECDOT_STAGED_S_PER_PAIR_COL = 2.8e-13
 VECDOT_S_PER_PAIR_COL = 5.9e-13
 HERK_S_PER_TILE_PRODUCT_COL = 1.03e-10
@@ -60,7 +64,7 @@ def pair_product(nant: int, nfeed: int, npairs: int, gemm_mode="fp16x3") -> str:
     else ``"vecdot"``.  Both give the reference's VectorDot output
     out[i, p, q] = sum_k Z[aj F + p, k] conj(Z[ai F + q, k]) (cpu/matprod.py:48-51);
     the per-column cost of each kernel is the measured one above, so the choice
-    does not depend on the source count.  Lists above ~5,750 pairs of a
+    does not depend on the source count.  Lists above ~5,790 pairs of a
     350-antenna two-feed array go to the Hermitian product; shorter ones
     (redundant-baseline sets of compact arrays, sparse pair selections) stay on
     per-pair sums.
